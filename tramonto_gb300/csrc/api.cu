@@ -400,7 +400,7 @@ void ensure_fft(Ctx *c)
   plan_geometry_args(c, P, nx, h, per);
   if (!tgpu::fft_make_plan(c->fft, P, nx, h, per, dg.ndim, c->stream)) return;
   c->fft_plan_ok = true;
-  const long NH = c->fft.NH, NR = c->fft.NR;
+  const long NH = c->fft.NS, NR = c->fft.NR;   // stored half-spectrum points
   // device memory: three work spectra and one spectrum per stencil coefficient
   size_t nspec = 0;
   for (int t = 0; t < 3; t++)
@@ -448,7 +448,7 @@ bool prepare_spec32(Ctx *c)
   if (c->spec32_built) return true;
   ensure_fft(c);
   if (!c->fft_plan_ok) return false;
-  const long NH = c->fft.NH, NR = c->fft.NR;
+  const long NH = c->fft.NS, NR = c->fft.NR;
   double2 *tmp = dalloc<double2>((size_t)NH);
   double *rbox = dalloc<double>((size_t)NR);
   for (int t = 0; t < 3; t++)
@@ -509,7 +509,7 @@ void fft_tr_sum(Ctx *c, const int *chs, const C *const *kern, int n, double *out
 {
   if (n > tgpu::fft_max_terms()) throw Error(TGPU_ERR_UNSUPPORTED, "too many channels for one FFT transposed sum");
   std::vector<C *> &boxes = tr_boxes<C>(c);
-  while ((int)boxes.size() < n) boxes.push_back(dalloc<C>((size_t)c->fft.NH));
+  while ((int)boxes.size() < n) boxes.push_back(dalloc<C>((size_t)c->fft.NS));
   std::vector<const C *> a(n);
   {   // the channels' spectra in one launch per pass
     std::vector<tgpu::MapSrc> ms(n);
@@ -543,7 +543,7 @@ void fft_conv_impl(Ctx *c, int ch0, int nin, const std::vector<C *> &spec, bool 
     const C *F = channel(c, ch0);
     {   // every output in one launch per pass
       std::vector<C *> &work = tr_boxes<C>(c);
-      while ((int)work.size() < nout) work.push_back(dalloc<C>((size_t)c->fft.NH));
+      while ((int)work.size() < nout) work.push_back(dalloc<C>((size_t)c->fft.NS));
       tgpu::rfft_inverse_batch(F, spec.data(), nout, work.data(), c->fft, 1.0 / (double)c->fft.NR, outs, true,
                                c->stream);
       c->stats.kernel_launches += 3;
@@ -783,7 +783,7 @@ void forward_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, boo
           }
         const double2 *F = fft_channel(c, jc);
         std::vector<double2 *> &work = tr_boxes<double2>(c);
-        while (work.size() < ks.size()) work.push_back(dalloc<double2>((size_t)c->fft.NH));
+        while (work.size() < ks.size()) work.push_back(dalloc<double2>((size_t)c->fft.NS));
         tgpu::rfft_inverse_batch(F, ks.data(), (int)ks.size(), work.data(), c->fft, 1.0 / (double)c->fft.NR,
                                  os.data(), true, c->stream);
         c->stats.kernel_launches += 3 * ((ks.size() + tgpu::fft_max_batch() - 1) / tgpu::fft_max_batch());
@@ -812,7 +812,7 @@ void forward_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, boo
           }
         const float2 *F = fft_channel32(c, jc);
         std::vector<float2 *> &work = tr_boxes<float2>(c);
-        while (work.size() < ks.size()) work.push_back(dalloc<float2>((size_t)c->fft.NH));
+        while (work.size() < ks.size()) work.push_back(dalloc<float2>((size_t)c->fft.NS));
         if (c->store32) {   // the FP32 shadows of the sums
           std::vector<float *> os32;
           for (double *o : os) os32.push_back(c->d_conv32 + (o - c->d_conv));

@@ -69,19 +69,18 @@ constexpr double kDensityMin = 1.e-20;   // integrands vanish at or below this d
 // dimensions (no padding) and F_d >= the padded extent elsewhere, half spectrum [F2][F1][F0/2 + 1]; each axis's
 // length is a product of radices 2, 3, 4, 5
 struct FftAxis {
-  int n = 1, nst = 0;
-  int rad[16] = {0};
+  int n = 1, R1 = 1, R2 = 1;   // length and its two radices
   double2 *d_tw = nullptr;   // exp(-2 pi i k / n), k < n
   float2 *d_tw32 = nullptr;  // the same rounded to FP32 (the FP32 transforms)
 };
 struct FftPlan {
   int F[3] = {1, 1, 1};
-  int Fh = 1;                // F[0] / 2 + 1
+  int Fh = 1, Fp = 1;        // F[0] / 2 + 1 and the pitch of a stored line
   int P[3] = {1, 1, 1}, nx[3] = {1, 1, 1}, h[3] = {0, 0, 0};
   int off[3] = {0, 0, 0};    // first padded index the box holds along d (h on an unpadded periodic dimension)
   int ext[3] = {1, 1, 1};    // padded extent the box holds (zeros beyond it)
   long NR = 0;               // real box points
-  long NH = 0;               // half-spectrum points
+  long NH = 0, NS = 0;       // half-spectrum points, points stored (pitch included)
   FftAxis ax[3];
 };
 bool fft_make_plan(FftPlan &p, const int P[3], const int nx[3], const int h[3], const int periodic[3], int ndim,
