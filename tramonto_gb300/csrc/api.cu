@@ -188,6 +188,7 @@ struct Ctx : tgpu_ctx {
   std::vector<double2 *> d_trbox;
   std::vector<float2 *> d_trbox32;
   int fft32_tc = 0, fft32_slab = 0;
+  int adj_fft = 0;               // the adjoint's transposed sums by FP64 FFT: 0 undecided, 1 yes, -1 direct sums
   float t32_att[2][2] = {{0.f, 0.f}, {0.f, 0.f}};   // [slab context, tensor-core context][direct, FFT] ms
   long fft32_gen = -1;
   int fft32_ch = -1;
@@ -385,7 +386,7 @@ void kernel_spectrum(Ctx *c, const DevStencil &st, int side, int q, double *rbox
 {
   const double *coef = side == 0 ? st.d_coef_fwd : st.d_coef_tr;
   const int nq = side == 0 ? st.nout_fwd : st.nin_tr;
-  tgpu::launch_fft_kernel_box(st.d_off, coef, st.L, nq, q, rbox, c->fft, c->stream);
+  tgpu::launch_fft_kernel_box(st.d_off, coef, st.L, nq, q, 1, rbox, c->fft, c->stream);
   tgpu::rfft_forward_box(rbox, spec, c->fft, c->stream);
 }
 
@@ -1579,6 +1580,102 @@ void adj_conv(Ctx *c, int ch0, int nin, const DevStencil &st, const double *coef
   }
 }
 
+// Whether the adjoint's transposed sums run as FP64 FFT convolutions (3-D, one quadrature zone, no reflecting
+// boundary, whose mirrored positions are folded back by the direct sums), with the spectra built on first use.  The
+// rule compares the direct FP64 point sums with the transforms: a term and output takes 1.65e-12 s at the FP64 pipe's
+// rate, a transform 8e-12 s per half-spectrum point and log2 of the box (as fft_worth).  Binary pore 96 x 96 x 64:
+// 11.6 ms of direct sums (theta 1015 and 123, delta 844 and 208 points) against 24 transforms, 1.5 ms.  Both are FP64
+// sums; the transforms' error against 64-bit values is not the larger one (eps log2 of the box against eps times the
+// root of the number of terms).
+bool adj_use_fft(Ctx *c)
+{
+  if (c->adj_fft != 0) return c->adj_fft == 1;
+  const tgpu::DevGeom &g = c->dg;
+  c->adj_fft = -1;
+  if (g.ndim != 3 || c->nzone != 1 || has_reflect(c)) return false;
+  ensure_fft(c);
+  if (!c->fft_plan_ok) return false;
+  double terms = 0.0;
+  size_t nspec = 0;
+  for (int t = 0; t < 3; t++)
+    for (auto &st : c->sten[t]) {
+      const int nq = t == TGPU_STEN_DELTA ? 1 + g.ndim : 1;
+      if (st.L == 0) continue;
+      terms += (t == TGPU_STEN_UATT ? 1.0 : 2.0) * nq * st.L;
+      nspec += nq;
+    }
+  const double transforms = g.ncomp * (2.0 * (g.ndim + 2) + 2.0 + (g.attraction ? g.ncomp : 0));
+  const double NH = (double)c->fft.NH;
+  if (terms * (double)g.N * 1.65e-12 <= transforms * NH * std::log2((double)c->fft.NR) * 8.0e-12) return false;
+  const size_t nbox = (size_t)(g.ndim + 3 + g.ncomp);
+  size_t free_b = 0, total_b = 0;
+  ck(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
+  if ((nspec + nbox) * (size_t)c->fft.NS * sizeof(double2) + (size_t)c->fft.NR * sizeof(double) > free_b / 2) return false;
+  double *rbox = dalloc<double>((size_t)c->fft.NR);
+  for (int t = 0; t < 3; t++)
+    for (auto &st : c->sten[t]) {
+      if (st.L == 0) continue;
+      const int nq = t == TGPU_STEN_DELTA ? 1 + g.ndim : 1;
+      for (int q = 0; q < nq; q++) {
+        double2 *k = dalloc<double2>((size_t)c->fft.NS);
+        tgpu::launch_fft_kernel_box(st.d_off, t == TGPU_STEN_DELTA ? st.d_coef_adj : st.d_coef_fwd, st.L, nq, q, -1,
+                                    rbox, c->fft, c->stream);
+        tgpu::rfft_forward_box(rbox, k, c->fft, c->stream);
+        st.spec_adj.push_back(k);
+      }
+    }
+  ck(cudaStreamSynchronize(c->stream), "sync");
+  dfree(rbox);
+  c->adj_fft = 1;
+  return true;
+}
+
+// adjoint channel ch with zeros outside the mesh (the zero extension of adj_pad)
+tgpu::MapSrc adj_src(const Ctx *c, int ch)
+{
+  const tgpu::DevGeom &g = c->dg;
+  tgpu::MapSrc m;
+  m.src = c->d_adj_chan + (long)ch * g.N;
+  m.ndim = g.ndim;
+  for (int d = 0; d < 3; d++) {
+    m.nx[d] = g.nx[d];
+    m.map[d] = g.map[d];
+  }
+  m.N = g.N;
+  return m;
+}
+
+std::vector<double2 *> &adj_boxes(Ctx *c, size_t n)
+{
+  while (c->d_trbox.size() < n) c->d_trbox.push_back(dalloc<double2>((size_t)c->fft.NS));
+  return c->d_trbox;
+}
+
+// out += the transposed sums of channels chs with kernels k, by one inverse transform
+void adj_fft_in(Ctx *c, const std::vector<int> &chs, const std::vector<const double2 *> &k, double *out)
+{
+  const int n = (int)chs.size();
+  std::vector<double2 *> &b = adj_boxes(c, n + 1);
+  std::vector<tgpu::MapSrc> ms(n);
+  for (int t = 0; t < n; t++) ms[t] = adj_src(c, chs[t]);
+  tgpu::rfft_forward_mapped_batch(ms.data(), n, b.data(), c->fft, c->stream);
+  std::vector<const double2 *> a(b.begin(), b.begin() + n);
+  tgpu::rfft_inverse_products(a.data(), k.data(), n, b[n], c->fft, 1.0 / (double)c->fft.NR, out, true, c->stream);
+  c->stats.kernel_launches += 6;
+  c->stats.conv_launches++;
+}
+
+// outs[q] = the transposed sum of channel ch with kernel k[q]
+void adj_fft_out(Ctx *c, int ch, const std::vector<const double2 *> &k, double *const *outs)
+{
+  const int n = (int)k.size();
+  std::vector<double2 *> &b = adj_boxes(c, n + 1);
+  tgpu::rfft_forward_mapped(adj_src(c, ch), b[n], c->fft, c->stream);
+  tgpu::rfft_inverse_batch(b[n], k.data(), n, b.data(), c->fft, 1.0 / (double)c->fft.NR, outs, false, c->stream);
+  c->stats.kernel_launches += 6;
+  c->stats.conv_launches++;
+}
+
 void adj_pad(Ctx *c, int nch)
 {
   tgpu::launch_pad<double>(c->d_adj_chan, c->d_adj_pad, nch, c->pads.zero_ext.bulk, c->pads.zero_ext.sign,
@@ -1594,6 +1691,7 @@ void jtv_device(Ctx *c, const double *d_w_in, double *d_out)
   const long N = g.N;
   const int nd = g.ndim;
   const int cpc = nd + 2;   // channels per component: A, B[d], C
+  const bool fft = adj_use_fft(c);
   ck(cudaMemsetAsync(d_out, 0, sizeof(double) * (size_t)g.nunk * N, c->stream), "memset");
   // the averaged rows of coarsened nodes are transposed apart (at the end); the stencil rows of each
   // quadrature zone with that zone's stencils
@@ -1609,6 +1707,23 @@ void jtv_device(Ctx *c, const double *d_w_in, double *d_out)
     for (int z = 0; z < c->nzone; z++) {
       const std::vector<DevStencil> *sten = z == 0 ? c->sten : c->zsten[z];
       tgpu::launch_adj_rb_channels(d_w, c->d_adj_chan, c->stream);
+      if (fft) {
+        for (int jc = 0; jc < g.ncomp; jc++) {
+          std::vector<int> chs;
+          std::vector<const double2 *> k;
+          for (int t = 0; t < cpc; t++) {
+            chs.push_back(jc * cpc + t);
+            k.push_back(t <= nd ? sten[TGPU_STEN_DELTA][jc].spec_adj[t] : sten[TGPU_STEN_THETA][jc].spec_adj[0]);
+          }
+          if (g.attraction)
+            for (int ic = 0; ic < g.ncomp; ic++) {
+              chs.push_back(g.ncomp * cpc + ic);
+              k.push_back(sten[TGPU_STEN_UATT][ic + g.ncomp * jc].spec_adj[0]);
+            }
+          adj_fft_in(c, chs, k, d_out + (long)(g.first_rho + jc) * N);
+        }
+        continue;
+      }
       if (c->nzone > 1) tgpu::launch_zone_mask(c->d_adj_chan, nch, N, c->d_zone, z, c->stream);
       adj_pad(c, nch);
       for (int jc = 0; jc < g.ncomp; jc++) {
@@ -1638,10 +1753,21 @@ void jtv_device(Ctx *c, const double *d_w_in, double *d_out)
   // (b) rb columns <- H(n) g with g gathered from the EL rows of w by the transposed delta/theta sums
   {
     const int gst = nd + 2;   // per component: delta outputs (scalar, vector[d]) then theta
-    ck(cudaMemsetAsync(c->d_adj_g, 0, sizeof(double) * (size_t)g.ncomp * gst * N, c->stream), "memset");
+    if (!fft) ck(cudaMemsetAsync(c->d_adj_g, 0, sizeof(double) * (size_t)g.ncomp * gst * N, c->stream), "memset");
     for (int z = 0; z < c->nzone; z++) {
       const std::vector<DevStencil> *sten = z == 0 ? c->sten : c->zsten[z];
       tgpu::launch_mask_rows(c->d_adj_chan, d_w, c->d_vext, c->d_zero, g.first_rho, g.ncomp, 0, c->stream);
+      if (fft) {
+        for (int ic = 0; ic < g.ncomp; ic++) {
+          double *o[tgpu::kMaxRb];
+          for (int q = 0; q < gst; q++) o[q] = c->d_adj_g + ((long)ic * gst + q) * N;
+          std::vector<const double2 *> k(sten[TGPU_STEN_DELTA][ic].spec_adj.begin(),
+                                         sten[TGPU_STEN_DELTA][ic].spec_adj.end());
+          k.push_back(sten[TGPU_STEN_THETA][ic].spec_adj[0]);
+          adj_fft_out(c, ic, k, o);
+        }
+        continue;
+      }
       if (c->nzone > 1) tgpu::launch_zone_mask(c->d_adj_chan, g.ncomp, N, c->d_zone, z, c->stream);
       adj_pad(c, g.ncomp);
       for (int ic = 0; ic < g.ncomp; ic++) {
@@ -1870,9 +1996,20 @@ void objective_grad_device(Ctx *c, const double *d_x, int kind, int icomp, doubl
     // the other nodes' mean-field terms: d/drho_jc(j) sum_i wf_ic rho_ic(i) S_ic(i) / 2 =
     // transposed attraction sums of wf rho / 2 (the kernel stored wf rho on rho > 0 nodes)
     tgpu::launch_scale(c->d_adj_chan, c->d_adj_chan, 0.5, (long)g.ncomp * N, c->stream);
-    adj_pad(c, g.ncomp);
+    const bool fft = adj_use_fft(c);
+    if (!fft) adj_pad(c, g.ncomp);
     for (int jc = 0; jc < g.ncomp; jc++) {
       double *o[1] = {d_gx + (long)(g.first_rho + jc) * N};
+      if (fft) {
+        std::vector<int> chs;
+        std::vector<const double2 *> k;
+        for (int ic = 0; ic < g.ncomp; ic++) {
+          chs.push_back(ic);
+          k.push_back(c->sten[TGPU_STEN_UATT][ic + g.ncomp * jc].spec_adj[0]);
+        }
+        adj_fft_in(c, chs, k, o[0]);
+        continue;
+      }
       for (int ic = 0; ic < g.ncomp; ic++) {
         const DevStencil &su = c->sten[TGPU_STEN_UATT][ic + g.ncomp * jc];
         adj_conv(c, ic, 1, su, su.d_coef_fwd, o, 1);
@@ -2604,7 +2741,7 @@ int tgpu_destroy(tgpu_handle h)
             dfree(L.d_planes); dfree(L.d_lines); dfree(L.d_w); dfree(L.d_w_lo);
           }
         tgpu::tc_free_tables(st.tc);
-        for (auto *V : {&st.spec_fwd, &st.spec_tr})
+        for (auto *V : {&st.spec_fwd, &st.spec_tr, &st.spec_adj})
           for (auto &k : *V) dfree(k);
         for (auto *V : {&st.spec_fwd32, &st.spec_tr32})
           for (auto &k : *V) dfree(k);
@@ -2927,7 +3064,7 @@ int tgpu_set_fft_threshold(tgpu_handle h, int min_points)
       ck(cudaStreamSynchronize(c->stream), "sync");
       for (int t = 0; t < 3; t++)
         for (auto &st : c->sten[t]) {
-          for (auto *V : {&st.spec_fwd, &st.spec_tr}) {
+          for (auto *V : {&st.spec_fwd, &st.spec_tr, &st.spec_adj}) {
             for (auto &k : *V) dfree(k);
             V->clear();
           }
@@ -2951,6 +3088,7 @@ int tgpu_set_fft_threshold(tgpu_handle h, int min_points)
       c->fft_gen = -1;
       c->fft_plan_ok = false;
       c->spec32_built = false;
+      c->adj_fft = 0;
       c->fft32_tc = c->fft32_slab = 0;
       c->fft32_gen = -1;
     }

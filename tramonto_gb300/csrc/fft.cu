@@ -209,7 +209,7 @@ struct MappedSrc {   // the unpadded channel through the boundary maps (the padd
 };
 
 // spectral products formed by a pass as it loads its lines: value = sum_t a_t * k_t (n = 0: the input itself)
-constexpr int kMaxTerms = 6;
+constexpr int kMaxTerms = 9;   // the adjoint's channels of one density: 5 and up to 4 mean fields
 template <class C>
 struct Terms {
   const C *a[kMaxTerms];
@@ -467,16 +467,16 @@ __global__ void __launch_bounds__((x_pairs<C>() * HI + 31) / 32 * 32) k_irfft_li
   }
 }
 
-// correlation kernel of coefficient q of a stencil in the real box: coef[k * ncoef + q] added at (-offset_k) mod F
-// (offsets that wrap onto the same position add up)
+// correlation kernel of coefficient q of a stencil in the real box: coef[k * ncoef + q] added at (-dir offset_k) mod F
+// (offsets that wrap onto the same position add up); dir 1: sums over f(i + offset), -1: over f(i - offset)
 __global__ void k_fft_kernel_box(const short *__restrict__ off3, const double *__restrict__ coef, int L, int ncoef,
-                                 int q, double *__restrict__ box, int F0, int F1, int F2)
+                                 int q, int dir, double *__restrict__ box, int F0, int F1, int F2)
 {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= L) return;
-  const int x = ((-(int)off3[3 * k]) % F0 + F0) % F0;
-  const int y = ((-(int)off3[3 * k + 1]) % F1 + F1) % F1;
-  const int z = ((-(int)off3[3 * k + 2]) % F2 + F2) % F2;
+  const int x = ((-dir * (int)off3[3 * k]) % F0 + F0) % F0;
+  const int y = ((-dir * (int)off3[3 * k + 1]) % F1 + F1) % F1;
+  const int z = ((-dir * (int)off3[3 * k + 2]) % F2 + F2) % F2;
   atomicAdd(box + ((long)z * F1 + y) * F0 + x, coef[(long)k * ncoef + q]);
 }
 
@@ -920,11 +920,11 @@ void fft_pass(float2 *spec, const FftPlan &p, int d, bool inverse, cudaStream_t 
   strided_pass<float2>(spec, spec, none, p, d, inverse, s);
 }
 
-void launch_fft_kernel_box(const short *off3, const double *coef, int L, int ncoef, int q, double *box,
+void launch_fft_kernel_box(const short *off3, const double *coef, int L, int ncoef, int q, int dir, double *box,
                            const FftPlan &p, cudaStream_t s)
 {
   cudaMemsetAsync(box, 0, sizeof(double) * p.NR, s);
-  if (L > 0) k_fft_kernel_box<<<(L + 255) / 256, 256, 0, s>>>(off3, coef, L, ncoef, q, box, p.F[0], p.F[1], p.F[2]);
+  if (L > 0) k_fft_kernel_box<<<(L + 255) / 256, 256, 0, s>>>(off3, coef, L, ncoef, q, dir, box, p.F[0], p.F[1], p.F[2]);
 }
 
 void launch_to_float2(const double2 *in, float2 *out, long n, cudaStream_t s)

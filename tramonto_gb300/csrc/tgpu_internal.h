@@ -133,8 +133,8 @@ void pass_timer_collect(long *launches, double *ms_total, double *bytes_total, l
 void fft_pass(double2 *spec, const FftPlan &p, int d, bool inverse, cudaStream_t s);
 void fft_pass(float2 *spec, const FftPlan &p, int d, bool inverse, cudaStream_t s);
 void launch_to_float2(const double2 *in, float2 *out, long n, cudaStream_t s);
-// real box <- the correlation kernel of coefficient q of a stencil: coef[k * ncoef + q] added at (-offset_k) mod F
-void launch_fft_kernel_box(const short *off3, const double *coef, int L, int ncoef, int q, double *box,
+// real box <- the correlation kernel of coefficient q of a stencil: coef[k * ncoef + q] added at (-dir offset_k) mod F
+void launch_fft_kernel_box(const short *off3, const double *coef, int L, int ncoef, int q, int dir, double *box,
                            const FftPlan &p, cudaStream_t s);
 
 // Averaged rows of coarsened nodes and the prolongation onto them (coarsen.cu)
@@ -434,6 +434,7 @@ struct DevStencil {
   // FFT spectra of the correlation kernels (FP64 fills by FFT): per forward output, per transpose input;
   // FP32 copies of the forward ones for the FP32 sums (products, FP32 fills)
   std::vector<double2 *> spec_fwd, spec_tr;
+  std::vector<double2 *> spec_adj;      // of the adjoint's transposed sums (offsets negated): delta 1 + ndim, others 1
   std::vector<float2 *> spec_fwd32, spec_tr32;
   int fft32_fwd = 0, fft32_tr = 0;      // short stencils: FP32 FFT (1) or slab (-1) sums, 0 undecided
   float t32[2][2] = {{0.f, 0.f}, {0.f, 0.f}};  // [forward, transposed][direct, FFT] ms of the timing that decided
