@@ -2,7 +2,8 @@
 of first radices, the longest transform (432), lengths of one radix only, odd numbers of lines (the last complex line
 of the x passes holds one real line) and tiles with idle lines.
 
-Periodic boxes of hard spheres whose stencils reach one node, so that the transforms run on the box's own lengths.
+Periodic boxes of hard spheres whose stencils reach one node, so that the transforms run on the box's own lengths (343 has
+no two radices and is padded).
 With every sum by FFT the FP64 fill equals the direct FP64 one to 1e-12 (transform rounding ~eps log2 of the box,
 4e-15, times the sums' scale of a few, with two orders to spare) and the FP32 products the FP64 ones to 1e-5 of their
 max norms."""
@@ -12,7 +13,8 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 BOXES = [(432, 25, 9), (27, 432, 4), (24, 5, 384), (405, 18, 5), (20, 400, 3), (375, 6, 15), (9, 27, 25), (250, 10, 12),
-         (8, 324, 8), (16, 16, 160), (360, 12, 3), (5, 135, 225)]
+         (8, 324, 8), (16, 16, 160), (360, 12, 3), (5, 135, 225),
+         (70, 7, 21), (14, 98, 9), (196, 5, 105), (5, 420, 28), (343, 3, 7)]
 
 
 def problem(box):

@@ -358,15 +358,23 @@ tgpu::MapSrc map_src(const Ctx *c, int ch)
 // ---- FP64 stencil sums by FFT ----------------------------------------------------
 
 // Which stencils take the FFT in TGPU_FILL_FFT (and TGPU_FP64_FFT products): those whose direct float-float sums
-// (measured on GB300: ~5.4e-13 s per term and output) cost more than the transforms (one per coefficient plus the
-// field's; measured ~8e-12 s per half-spectrum point and log2 of the box: 0.26 ms for the 180 x 128 x 128 box of
-// the 128^3 workload), unless tgpu_set_fft_threshold fixed a length.  At 128^3 every stencil qualifies: the
-// attraction stencil (7e4 points), theta (1015) and delta (844 points, four outputs).
+// cost more than the transforms (one per coefficient plus the field's), unless tgpu_set_fft_threshold fixed a length.
+// Direct, measured on GB300: 5.4e-13 s per term and output of the 128 x 16 tiles, plus 13 us per z-plane of the
+// stencil and wave of tiles for the slabs (one CTA per SM): 81 + 5 ms for the attraction stencil at 128^3 (81), 0.5 +
+// 0.6 ms for the 844-point delta shell on 83 x 101 x 70 nodes (1.02), 0.05 + 0.2 ms for a 123-point ball on 96 x 96 x
+// 64 (0.25).  A transform: 7e-12 s per half-spectrum point and log2 of the box (0.22 ms for the 180 x 128 x 128 box).
 bool fft_worth(const Ctx *c, const DevStencil &st, int nq)
 {
   if (c->fft_min_points >= 0) return st.L >= c->fft_min_points;
+  const tgpu::DevGeom &g = c->dg;
   const double NR = (double)c->fft.NR, NH = (double)c->fft.NH;
-  return (double)st.L * (double)c->dg.N * nq * 5.4e-13 > (nq + 1) * NH * std::log2(NR) * 8.0e-12;
+  const long tiles = (long)((g.nx[0] + tgpu::kSlabTileX - 1) / tgpu::kSlabTileX) *
+                     ((g.nx[1] + tgpu::kSlabTileY - 1) / tgpu::kSlabTileY) * g.nx[2];
+  int zmax = 0;
+  for (int k = 0; k < st.L; k++) zmax = std::max(zmax, std::abs((int)st.off[(size_t)k * 3 + 2]));
+  const double direct = (double)tiles * tgpu::kSlabTileX * tgpu::kSlabTileY * st.L * 5.4e-13 +
+                        (double)((tiles + 151) / 152) * (2 * zmax + 1) * 13e-6;
+  return direct * nq > (nq + 1) * NH * std::log2(NR) * 7.0e-12;
 }
 
 // the plan's geometry: padded extents, mesh, reach, and the dimensions periodic at both ends (left unpadded)
@@ -1583,7 +1591,7 @@ void adj_conv(Ctx *c, int ch0, int nin, const DevStencil &st, const double *coef
 // Whether the adjoint's transposed sums run as FP64 FFT convolutions (3-D, one quadrature zone, no reflecting
 // boundary, whose mirrored positions are folded back by the direct sums), with the spectra built on first use.  The
 // rule compares the direct FP64 point sums with the transforms: a term and output takes 1.65e-12 s at the FP64 pipe's
-// rate, a transform 8e-12 s per half-spectrum point and log2 of the box (as fft_worth).  Binary pore 96 x 96 x 64:
+// rate, a transform 7e-12 s per half-spectrum point and log2 of the box (as fft_worth).  Binary pore 96 x 96 x 64:
 // 11.6 ms of direct sums (theta 1015 and 123, delta 844 and 208 points) against 24 transforms, 1.5 ms.  Both are FP64
 // sums; the transforms' error against 64-bit values is not the larger one (eps log2 of the box against eps times the
 // root of the number of terms).
@@ -1606,7 +1614,7 @@ bool adj_use_fft(Ctx *c)
     }
   const double transforms = g.ncomp * (2.0 * (g.ndim + 2) + 2.0 + (g.attraction ? g.ncomp : 0));
   const double NH = (double)c->fft.NH;
-  if (terms * (double)g.N * 1.65e-12 <= transforms * NH * std::log2((double)c->fft.NR) * 8.0e-12) return false;
+  if (terms * (double)g.N * 1.65e-12 <= transforms * NH * std::log2((double)c->fft.NR) * 7.0e-12) return false;
   const size_t nbox = (size_t)(g.ndim + 3 + g.ncomp);
   size_t free_b = 0, total_b = 0;
   ck(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");

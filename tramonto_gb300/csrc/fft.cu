@@ -6,7 +6,7 @@
 // any other dimension the padded channel (the field extended by the boundary rules over the stencil's reach h)
 // is transformed on a length F >= P = n + 2h, where the circular correlation equals the sum for every interior
 // output.  So the transform box is [F2][F1][F0] with F_d = n_d on periodic dimensions (when n_d is a product of
-// 2, 3 and 5) and the smallest such F_d >= P_d elsewhere; with the correlation kernel g[(-o) mod F] = c(o)
+// 2, 3, 5 and 7) and the smallest such F_d >= P_d elsewhere; with the correlation kernel g[(-o) mod F] = c(o)
 // (points that wrap onto the same position add up, as the reference folds a stencil wider than a periodic box),
 // one forward transform of the field, a product with the kernel's spectrum and one inverse transform give the
 // sum at a cost that does not depend on the stencil's length.  At 128^3 with the attraction reach of 25 nodes
@@ -59,9 +59,9 @@ __device__ __forceinline__ void with_radix(int R, F &&f)
     if constexpr (r > LO && r <= HI) f(std::integral_constant<int, r>{});          \
     break;
   switch (R) {
-    TGPU_RADIX(1) TGPU_RADIX(2) TGPU_RADIX(3) TGPU_RADIX(4) TGPU_RADIX(5) TGPU_RADIX(6) TGPU_RADIX(8) TGPU_RADIX(9)
-    TGPU_RADIX(10) TGPU_RADIX(12) TGPU_RADIX(15) TGPU_RADIX(16) TGPU_RADIX(18) TGPU_RADIX(20) TGPU_RADIX(24)
-    TGPU_RADIX(25) TGPU_RADIX(27)
+    TGPU_RADIX(1) TGPU_RADIX(2) TGPU_RADIX(3) TGPU_RADIX(4) TGPU_RADIX(5) TGPU_RADIX(6) TGPU_RADIX(7) TGPU_RADIX(8)
+    TGPU_RADIX(9) TGPU_RADIX(10) TGPU_RADIX(12) TGPU_RADIX(14) TGPU_RADIX(15) TGPU_RADIX(16) TGPU_RADIX(18)
+    TGPU_RADIX(20) TGPU_RADIX(21) TGPU_RADIX(24) TGPU_RADIX(25) TGPU_RADIX(27)
   }
 #undef TGPU_RADIX
 }
@@ -119,7 +119,8 @@ template <class T>
 struct MappedSrc {   // the unpadded channel through the boundary maps (the padded box's values, computed)
   MapSrc m;
   T lo, hi;          // the bulk values in arithmetic T (converted once)
-  explicit MappedSrc(const MapSrc &s = MapSrc()) : m(s), lo((T)s.bulk_lo), hi((T)s.bulk_hi) {}
+  MappedSrc() : lo(0), hi(0) {}
+  explicit MappedSrc(const MapSrc &s) : m(s), lo((T)s.bulk_lo), hi((T)s.bulk_hi) {}
   // the node offset and reflections of the line, or the sentinel of its first out-of-range dimension after x
   // (x still decides first)
   struct Line {
@@ -275,11 +276,13 @@ __global__ void __launch_bounds__(lines_per_cta<C>() * HI) k_fft_lines(PassBatch
           const C *a = terms.a[0] + i0, *k = terms.k[0] + i0;
 #pragma unroll
           for (int r = 0; r < R; r++) v[r] = cmul(a[r * step], __ldg(k + r * step));
-          for (int t = 1; t < terms.n; t++) {
-            a = terms.a[t] + i0;
-            k = terms.k[t] + i0;
+          if (std::is_same<C, double2>::value) {   // (FP32 sums of several products: launch_spec_terms)
+            for (int t = 1; t < terms.n; t++) {
+              a = terms.a[t] + i0;
+              k = terms.k[t] + i0;
 #pragma unroll
-            for (int r = 0; r < R; r++) v[r] = cadd(v[r], cmul(a[r * step], __ldg(k + r * step)));
+              for (int r = 0; r < R; r++) v[r] = cadd(v[r], cmul(a[r * step], __ldg(k + r * step)));
+            }
           }
         }
       }
@@ -480,15 +483,47 @@ __global__ void k_fft_kernel_box(const short *__restrict__ off3, const double *_
   atomicAdd(box + ((long)z * F1 + y) * F0 + x, coef[(long)k * ncoef + q]);
 }
 
-// the products of `t` as a spectrum (a box without y or z passes to form them in)
-template <class C>
-__global__ void k_spec_terms(Terms<C> t, C *__restrict__ out, long n)
+// the products of `t` as a spectrum, two points per thread and iteration, every term's loads issued before the sums
+template <int N, class C>
+__global__ void __launch_bounds__(256) k_spec_terms(Terms<C> t, C *__restrict__ out, long n)
 {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    C v = cmul(t.a[0][i], t.k[0][i]);
-    for (int j = 1; j < t.n; j++) v = cadd(v, cmul(t.a[j][i], t.k[j][i]));
-    out[i] = v;
+  for (long i = 2 * (blockIdx.x * (long)blockDim.x + threadIdx.x); i < n; i += 2L * gridDim.x * blockDim.x) {
+    C a[N][2], k[N][2];
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+      if constexpr (std::is_same<C, float2>::value) {   // (spectra are 256-byte aligned and n is even)
+        const float4 va = *reinterpret_cast<const float4 *>(t.a[j] + i), vk = *reinterpret_cast<const float4 *>(t.k[j] + i);
+        a[j][0] = C{va.x, va.y};
+        a[j][1] = C{va.z, va.w};
+        k[j][0] = C{vk.x, vk.y};
+        k[j][1] = C{vk.z, vk.w};
+      } else {
+        for (int h = 0; h < 2; h++) {
+          a[j][h] = t.a[j][i + h];
+          k[j][h] = t.k[j][i + h];
+        }
+      }
+    }
+    C v[2] = {cmul(a[0][0], k[0][0]), cmul(a[0][1], k[0][1])};
+#pragma unroll
+    for (int j = 1; j < N; j++)
+      for (int h = 0; h < 2; h++) v[h] = cadd(v[h], cmul(a[j][h], k[j][h]));
+    out[i] = v[0];
+    out[i + 1] = v[1];
   }
+}
+
+template <class C>
+void launch_spec_terms(const Terms<C> &t, C *out, long n, cudaStream_t s)
+{
+  const int grid = (int)std::min<long>((n / 2 + 255) / 256, 152L * 8);
+  switch (t.n) {
+#define TGPU_TERMS(N) case N: k_spec_terms<N, C><<<grid, 256, 0, s>>>(t, out, n); break;
+    TGPU_TERMS(1) TGPU_TERMS(2) TGPU_TERMS(3) TGPU_TERMS(4) TGPU_TERMS(5) TGPU_TERMS(6) TGPU_TERMS(7) TGPU_TERMS(8)
+    TGPU_TERMS(9)
+#undef TGPU_TERMS
+  }
+  static_assert(kMaxTerms == 9, "a case per number of terms");
 }
 
 __global__ void k_to_float2(const double2 *__restrict__ in, float2 *__restrict__ out, long n)
@@ -499,19 +534,12 @@ __global__ void k_to_float2(const double2 *__restrict__ in, float2 *__restrict__
 
 int grid_for(long n) { return (int)std::min<long>((n + 255) / 256, 152L * 16); }
 
-bool smooth(int F)
-{
-  int m = F;
-  for (int r : {2, 3, 5})
-    while (m % r == 0) m /= r;
-  return m == 1;
-}
-
-// the two radices of a length: the factors nearest each other among the register DFT lengths
+// the two radices of a length: the factors nearest each other among the register DFT lengths (every product of 2, 3,
+// 5 and 7 up to 432 but 245, 343 and 392 has them)
 bool radices_of(int F, int &R1, int &R2)
 {
-  static const int kRadix[] = {1, 2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 20, 24, 25, 27};
-  if (F < 1 || F > kFftMaxN || !smooth(F)) return false;
+  static const int kRadix[] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 15, 16, 18, 20, 21, 24, 25, 27};
+  if (F < 1 || F > kFftMaxN) return false;
   for (int a : kRadix)
     for (int b : kRadix)
       if (b <= a && a * b == F) {
@@ -690,13 +718,15 @@ void rfft_inverse_impl(const Terms<C> &terms, C *spec, const FftPlan &p, double 
                        bool accumulate, cudaStream_t s)
 {
   const Terms<C> none{};
-  bool pending = true;   // products not formed yet
+  // A sum of several FP32 products is formed by a pass of its own (five terms at 128^3: 24 + 9 us; 70 us inside the
+  // z pass, whose threads wait for each term in turn).  FP64 sums stay in the z pass, bound by their arithmetic there.
+  bool pending = !(std::is_same<C, float2>::value && terms.n > 1) && p.F[2] * p.F[1] > 1;   // products not formed yet
+  if (!pending) launch_spec_terms<C>(terms, spec, p.NS, s);
   for (int d = 2; d >= 1; d--) {
     if (p.F[d] == 1) continue;
     strided_pass<C>(spec, spec, pending ? terms : none, p, d, true, s);
     pending = false;
   }
-  if (pending) k_spec_terms<C><<<grid_for(p.NS), 256, 0, s>>>(terms, spec, p.NS);
   OutBatch<C> ob{};
   ob.spec[0] = spec;
   ob.out[0] = out;
@@ -745,7 +775,7 @@ void rfft_inverse_batch_impl(const C *a, const C *const *k, int nb, C *const *wo
     pending = false;
   }
   if (pending)
-    for (int b = 0; b < nb; b++) k_spec_terms<C><<<grid_for(p.NS), 256, 0, s>>>(pb.terms[b], work[b], p.NS);
+    for (int b = 0; b < nb; b++) launch_spec_terms<C>(pb.terms[b], work[b], p.NS, s);
   inverse_x<C>(ob, nb, p, scale, accumulate, s);
 }
 
@@ -773,8 +803,8 @@ bool fft_make_plan(FftPlan &p, const int P[3], const int nx[3], const int h[3], 
       p.ext[d] = nx[d];
     } else {
       int F = P[d];
-      while (F <= kFftMaxN && !smooth(F)) F++;
-      if (!radices_of(F, a.R1, a.R2)) return false;
+      while (F <= kFftMaxN && !radices_of(F, a.R1, a.R2)) F++;
+      if (F > kFftMaxN) return false;
       p.F[d] = F;
       p.off[d] = 0;
       p.ext[d] = P[d];

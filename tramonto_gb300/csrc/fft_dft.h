@@ -195,6 +195,25 @@ __device__ __forceinline__ void run(C *v)
     v[4] = sub_mi<INV, C>(m1, n1);
     v[2] = add_mi<INV, C>(m2, n2);
     v[3] = sub_mi<INV, C>(m2, n2);
+  } else if constexpr (R == 7) {
+    // with a_k = v_k + v_7-k, b_k = v_k - v_7-k: y_k, y_7-k = v0 + sum_j cos(2 pi jk / 7) a_j -/+ i sum_j sin(2 pi jk / 7) b_j
+    const T c1 = (T)0.62348980185873353053, c2 = (T)-0.22252093395631440429, c3 = (T)-0.90096886790241912624;
+    const T s1 = (T)0.78183148246802980871, s2 = (T)0.97492791218182360702, s3 = (T)0.43388373911755812048;
+    const C a1 = cadd(v[1], v[6]), a2 = cadd(v[2], v[5]), a3 = cadd(v[3], v[4]);
+    const C b1 = csub(v[1], v[6]), b2 = csub(v[2], v[5]), b3 = csub(v[3], v[4]);
+    const C m1 = C{v[0].x + c1 * a1.x + c2 * a2.x + c3 * a3.x, v[0].y + c1 * a1.y + c2 * a2.y + c3 * a3.y};
+    const C m2 = C{v[0].x + c2 * a1.x + c3 * a2.x + c1 * a3.x, v[0].y + c2 * a1.y + c3 * a2.y + c1 * a3.y};
+    const C m3 = C{v[0].x + c3 * a1.x + c1 * a2.x + c2 * a3.x, v[0].y + c3 * a1.y + c1 * a2.y + c2 * a3.y};
+    const C n1 = C{s1 * b1.x + s2 * b2.x + s3 * b3.x, s1 * b1.y + s2 * b2.y + s3 * b3.y};
+    const C n2 = C{s2 * b1.x - s3 * b2.x - s1 * b3.x, s2 * b1.y - s3 * b2.y - s1 * b3.y};
+    const C n3 = C{s3 * b1.x - s1 * b2.x + s2 * b3.x, s3 * b1.y - s1 * b2.y + s2 * b3.y};
+    v[0] = C{v[0].x + a1.x + a2.x + a3.x, v[0].y + a1.y + a2.y + a3.y};
+    v[1] = add_mi<INV, C>(m1, n1);
+    v[6] = sub_mi<INV, C>(m1, n1);
+    v[2] = add_mi<INV, C>(m2, n2);
+    v[5] = sub_mi<INV, C>(m2, n2);
+    v[3] = add_mi<INV, C>(m3, n3);
+    v[4] = sub_mi<INV, C>(m3, n3);
   } else if constexpr (R == 8) {
     C e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
     run<4, INV, C>(e);
@@ -217,6 +236,10 @@ __device__ __forceinline__ void run(C *v)
     prime_factor<5, 2, INV, C>(v);
   } else if constexpr (R == 12) {
     prime_factor<4, 3, INV, C>(v);
+  } else if constexpr (R == 14) {
+    prime_factor<7, 2, INV, C>(v);
+  } else if constexpr (R == 21) {
+    prime_factor<7, 3, INV, C>(v);
   } else if constexpr (R == 15) {
     prime_factor<5, 3, INV, C>(v);
   } else if constexpr (R == 18) {
