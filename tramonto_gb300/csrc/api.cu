@@ -211,6 +211,12 @@ struct Ctx : tgpu_ctx {
   // there while such a product runs
   bool store32 = false;
   float *d_conv32 = nullptr, *d_chan32 = nullptr, *d_tr32 = nullptr, *d_ymf32 = nullptr, *d_hcoef32 = nullptr;
+  // one-launch GMRES of 1-D problems: workspace (for line_kdim steps), device limits
+  double *d_line_R = nullptr, *d_line_y = nullptr;
+  signed char *d_line_kind = nullptr;
+  unsigned *d_line_bar = nullptr;
+  tgpu::LineResult *d_line_res = nullptr, *h_line_res = nullptr;
+  int line_kdim = 0, nsm = 0, smem_max = 0;
   double *d_inv32 = nullptr;           // 1/rho of the state's Euler-Lagrange rows, and their kinds (k_row_info32)
   signed char *d_kind32 = nullptr;
   int hcoef32_form = -1;
@@ -1306,6 +1312,88 @@ void red_to_host(Ctx *c, int n)
 void tc_check(Ctx *c);
 void schur_t_device(Ctx *c, const double *d_v2, double *d_y2);
 
+void ensure_adjoint(Ctx *c);
+bool has_reflect(const Ctx *c);
+
+// Whether a cycle of kdim steps runs as one cooperative launch (gmres_line.h): 1-D, one quadrature zone, no hard-wall
+// corrections, coarsened nodes or (transposed) reflecting boundaries, at most 64 nodes per SM, and windows that fit in
+// shared memory.  Measured per iteration, launches and host wait against the one launch: HS wall, 2001 nodes, FP64 210
+// -> 43 us; slit pore, 1487 nodes, FP32 products 185 -> 38 us; its adjoint at 801 nodes 400 -> 36 us.
+int line_per(Ctx *c, int kdim)
+{
+  const tgpu::DevGeom &g = c->dg;
+  if (g.ndim != 1 || c->nzone != 1 || c->coarse() || !c->hw_targets.empty()) return 0;
+  if (c->gmres_transpose && has_reflect(c)) return 0;
+  if (c->nsm == 0) {
+    int coop = 0, dev = c->device;
+    ck(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev), "attribute");
+    ck(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, dev), "attribute");
+    ck(cudaDeviceGetAttribute(&c->smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "attribute");
+    if (!coop) c->nsm = 1;
+  }
+  const int per = tgpu::gmres_line_per(g.N, c->nsm);
+  const bool f32 = prod_f32(c) && !c->gmres_transpose;
+  if (per == 0 || (long)tgpu::gmres_line_smem(g.ncomp, c->gmres_transpose, f32, kdim, per, g.h[0]) > c->smem_max - 1024)
+    return 0;
+  if (2L * (kdim + 2) * c->nsm >= tgpu::kPartialWords) return 0;
+  return per;
+}
+
+tgpu::LineResult gmres_line(Ctx *c, int per, const double *d_rhs, double *d_x2, double tol, int kdim, int m)
+{
+  const tgpu::DevGeom &g = c->dg;
+  if (c->gmres_transpose) ensure_adjoint(c);
+  if (c->line_kdim < kdim) {
+    dfree(c->d_line_R);
+    dfree(c->d_line_y);
+    c->d_line_R = dalloc<double>((size_t)kdim * (kdim + 1));
+    c->d_line_y = dalloc<double>(kdim);
+    c->line_kdim = kdim;
+  }
+  if (!c->d_line_kind) {
+    c->d_line_kind = dalloc<signed char>(c->n2);
+    c->d_line_bar = dalloc<unsigned>(2);
+    c->d_line_res = dalloc<tgpu::LineResult>(1);
+    ck(cudaMallocHost(&c->h_line_res, sizeof(tgpu::LineResult) + 2 * sizeof(unsigned)), "cudaMallocHost");
+  }
+  tgpu::LineCall q{};
+  q.sten = c->sten;
+  q.ncomp = g.ncomp;
+  q.attraction = g.attraction;
+  q.per = per;
+  q.h = g.h[0];
+  q.kdim = kdim;
+  q.m = m;
+  q.transpose = c->gmres_transpose;
+  q.f32 = prod_f32(c) && !c->gmres_transpose;
+  q.N = g.N;
+  q.tol = tol;
+  q.x = c->d_x;
+  q.vext = c->d_vext;
+  q.hcoef = hess_coef(c);
+  q.rhs = d_rhs;
+  q.zero = c->d_zero;
+  q.V = c->d_V;
+  q.part = c->d_partial;
+  q.R = c->d_line_R;
+  q.y = c->d_line_y;
+  q.xout = d_x2;
+  q.chan = c->gmres_transpose ? (void *)c->d_adj_chan : (void *)c->d_chan;
+  q.kind = c->d_line_kind;
+  q.bar = c->d_line_bar;
+  q.res = c->d_line_res;
+  ck(cudaMemsetAsync(c->d_line_bar, 0, 2 * sizeof(unsigned), c->stream), "memset");
+  ck(tgpu::launch_gmres_line(q, c->stream), "one-launch GMRES");
+  unsigned *h_bar = reinterpret_cast<unsigned *>(c->h_line_res + 1);
+  ck(cudaMemcpyAsync(c->h_line_res, c->d_line_res, sizeof(tgpu::LineResult), cudaMemcpyDeviceToHost, c->stream), "d2h");
+  ck(cudaMemcpyAsync(h_bar, c->d_line_bar, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream), "d2h");
+  ck(cudaStreamSynchronize(c->stream), "sync");
+  if (h_bar[1]) throw Error(TGPU_ERR_CUDA, "one-launch GMRES: a bounded wait ran out");
+  c->stats.kernel_launches++;
+  c->stats.schur_applies += c->h_line_res->its;
+  return *c->h_line_res;
+}
+
 int gmres(Ctx *c, const double *d_rhs, double *d_x2, double tol, int maxit, int *iters, double *relres)
 {
   const long n = c->n2;
@@ -1313,22 +1401,36 @@ int gmres(Ctx *c, const double *d_rhs, double *d_x2, double tol, int maxit, int 
   const int kdim = std::max(1, std::min(maxit, 500));
   ensure_krylov(c, kdim);
   double *V = c->d_V;
-  ck(cudaMemsetAsync(d_x2, 0, sizeof(double) * n, c->stream), "memset");
-  // r0 = M^-1 b
-  tgpu::launch_precond(c->d_x, c->d_vext, c->d_zero, d_rhs, c->d_gt, c->stream);
-  tgpu::launch_norm2(c->d_gt, n, c->d_partial, nb, c->d_red, c->stream);
-  red_to_host(c, 1);
-  const double r0 = std::sqrt(c->h_red[0]);
-  *iters = 0;
-  *relres = 0.0;
-  if (!(r0 > 0.0)) {
-    if (!std::isfinite(r0)) throw Error(TGPU_ERR_NONFINITE, "non-finite right-hand side in the Schur solve");
-    return TGPU_OK;
-  }
   int it = 0;
-  double rel = 1.0;
-  std::vector<double> H((size_t)(kdim + 1) * kdim), cs(kdim), sn(kdim), gv(kdim + 1), y(kdim);
+  double rel = 1.0, r0 = 0.0;
   bool first = true;
+  if (const int per = maxit > 0 ? line_per(c, kdim) : 0) {   // the first cycle in one launch; restarts (rare) below
+    const tgpu::LineResult r = gmres_line(c, per, d_rhs, d_x2, tol, kdim, kdim);
+    *iters = r.its;
+    *relres = r.rel;
+    if (!std::isfinite(r.r0)) throw Error(TGPU_ERR_NONFINITE, "non-finite right-hand side in the Schur solve");
+    if (!(r.r0 > 0.0)) return TGPU_OK;
+    if (r.status != 0) throw Error(TGPU_ERR_NONFINITE, "non-finite Krylov vector in the Schur solve");
+    if (r.rel < tol || r.its >= maxit) return r.rel < tol ? TGPU_OK : TGPU_ERR_NOCONV;
+    it = r.its;
+    rel = r.rel;
+    r0 = r.r0;
+    first = false;
+  } else {
+    ck(cudaMemsetAsync(d_x2, 0, sizeof(double) * n, c->stream), "memset");
+    // r0 = M^-1 b
+    tgpu::launch_precond(c->d_x, c->d_vext, c->d_zero, d_rhs, c->d_gt, c->stream);
+    tgpu::launch_norm2(c->d_gt, n, c->d_partial, nb, c->d_red, c->stream);
+    red_to_host(c, 1);
+    r0 = std::sqrt(c->h_red[0]);
+    *iters = 0;
+    *relres = 0.0;
+    if (!(r0 > 0.0)) {
+      if (!std::isfinite(r0)) throw Error(TGPU_ERR_NONFINITE, "non-finite right-hand side in the Schur solve");
+      return TGPU_OK;
+    }
+  }
+  std::vector<double> H((size_t)(kdim + 1) * kdim), cs(kdim), sn(kdim), gv(kdim + 1), y(kdim);
   while (it < maxit) {
     double beta;
     if (first) {
@@ -2771,6 +2873,8 @@ int tgpu_destroy(tgpu_handle h)
     dfree(c->cr.d_pptr); dfree(c->cr.d_pcol); dfree(c->cr.d_pw); dfree(c->cr.d_kind); dfree(c->d_rowkind);
     dfree(c->d_conv32); dfree(c->d_chan32); dfree(c->d_tr32); dfree(c->d_ymf32); dfree(c->d_hcoef32);
     dfree(c->d_inv32); dfree(c->d_kind32);
+    dfree(c->d_line_R); dfree(c->d_line_y); dfree(c->d_line_kind); dfree(c->d_line_bar); dfree(c->d_line_res);
+    if (c->h_line_res) cudaFreeHost(c->h_line_res);
     for (int d = 0; d < 3; d++) dfree(c->d_map[d]);
     tgpu::tc_free_slab(c->tcslab);
     dfree(c->d_vext); dfree(c->d_zero); dfree(c->d_bnodes); dfree(c->d_fmask); dfree(c->d_hw_targets);

@@ -17,6 +17,7 @@
 //                    local Hessian that the reference spreads over d2phi_drb2_* per stencil
 //                    point (src/dft_physics_FMT1.c:79-168, src/dft_physics_FMT3.c:101-265)
 //   k_newton_*       update_solution                            src/dft_newton.c:266-381
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 
@@ -681,12 +682,12 @@ __device__ __forceinline__ void fmt_hess_apply(const double *n, const double *y,
 // H y at node i from the state x, with the node's Hessian scalars from coef ([kHessCoef][N], the state's, see
 // k_hess_coef) when given: the products of one Newton state then skip the FP64 evaluation of f(n3), g(n2, V2)
 __device__ __forceinline__ void hess_apply_node(const double *x, const double *coef, long i, const double *y,
-                                                double *z)
+                                                double *z, bool transpose = false)
 {
   double n[kMaxRb];
   load_n(x, i, n);
   if (!coef) {
-    fmt_hess_apply(n, y, z);
+    fmt_hess_apply(n, y, z, transpose);
     return;
   }
   const long N = c_g.N;
@@ -703,7 +704,7 @@ __device__ __forceinline__ void hess_apply_node(const double *x, const double *c
   c.g2vc_f = coef[9 * N + i];
   c.gvv = coef[10 * N + i];
   c.gvv_out = coef[11 * N + i];
-  fmt_hess_apply_coef(c, n, y, z, c_g.ndim, false);
+  fmt_hess_apply_coef(c, n, y, z, c_g.ndim, transpose);
 }
 
 // the same in arithmetic T from the state's Hessian scalars (coef must be given)
@@ -2199,5 +2200,7 @@ void launch_vext_sens(const double *lam, const double *gv, const double *vext, c
 {
   k_vext_sens<<<1184, kThreads, 0, s>>>(lam, gv, vext, zero, out);
 }
+
+#include "gmres_line.h"
 
 }  // namespace tgpu

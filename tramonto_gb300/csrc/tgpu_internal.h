@@ -604,6 +604,29 @@ void launch_check_finite(const double *x, long n, double *partial, int nblocks, 
 
 int reduce_blocks(long n);
 
+// GMRES of a 1-D problem in one cooperative launch (gmres_line.h)
+struct LineResult {
+  int status, its;      // status 1: a non-finite norm
+  double r0, rel;       // |M^-1 b|, the last residual estimate over it
+};
+struct LineCall {
+  const std::vector<DevStencil> *sten;   // [3]
+  int ncomp, attraction, per, h, kdim, m;
+  bool transpose, f32;
+  long N;
+  double tol;
+  const double *x, *vext, *hcoef, *rhs;
+  const signed char *zero;
+  double *V, *part, *R, *y, *xout;
+  void *chan;
+  signed char *kind;
+  unsigned *bar;        // two words, zero before the launch; the second is set when a barrier gave up
+  LineResult *res;
+};
+int gmres_line_per(long N, int nsm);   // nodes per CTA, 0: the mesh is too large
+size_t gmres_line_smem(int nc, bool tr, bool f32, int kdim, int per, int h);
+cudaError_t launch_gmres_line(const LineCall &q, cudaStream_t s);
+
 // the n-point Gauss-Legendre rule mapped to [0,1] (nodes ascending, weights summing to 1; stencils.cu)
 void gauss_rule01(int n, double *x, double *w);
 
