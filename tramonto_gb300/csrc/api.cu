@@ -410,11 +410,12 @@ void ensure_fft(Ctx *c)
   if (c->fft_state != 0) return;
   c->fft_state = -1;
   const tgpu::DevGeom &dg = c->dg;
-  if (dg.ndim != 3) return;
+  if (dg.ndim < 2) return;
   int P[3], nx[3], h[3], per[3];
   plan_geometry_args(c, P, nx, h, per);
   if (!tgpu::fft_make_plan(c->fft, P, nx, h, per, dg.ndim, c->stream)) return;
   c->fft_plan_ok = true;
+  if (dg.ndim != 3) return;   // in 2-D the accurate fills keep the direct FP64 sums
   const long NH = c->fft.NS, NR = c->fft.NR;   // stored half-spectrum points
   // device memory: three work spectra and one spectrum per stencil coefficient
   size_t nspec = 0;
@@ -517,10 +518,10 @@ std::vector<double2 *> &tr_boxes<double2>(Ctx *c) { return c->d_trbox; }
 template <>
 std::vector<float2 *> &tr_boxes<float2>(Ctx *c) { return c->d_trbox32; }
 
-// transposed sum: out += the inverse of sum_t (spectrum of channel chs[t]) * kern[t], over channels of the last
+// transposed sum: out (+)= the inverse of sum_t (spectrum of channel chs[t]) * kern[t], over channels of the last
 // pad(), in one inverse transform
 template <class C>
-void fft_tr_sum(Ctx *c, const int *chs, const C *const *kern, int n, double *out)
+void fft_tr_sum(Ctx *c, const int *chs, const C *const *kern, int n, double *out, bool accumulate = true)
 {
   if (n > tgpu::fft_max_terms()) throw Error(TGPU_ERR_UNSUPPORTED, "too many channels for one FFT transposed sum");
   std::vector<C *> &boxes = tr_boxes<C>(c);
@@ -537,13 +538,13 @@ void fft_tr_sum(Ctx *c, const int *chs, const C *const *kern, int n, double *out
   if constexpr (std::is_same<C, float2>::value) {
     if (c->store32) {   // the FP32 shadow of the transposed-sum output
       tgpu::rfft_inverse_products(a.data(), kern, n, work, c->fft, 1.0 / (double)c->fft.NR,
-                                  c->d_tr32 + (out - c->d_tr), true, c->stream);
+                                  c->d_tr32 + (out - c->d_tr), accumulate, c->stream);
       c->stats.kernel_launches += 3;
       c->stats.conv_launches++;
       return;
     }
   }
-  tgpu::rfft_inverse_products(a.data(), kern, n, work, c->fft, 1.0 / (double)c->fft.NR, out, true, c->stream);
+  tgpu::rfft_inverse_products(a.data(), kern, n, work, c->fft, 1.0 / (double)c->fft.NR, out, accumulate, c->stream);
   c->stats.kernel_launches += 3;
   c->stats.conv_launches++;
 }
@@ -680,10 +681,10 @@ void conv(Ctx *c, int ch0, int nin, const DevStencil &st, bool tr, double *const
   }
   if (!f32)
     tgpu::launch_conv<double>(c->d_pad + (long)ch0 * NP, NP, nin, st.d_loff, tr ? st.d_coef_tr : st.d_coef_fwd, st.L,
-                              outs, nout, true, c->dg.N, c->stream);
+                              outs, nout, true, c->dg.N, c->dg.ndim, c->stream);
   else
     tgpu::launch_conv<float>(c->d_pad32 + (long)ch0 * NP, NP, nin, st.d_loff, tr ? st.d_coef_tr32 : st.d_coef_fwd32,
-                             st.L, outs, nout, true, c->dg.N, c->stream);
+                             st.L, outs, nout, true, c->dg.N, c->dg.ndim, c->stream);
   c->stats.conv_launches++;
   c->stats.kernel_launches++;
 }
@@ -757,9 +758,32 @@ void decide_fft32_sten(Ctx *c, DevStencil &st, bool tr, int ch0, int nin, int no
   st.t32[tr ? 1 : 0][1] = 0.5f * t_fft;
 }
 
+// whether every forward sum of density jc takes the FFT (FP32 sums, or the FP64-accurate ones)
+bool fwd_all_fft(const Ctx *c, int jc, bool f32)
+{
+  const tgpu::DevGeom &g = c->dg;
+  const DevStencil &sth = c->sten[TGPU_STEN_THETA][jc], &sde = c->sten[TGPU_STEN_DELTA][jc];
+  const int nde = (g.single_size ? 1 : 3) + (g.single_size ? 1 : 2) * g.ndim;
+  bool all;
+  if (f32) {
+    if (!c->spec32_built) return false;
+    all = use_fft32(c, sth, false, 1, 1) && use_fft32(c, sde, false, 1, nde);
+  } else {
+    if (!c->fft_on || c->fft_state != 1) return false;
+    all = sth.spec_fwd.size() == 1 && (int)sde.spec_fwd.size() == nde;
+  }
+  if (g.attraction)
+    for (int ic = 0; ic < g.ncomp; ic++) {
+      const DevStencil &su = c->sten[TGPU_STEN_UATT][ic + g.ncomp * jc];
+      all = all && (f32 ? use_fft32(c, su, false, 1, 1) : su.spec_fwd.size() == 1);
+    }
+  return all;
+}
+
 // Weighted-density (and mean-field) sums of the padded density channels with one zone's stencils
-// into out (rows as d_conv)
-void forward_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, bool f32)
+// into out (rows as d_conv); fresh: the rows hold nothing yet and every sum takes the FFT, the first density's sums
+// are written instead of added
+void forward_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, bool f32, bool fresh = false)
 {
   const tgpu::DevGeom &g = c->dg;
   const long N = g.N;
@@ -775,72 +799,44 @@ void forward_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, boo
     for (int d = 0; d < nd; d++) o_de.push_back(out + (long)(4 + d) * N);
     if (!g.single_size)
       for (int d = 0; d < nd; d++) o_de.push_back(out + (long)(4 + nd + d) * N);
-    // every sum of this density by FFT (FP64 accurate fills, or FP32): all their inverse transforms in one launch
-    // per pass
-    if (!f32 && sten == c->sten && c->fft_on && c->fft_state == 1) {
-      const DevStencil &sth = sten[TGPU_STEN_THETA][jc], &sde = sten[TGPU_STEN_DELTA][jc];
-      bool all = sth.spec_fwd.size() == 1 && sde.spec_fwd.size() == o_de.size();
+    // every sum of this density by FFT: all their inverse transforms in one launch per pass
+    if (sten == c->sten && fwd_all_fft(c, jc, f32)) {
+      const bool acc = !(fresh && jc == 0);
+      std::vector<const double2 *> ks;
+      std::vector<const float2 *> ks32;
+      std::vector<double *> os;
+      auto add = [&](const DevStencil &st, int q, double *o) {
+        if (f32) ks32.push_back(st.spec_fwd32[q]);
+        else ks.push_back(st.spec_fwd[q]);
+        os.push_back(o);
+      };
+      add(sten[TGPU_STEN_THETA][jc], 0, out);
+      for (size_t q = 0; q < o_de.size(); q++) add(sten[TGPU_STEN_DELTA][jc], (int)q, o_de[q]);
       if (g.attraction)
-        for (int ic = 0; ic < g.ncomp; ic++) all = all && sten[TGPU_STEN_UATT][ic + g.ncomp * jc].spec_fwd.size() == 1;
-      if (all) {
-        std::vector<const double2 *> ks;
-        std::vector<double *> os;
-        ks.push_back(sth.spec_fwd[0]);
-        os.push_back(out);
-        for (size_t q = 0; q < o_de.size(); q++) {
-          ks.push_back(sde.spec_fwd[q]);
-          os.push_back(o_de[q]);
-        }
-        if (g.attraction)
-          for (int ic = 0; ic < g.ncomp; ic++) {
-            ks.push_back(sten[TGPU_STEN_UATT][ic + g.ncomp * jc].spec_fwd[0]);
-            os.push_back(out + (long)(g.nrb + ic) * N);
-          }
-        const double2 *F = fft_channel(c, jc);
-        std::vector<double2 *> &work = tr_boxes<double2>(c);
-        while (work.size() < ks.size()) work.push_back(dalloc<double2>((size_t)c->fft.NS));
-        tgpu::rfft_inverse_batch(F, ks.data(), (int)ks.size(), work.data(), c->fft, 1.0 / (double)c->fft.NR,
-                                 os.data(), true, c->stream);
-        c->stats.kernel_launches += 3 * ((ks.size() + tgpu::fft_max_batch() - 1) / tgpu::fft_max_batch());
-        c->stats.conv_launches++;
-        continue;
-      }
-    }
-    if (f32 && sten == c->sten && c->spec32_built) {
-      const DevStencil &sth = sten[TGPU_STEN_THETA][jc], &sde = sten[TGPU_STEN_DELTA][jc];
-      bool all = use_fft32(c, sth, false, 1, 1) && use_fft32(c, sde, false, 1, (int)o_de.size());
-      if (g.attraction)
-        for (int ic = 0; ic < g.ncomp; ic++) all = all && use_fft32(c, sten[TGPU_STEN_UATT][ic + g.ncomp * jc], false, 1, 1);
-      if (all) {
-        std::vector<const float2 *> ks;
-        std::vector<double *> os;
-        ks.push_back(sth.spec_fwd32[0]);
-        os.push_back(out);
-        for (size_t q = 0; q < o_de.size(); q++) {
-          ks.push_back(sde.spec_fwd32[q]);
-          os.push_back(o_de[q]);
-        }
-        if (g.attraction)
-          for (int ic = 0; ic < g.ncomp; ic++) {
-            ks.push_back(sten[TGPU_STEN_UATT][ic + g.ncomp * jc].spec_fwd32[0]);
-            os.push_back(out + (long)(g.nrb + ic) * N);
-          }
+        for (int ic = 0; ic < g.ncomp; ic++)
+          add(sten[TGPU_STEN_UATT][ic + g.ncomp * jc], 0, out + (long)(g.nrb + ic) * N);
+      const int n = (int)os.size();
+      const double scale = 1.0 / (double)c->fft.NR;
+      if (f32) {
         const float2 *F = fft_channel32(c, jc);
         std::vector<float2 *> &work = tr_boxes<float2>(c);
-        while (work.size() < ks.size()) work.push_back(dalloc<float2>((size_t)c->fft.NS));
+        while ((int)work.size() < n) work.push_back(dalloc<float2>((size_t)c->fft.NS));
         if (c->store32) {   // the FP32 shadows of the sums
           std::vector<float *> os32;
           for (double *o : os) os32.push_back(c->d_conv32 + (o - c->d_conv));
-          tgpu::rfft_inverse_batch(F, ks.data(), (int)ks.size(), work.data(), c->fft, 1.0 / (double)c->fft.NR,
-                                   os32.data(), true, c->stream);
+          tgpu::rfft_inverse_batch(F, ks32.data(), n, work.data(), c->fft, scale, os32.data(), acc, c->stream);
         } else {
-          tgpu::rfft_inverse_batch(F, ks.data(), (int)ks.size(), work.data(), c->fft, 1.0 / (double)c->fft.NR,
-                                   os.data(), true, c->stream);
+          tgpu::rfft_inverse_batch(F, ks32.data(), n, work.data(), c->fft, scale, os.data(), acc, c->stream);
         }
-        c->stats.kernel_launches += 3 * ((ks.size() + tgpu::fft_max_batch() - 1) / tgpu::fft_max_batch());
-        c->stats.conv_launches++;
-        continue;
+      } else {
+        const double2 *F = fft_channel(c, jc);
+        std::vector<double2 *> &work = tr_boxes<double2>(c);
+        while ((int)work.size() < n) work.push_back(dalloc<double2>((size_t)c->fft.NS));
+        tgpu::rfft_inverse_batch(F, ks.data(), n, work.data(), c->fft, scale, os.data(), acc, c->stream);
       }
+      c->stats.kernel_launches += 3 * ((n + tgpu::fft_max_batch() - 1) / tgpu::fft_max_batch());
+      c->stats.conv_launches++;
+      continue;
     }
     if (c->store32) throw Error(TGPU_ERR_STATE, "an FP32-storage product needs a direct stencil sum");
     conv(c, jc, 1, sten[TGPU_STEN_THETA][jc], false, o_th, 1, f32);
@@ -860,18 +856,21 @@ void forward_pass(Ctx *c, const double *field, const PadParams &pp, bool f32, bo
   const tgpu::DevGeom &g = c->dg;
   const long N = g.N;
   const size_t nrows = (size_t)(g.nrb + g.ncomp);
-  if (zero_first) {
-    if (c->store32) ck(cudaMemsetAsync(c->d_conv32, 0, sizeof(float) * nrows * N, c->stream), "memset");
-    else ck(cudaMemsetAsync(c->d_conv, 0, sizeof(double) * nrows * N, c->stream), "memset");
-  }
   pad(c, field, pp, f32);
-  if (f32 && g.attraction && g.ndim == 3) decide_fft32(c);
-  if (f32 && g.ndim == 3)
+  if (f32 && g.attraction && g.ndim >= 2) decide_fft32(c);
+  if (f32 && g.ndim >= 2)
     for (int jc = 0; jc < g.ncomp; jc++) {
       decide_fft32_sten(c, c->sten[TGPU_STEN_THETA][jc], false, jc, 1, 1);
       decide_fft32_sten(c, c->sten[TGPU_STEN_DELTA][jc], false, jc, 1, c->sten[TGPU_STEN_DELTA][jc].nout_fwd);
     }
-  forward_convs(c, c->sten, c->d_conv, f32);
+  // sums that all take the FFT need no zeroed rows (the copies' rows n1, n0, V1 of one particle size are not read)
+  bool fresh = zero_first && c->nzone == 1 && !c->coarse() && c->hw_targets.empty();
+  for (int jc = 0; jc < g.ncomp; jc++) fresh = fresh && fwd_all_fft(c, jc, f32);
+  if (zero_first && !fresh) {
+    if (c->store32) ck(cudaMemsetAsync(c->d_conv32, 0, sizeof(float) * nrows * N, c->stream), "memset");
+    else ck(cudaMemsetAsync(c->d_conv, 0, sizeof(double) * nrows * N, c->stream), "memset");
+  }
+  forward_convs(c, c->sten, c->d_conv, f32, fresh);
   // nodes of the coarser quadrature zones keep their own zone's sums (zero_first holds with zones)
   for (int z = 1; z < c->nzone; z++) {
     ck(cudaMemsetAsync(c->d_zbuf, 0, sizeof(double) * nrows * N, c->stream), "memset");
@@ -888,9 +887,18 @@ void forward_pass(Ctx *c, const double *field, const PadParams &pp, bool f32, bo
   }
 }
 
-// Euler-Lagrange stencil sums of the padded channels with one zone's stencils into out ([ncomp][N]); where both the
-// delta and the theta sums of a component take FFTs, their 2 + ndim channels share one inverse transform
-void transpose_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, bool f32)
+// whether the transposed delta and theta sums of component ic share one FFT (their 2 + ndim channels one inverse)
+bool tr_all_fft(const Ctx *c, int ic, bool f32)
+{
+  const int nd = c->dg.ndim;
+  const DevStencil &sd = c->sten[TGPU_STEN_DELTA][ic], &st = c->sten[TGPU_STEN_THETA][ic];
+  if (f32) return c->spec32_built && use_fft32(c, sd, true, 1 + nd, 1) && use_fft32(c, st, true, 1, 1);
+  return c->fft_on && c->fft_state == 1 && (int)sd.spec_tr.size() == 1 + nd && st.spec_tr.size() == 1;
+}
+
+// Euler-Lagrange stencil sums of the padded channels with one zone's stencils into out ([ncomp][N]); fresh: the rows
+// hold nothing yet and every component's sums take the FFT, which writes them
+void transpose_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, bool f32, bool fresh = false)
 {
   const tgpu::DevGeom &g = c->dg;
   const long N = g.N;
@@ -901,20 +909,18 @@ void transpose_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, b
     const int base = ic * (nd + 2);
     int chs[tgpu::kMaxRb];
     for (int t = 0; t < nd + 2; t++) chs[t] = base + t;
-    if (sten == c->sten && f32 && c->spec32_built && use_fft32(c, sd, true, 1 + nd, 1) &&
-        use_fft32(c, st, true, 1, 1)) {
-      const float2 *k[tgpu::kMaxRb];
-      for (int t = 0; t <= nd; t++) k[t] = sd.spec_tr32[t];
-      k[nd + 1] = st.spec_tr32[0];
-      fft_tr_sum<float2>(c, chs, k, nd + 2, o[0]);
-      continue;
-    }
-    if (sten == c->sten && !f32 && c->fft_on && c->fft_state == 1 && (int)sd.spec_tr.size() == 1 + nd &&
-        st.spec_tr.size() == 1) {
-      const double2 *k[tgpu::kMaxRb];
-      for (int t = 0; t <= nd; t++) k[t] = sd.spec_tr[t];
-      k[nd + 1] = st.spec_tr[0];
-      fft_tr_sum<double2>(c, chs, k, nd + 2, o[0]);
+    if (sten == c->sten && tr_all_fft(c, ic, f32)) {
+      if (f32) {
+        const float2 *k[tgpu::kMaxRb];
+        for (int t = 0; t <= nd; t++) k[t] = sd.spec_tr32[t];
+        k[nd + 1] = st.spec_tr32[0];
+        fft_tr_sum<float2>(c, chs, k, nd + 2, o[0], !fresh);
+      } else {
+        const double2 *k[tgpu::kMaxRb];
+        for (int t = 0; t <= nd; t++) k[t] = sd.spec_tr[t];
+        k[nd + 1] = st.spec_tr[0];
+        fft_tr_sum<double2>(c, chs, k, nd + 2, o[0], !fresh);
+      }
       continue;
     }
     if (c->store32) throw Error(TGPU_ERR_STATE, "an FP32-storage product needs a direct stencil sum");
@@ -928,20 +934,21 @@ void transpose_pass(Ctx *c, const PadParams &pp, bool f32, const double *chan = 
 {
   const tgpu::DevGeom &g = c->dg;
   const long N = g.N;
-  if (c->store32) {
-    if (zero_first) ck(cudaMemsetAsync(c->d_tr32, 0, sizeof(float) * (size_t)g.ncomp * N, c->stream), "memset");
-    pad32(c, c->d_chan32, pp);
-  } else {
-    if (zero_first) ck(cudaMemsetAsync(c->d_tr, 0, sizeof(double) * (size_t)g.ncomp * N, c->stream), "memset");
-    pad(c, chan ? chan : c->d_chan, pp, f32);
-  }
-  if (f32 && g.ndim == 3)
+  if (c->store32) pad32(c, c->d_chan32, pp);
+  else pad(c, chan ? chan : c->d_chan, pp, f32);
+  if (f32 && g.ndim >= 2)
     for (int ic = 0; ic < g.ncomp; ic++) {
       const int base = ic * (g.ndim + 2);
       decide_fft32_sten(c, c->sten[TGPU_STEN_DELTA][ic], true, base, 1 + g.ndim, 1);
       decide_fft32_sten(c, c->sten[TGPU_STEN_THETA][ic], true, base + g.ndim + 1, 1, 1);
     }
-  transpose_convs(c, c->sten, c->d_tr, f32);
+  bool fresh = zero_first && c->nzone == 1;
+  for (int ic = 0; ic < g.ncomp; ic++) fresh = fresh && tr_all_fft(c, ic, f32);
+  if (zero_first && !fresh) {
+    if (c->store32) ck(cudaMemsetAsync(c->d_tr32, 0, sizeof(float) * (size_t)g.ncomp * N, c->stream), "memset");
+    else ck(cudaMemsetAsync(c->d_tr, 0, sizeof(double) * (size_t)g.ncomp * N, c->stream), "memset");
+  }
+  transpose_convs(c, c->sten, c->d_tr, f32, fresh);
   for (int z = 1; z < c->nzone; z++) {
     ck(cudaMemsetAsync(c->d_zbuf, 0, sizeof(double) * (size_t)g.ncomp * N, c->stream), "memset");
     transpose_convs(c, c->zsten[z], c->d_zbuf, f32);
@@ -1129,11 +1136,11 @@ const double *prolonged(Ctx *c, const double *v, int nrows)
 }
 
 // The FP32 Schur product with FP32 storage: every stencil sum an FP32 FFT (the choices already made by timing), in
-// 3-D, with one quadrature zone, no hard-wall corrections and no coarsened nodes
+// 2-D or 3-D, with one quadrature zone, no hard-wall corrections and no coarsened nodes
 bool schur_store32_ok(Ctx *c)
 {
   const tgpu::DevGeom &g = c->dg;
-  if (!prod_f32(c) || !c->spec32_built || g.ndim != 3 || c->nzone != 1 || !c->hw_targets.empty() || c->coarse())
+  if (!prod_f32(c) || !c->spec32_built || g.ndim < 2 || c->nzone != 1 || !c->hw_targets.empty() || c->coarse())
     return false;
   const int nde = 1 + (g.single_size ? 0 : 2) + g.ndim * (g.single_size ? 1 : 2);
   for (int jc = 0; jc < g.ncomp; jc++) {
@@ -1678,7 +1685,7 @@ void adj_conv(Ctx *c, int ch0, int nin, const DevStencil &st, const double *coef
               const int *vecdim = nullptr)
 {
   tgpu::launch_conv<double>(c->d_adj_pad + (long)ch0 * c->dg.NP, c->dg.NP, nin, st.d_loff_neg, coef, st.L, outs, nout,
-                            true, c->dg.N, c->stream);
+                            true, c->dg.N, c->dg.ndim, c->stream);
   c->stats.conv_launches++;
   c->stats.kernel_launches++;
   if (has_reflect(c)) {
@@ -3155,6 +3162,7 @@ int tgpu_set_fft32_policy(tgpu_handle h, int policy)
     Ctx *c = C(h);
     need_final(c);
     if (policy < -1 || policy > 1) throw Error(TGPU_ERR_ARG, "policy");
+    if (policy == 1 && c->dg.ndim != 3) throw Error(TGPU_ERR_UNSUPPORTED, "FP32 FFT sums unavailable for this problem");
     int v = 0;
     if (policy != -1) {
       v = policy == 1 ? 1 : -1;
@@ -3494,7 +3502,7 @@ int tgpu_time_stencil_sum(tgpu_handle h, int type, int index, int precision, int
     if (precision != TGPU_FP64 && precision != TGPU_FP32 && precision != TGPU_FP16TC && precision != TGPU_FILL_FF &&
         precision != TGPU_FILL_FFT && precision != TGPU_TIME_FFT32)
       throw Error(TGPU_ERR_ARG, "precision");
-    if (precision == TGPU_TIME_FFT32 && (type != TGPU_STEN_UATT || !prepare_spec32(c) ||
+    if (precision == TGPU_TIME_FFT32 && (type != TGPU_STEN_UATT || c->dg.ndim != 3 || !prepare_spec32(c) ||
                                          c->sten[type][index].spec_fwd32.empty()))
       throw Error(TGPU_ERR_UNSUPPORTED, "FP32 FFT sums exist for 3-D attraction stencils only");
     if (precision == TGPU_FILL_FFT) {
@@ -3562,7 +3570,7 @@ int tgpu_time_fft_pass(tgpu_handle h, int precision, int axis, int reps, double 
     need_final(c);
     if ((precision != TGPU_FP32 && precision != TGPU_FP64) || axis < 1 || axis > 2 || reps < 1 || !ms_per_pass)
       throw Error(TGPU_ERR_ARG, "precision, axis or reps");
-    if (precision == TGPU_FP32 ? !prepare_spec32(c) : (ensure_fft(c), c->fft_state != 1))
+    if (c->dg.ndim != 3 || (precision == TGPU_FP32 ? !prepare_spec32(c) : (ensure_fft(c), c->fft_state != 1)))
       throw Error(TGPU_ERR_UNSUPPORTED, "FFT sums unavailable for this problem");
     if (c->fft.F[axis] == 1) throw Error(TGPU_ERR_UNSUPPORTED, "no transform along that axis");
     cudaEvent_t e0, e1;

@@ -159,10 +159,74 @@ __global__ void __launch_bounds__(kThreads) k_conv(const T *__restrict__ in, lon
   }
 }
 
+// The same sums with a node's taps split over the eight warps of a block (32 nodes each), added in warp order at the
+// end.  A block of k_conv holds 256 nodes for the whole stencil: at 157 x 143 nodes that is 88 blocks on 152 SMs, each
+// at the FP64 pipe's rate, 560 us for the 7.9e3-point attraction stencil where the pipe of the whole chip needs 290.
+// Here 702 blocks share the SMs: 315 us.
+template <typename T, typename Acc, int NIN, int NOUT>
+__global__ void __launch_bounds__(kThreads) k_conv_split(const T *__restrict__ in, long cstride,
+                                                          const int *__restrict__ loff, const T *__restrict__ coef,
+                                                          int L, OutPtrs out, int accumulate)
+{
+  constexpr int kWarps = kThreads / 32;
+  __shared__ int s_off[kChunk];
+  __shared__ T s_coef[kChunk * NIN * NOUT];
+  __shared__ Acc s_sum[kWarps][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long i = blockIdx.x * 32L + lane;
+  const bool active = i < c_g.N;
+  const long ip = active ? pad_center(i) : 0;
+  Acc acc[NOUT];
+#pragma unroll
+  for (int o = 0; o < NOUT; o++) acc[o] = 0;
+  for (int k0 = 0; k0 < L; k0 += kChunk) {
+    const int n = min(kChunk, L - k0);
+    __syncthreads();
+    for (int t = threadIdx.x; t < n; t += kThreads) s_off[t] = loff[k0 + t];
+    for (int t = threadIdx.x; t < n * NIN * NOUT; t += kThreads) s_coef[t] = coef[(long)k0 * NIN * NOUT + t];
+    __syncthreads();
+    if (active) {
+#pragma unroll 4
+      for (int k = warp; k < n; k += kWarps) {
+        const long j = ip + s_off[k];
+        T v[NIN];
+#pragma unroll
+        for (int c = 0; c < NIN; c++) v[c] = __ldg(in + c * cstride + j);
+#pragma unroll
+        for (int o = 0; o < NOUT; o++)
+#pragma unroll
+          for (int c = 0; c < NIN; c++) acc[o] = fma((Acc)s_coef[(k * NOUT + o) * NIN + c], (Acc)v[c], acc[o]);
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 0; o < NOUT; o++) {
+    __syncthreads();
+    s_sum[warp][lane] = acc[o];
+    __syncthreads();
+    if (warp == o % kWarps && active) {
+      Acc s = s_sum[0][lane];
+#pragma unroll
+      for (int w = 1; w < kWarps; w++) s += s_sum[w][lane];
+      double *dst = out.p[o];
+      dst[i] = accumulate ? dst[i] + (double)s : (double)s;
+    }
+  }
+}
+
+// Split taps in 2-D and 3-D while k_conv's 256-node blocks would leave SMs idle or unevenly loaded, up to eight blocks
+// per SM (311 000 nodes; beyond, the last wave costs k_conv under 10% and it stages each tap for eight times the
+// nodes).  1-D problems keep k_conv (their solves run in gmres_line.h; a few hundred taps leave little to split).
+static bool conv_split(long N, int ndim) { return ndim >= 2 && N < 8L * 152 * kThreads; }
+
 template <typename T, typename Acc, int NIN, int NOUT>
 static void conv_dispatch(const T *in, long cstride, const int *loff, const T *coef, int L, const OutPtrs &out,
-                          bool acc, cudaStream_t s, long N)
+                          bool acc, cudaStream_t s, long N, int ndim)
 {
+  if (conv_split(N, ndim)) {
+    k_conv_split<T, Acc, NIN, NOUT><<<(int)((N + 31) / 32), kThreads, 0, s>>>(in, cstride, loff, coef, L, out, acc ? 1 : 0);
+    return;
+  }
   const int grid = (int)((N + kThreads - 1) / kThreads);
   k_conv<T, Acc, NIN, NOUT><<<grid, kThreads, 0, s>>>(in, cstride, loff, coef, L, out, acc ? 1 : 0);
 }
@@ -170,12 +234,12 @@ static void conv_dispatch(const T *in, long cstride, const int *loff, const T *c
 // Coefficient rows: `coef` is the table for the shape (nin, nout) this call uses.
 template <>
 void launch_conv<double>(const double *in, long cstride, int nin, const int *loff, const double *coef, int L,
-                         double *const *out, int nout, bool acc, long N, cudaStream_t s)
+                         double *const *out, int nout, bool acc, long N, int ndim, cudaStream_t s)
 {
   OutPtrs o{};
   for (int k = 0; k < nout; k++) o.p[k] = out[k];
 #define TGPU_CONV(NI, NO) \
-  if (nin == NI && nout == NO) { conv_dispatch<double, double, NI, NO>(in, cstride, loff, coef, L, o, acc, s, N); return; }
+  if (nin == NI && nout == NO) { conv_dispatch<double, double, NI, NO>(in, cstride, loff, coef, L, o, acc, s, N, ndim); return; }
   TGPU_CONV(1, 1) TGPU_CONV(1, 2) TGPU_CONV(1, 3) TGPU_CONV(1, 4) TGPU_CONV(1, 5) TGPU_CONV(1, 6) TGPU_CONV(1, 7)
   TGPU_CONV(1, 8) TGPU_CONV(1, 9) TGPU_CONV(2, 1) TGPU_CONV(3, 1) TGPU_CONV(4, 1)
 #undef TGPU_CONV
@@ -185,12 +249,12 @@ void launch_conv<double>(const double *in, long cstride, int nin, const int *lof
 
 template <>
 void launch_conv<float>(const float *in, long cstride, int nin, const int *loff, const float *coef, int L,
-                        double *const *out, int nout, bool acc, long N, cudaStream_t s)
+                        double *const *out, int nout, bool acc, long N, int ndim, cudaStream_t s)
 {
   OutPtrs o{};
   for (int k = 0; k < nout; k++) o.p[k] = out[k];
 #define TGPU_CONV(NI, NO) \
-  if (nin == NI && nout == NO) { conv_dispatch<float, float, NI, NO>(in, cstride, loff, coef, L, o, acc, s, N); return; }
+  if (nin == NI && nout == NO) { conv_dispatch<float, float, NI, NO>(in, cstride, loff, coef, L, o, acc, s, N, ndim); return; }
   TGPU_CONV(1, 1) TGPU_CONV(1, 2) TGPU_CONV(1, 3) TGPU_CONV(1, 4) TGPU_CONV(1, 5) TGPU_CONV(1, 6) TGPU_CONV(1, 7)
   TGPU_CONV(1, 8) TGPU_CONV(1, 9) TGPU_CONV(2, 1) TGPU_CONV(3, 1) TGPU_CONV(4, 1)
 #undef TGPU_CONV

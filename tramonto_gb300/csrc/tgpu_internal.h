@@ -501,7 +501,7 @@ void launch_pad(const double *src, T *dst, int nch, const double *bulk, const in
 // out[o][i] (+)= sum_k sum_c coef[k][o][c] * in[c][pad(i) + loff[k]]
 template <typename T>
 void launch_conv(const T *in, long in_cstride, int nin, const int *loff, const T *coef, int L, double *const *out,
-                 int nout, bool accumulate, long N, cudaStream_t s);
+                 int nout, bool accumulate, long N, int ndim, cudaStream_t s);
 void launch_conv_slab(const float *in, long in_total, const int4 *planes, int nplanes, const int4 *lines,
                       const float *lw, double *out, int pitch, int ncols, int max_rows, int max_lines, int max_w,
                       int nx, int ny, int nz, cudaStream_t s);
