@@ -849,44 +849,6 @@ void forward_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, boo
   }
 }
 
-// Weighted-density (and mean-field) sums of a density-shaped field
-// (`field` points at the first density row, rows N apart) into d_conv.
-void forward_pass(Ctx *c, const double *field, const PadParams &pp, bool f32, bool zero_first = true)
-{
-  const tgpu::DevGeom &g = c->dg;
-  const long N = g.N;
-  const size_t nrows = (size_t)(g.nrb + g.ncomp);
-  pad(c, field, pp, f32);
-  if (f32 && g.attraction && g.ndim >= 2) decide_fft32(c);
-  if (f32 && g.ndim >= 2)
-    for (int jc = 0; jc < g.ncomp; jc++) {
-      decide_fft32_sten(c, c->sten[TGPU_STEN_THETA][jc], false, jc, 1, 1);
-      decide_fft32_sten(c, c->sten[TGPU_STEN_DELTA][jc], false, jc, 1, c->sten[TGPU_STEN_DELTA][jc].nout_fwd);
-    }
-  // sums that all take the FFT need no zeroed rows (the copies' rows n1, n0, V1 of one particle size are not read)
-  bool fresh = zero_first && c->nzone == 1 && !c->coarse() && c->hw_targets.empty();
-  for (int jc = 0; jc < g.ncomp; jc++) fresh = fresh && fwd_all_fft(c, jc, f32);
-  if (zero_first && !fresh) {
-    if (c->store32) ck(cudaMemsetAsync(c->d_conv32, 0, sizeof(float) * nrows * N, c->stream), "memset");
-    else ck(cudaMemsetAsync(c->d_conv, 0, sizeof(double) * nrows * N, c->stream), "memset");
-  }
-  forward_convs(c, c->sten, c->d_conv, f32, fresh);
-  // nodes of the coarser quadrature zones keep their own zone's sums (zero_first holds with zones)
-  for (int z = 1; z < c->nzone; z++) {
-    ck(cudaMemsetAsync(c->d_zbuf, 0, sizeof(double) * nrows * N, c->stream), "memset");
-    forward_convs(c, c->zsten[z], c->d_zbuf, f32);
-    tgpu::launch_zone_merge(c->d_zbuf, c->d_conv, (int)nrows, N, c->d_zone, z, c->stream);
-    c->stats.kernel_launches++;
-  }
-  if (g.hard_surf && !c->hw_targets.empty()) {
-    tgpu::launch_hw_correct(field, N, 0, c->sten[TGPU_STEN_THETA].data(), c->sten[TGPU_STEN_DELTA].data(),
-                            g.attraction ? c->sten[TGPU_STEN_UATT].data() : nullptr, g.ncomp, true, g.attraction != 0,
-                            c->d_hw_targets, (int)c->hw_targets.size(), c->d_zero, c->d_bnodes, c->d_fmask,
-                            c->d_conv, c->stream);
-    c->stats.kernel_launches++;
-  }
-}
-
 // whether the transposed delta and theta sums of component ic share one FFT (their 2 + ndim channels one inverse)
 bool tr_all_fft(const Ctx *c, int ic, bool f32)
 {
@@ -929,6 +891,89 @@ void transpose_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, b
   }
 }
 
+// In 2-D the FP32 sums of a pass choose together: one transform of the field (or of the channels) serves them all and a
+// pass of FFTs is a few launches whatever the stencils, so a sum alone says little (201 x 201 slit: theta 11 us and
+// delta 17 us direct against 42 us as an FFT of its own, but 38 us of direct sums next to the attraction's FFT against
+// 8 us more for its outputs).  The whole pass is timed both ways, on the recorded channels into the pass's own output.
+void decide_fft32_2d(Ctx *c, bool tr)
+{
+  const tgpu::DevGeom &g = c->dg;
+  std::vector<int *> flags;
+  for (int jc = 0; jc < g.ncomp; jc++)
+    for (int t : {TGPU_STEN_THETA, TGPU_STEN_DELTA}) {
+      DevStencil &st = c->sten[t][jc];
+      flags.push_back(tr ? &st.fft32_tr : &st.fft32_fwd);
+    }
+  if (!tr && g.attraction) flags.push_back(&c->fft32_slab);
+  bool open = false;
+  for (int *f : flags) open = open || *f == 0;
+  if (!open) return;
+  for (int *f : flags) *f = -1;
+  if (!prepare_spec32(c)) return;
+  auto pass = [&] {
+    if (tr) transpose_convs(c, c->sten, c->d_tr, true);
+    else forward_convs(c, c->sten, c->d_conv, true);
+  };
+  cudaEvent_t ev[4];
+  for (auto &e : ev) ck(cudaEventCreate(&e), "event");
+  float t[2] = {0.f, 0.f};
+  for (int way = 0; way < 2; way++) {
+    for (int *f : flags) *f = way == 0 ? -1 : 1;
+    pass();   // warm-up
+    ck(cudaEventRecord(ev[2 * way], c->stream), "event");
+    for (int r = 0; r < 2; r++) {
+      c->fft32_gen = -1;   // each FFT pass transforms its field afresh
+      pass();
+    }
+    ck(cudaEventRecord(ev[2 * way + 1], c->stream), "event");
+    ck(cudaEventSynchronize(ev[2 * way + 1]), "event");
+    ck(cudaEventElapsedTime(&t[way], ev[2 * way], ev[2 * way + 1]), "event");
+  }
+  for (auto &e : ev) cudaEventDestroy(e);
+  // once both directions take FFTs the product runs in FP32 storage, which saves about 12 us of conversions and copies
+  const float bias = tr && c->sten[TGPU_STEN_THETA][0].fft32_fwd == 1 ? 2 * 0.012f : 0.f;   // (ms, two passes timed)
+  for (int *f : flags) *f = t[1] < t[0] + bias ? 1 : -1;
+}
+
+// Weighted-density (and mean-field) sums of a density-shaped field
+// (`field` points at the first density row, rows N apart) into d_conv.
+void forward_pass(Ctx *c, const double *field, const PadParams &pp, bool f32, bool zero_first = true)
+{
+  const tgpu::DevGeom &g = c->dg;
+  const long N = g.N;
+  const size_t nrows = (size_t)(g.nrb + g.ncomp);
+  pad(c, field, pp, f32);
+  if (f32 && g.ndim == 2) decide_fft32_2d(c, false);
+  if (f32 && g.attraction && g.ndim == 3) decide_fft32(c);
+  if (f32 && g.ndim == 3)
+    for (int jc = 0; jc < g.ncomp; jc++) {
+      decide_fft32_sten(c, c->sten[TGPU_STEN_THETA][jc], false, jc, 1, 1);
+      decide_fft32_sten(c, c->sten[TGPU_STEN_DELTA][jc], false, jc, 1, c->sten[TGPU_STEN_DELTA][jc].nout_fwd);
+    }
+  // sums that all take the FFT need no zeroed rows (the copies' rows n1, n0, V1 of one particle size are not read)
+  bool fresh = zero_first && c->nzone == 1 && !c->coarse() && c->hw_targets.empty();
+  for (int jc = 0; jc < g.ncomp; jc++) fresh = fresh && fwd_all_fft(c, jc, f32);
+  if (zero_first && !fresh) {
+    if (c->store32) ck(cudaMemsetAsync(c->d_conv32, 0, sizeof(float) * nrows * N, c->stream), "memset");
+    else ck(cudaMemsetAsync(c->d_conv, 0, sizeof(double) * nrows * N, c->stream), "memset");
+  }
+  forward_convs(c, c->sten, c->d_conv, f32, fresh);
+  // nodes of the coarser quadrature zones keep their own zone's sums (zero_first holds with zones)
+  for (int z = 1; z < c->nzone; z++) {
+    ck(cudaMemsetAsync(c->d_zbuf, 0, sizeof(double) * nrows * N, c->stream), "memset");
+    forward_convs(c, c->zsten[z], c->d_zbuf, f32);
+    tgpu::launch_zone_merge(c->d_zbuf, c->d_conv, (int)nrows, N, c->d_zone, z, c->stream);
+    c->stats.kernel_launches++;
+  }
+  if (g.hard_surf && !c->hw_targets.empty()) {
+    tgpu::launch_hw_correct(field, N, 0, c->sten[TGPU_STEN_THETA].data(), c->sten[TGPU_STEN_DELTA].data(),
+                            g.attraction ? c->sten[TGPU_STEN_UATT].data() : nullptr, g.ncomp, true, g.attraction != 0,
+                            c->d_hw_targets, (int)c->hw_targets.size(), c->d_zero, c->d_bnodes, c->d_fmask,
+                            c->d_conv, c->stream);
+    c->stats.kernel_launches++;
+  }
+}
+
 // Euler-Lagrange stencil sums over the channels in d_chan into d_tr.
 void transpose_pass(Ctx *c, const PadParams &pp, bool f32, const double *chan = nullptr, bool zero_first = true)
 {
@@ -936,7 +981,8 @@ void transpose_pass(Ctx *c, const PadParams &pp, bool f32, const double *chan = 
   const long N = g.N;
   if (c->store32) pad32(c, c->d_chan32, pp);
   else pad(c, chan ? chan : c->d_chan, pp, f32);
-  if (f32 && g.ndim >= 2)
+  if (f32 && g.ndim == 2) decide_fft32_2d(c, true);
+  if (f32 && g.ndim == 3)
     for (int ic = 0; ic < g.ncomp; ic++) {
       const int base = ic * (g.ndim + 2);
       decide_fft32_sten(c, c->sten[TGPU_STEN_DELTA][ic], true, base, 1 + g.ndim, 1);
@@ -1176,7 +1222,8 @@ void ensure_store32(Ctx *c)
   }
 }
 
-void schur_device_store32(Ctx *c, const double *d_v2, double *d_y2)
+// precond: y2 = M^-1 S v2, with GMRES's diagonal preconditioner
+void schur_device_store32(Ctx *c, const double *d_v2, double *d_y2, bool precond)
 {
   const tgpu::DevGeom &g = c->dg;
   ensure_store32(c);
@@ -1192,19 +1239,20 @@ void schur_device_store32(Ctx *c, const double *d_v2, double *d_y2)
   }
   c->store32 = false;
   c->pad_src32 = nullptr;
-  tgpu::launch_schur_combine32(c->d_inv32, c->d_kind32, d_v2, c->d_tr32, c->d_ymf32, d_y2, c->stream);
+  tgpu::launch_schur_combine32(c->d_inv32, c->d_kind32, d_v2, c->d_tr32, c->d_ymf32, d_y2,
+                                precond ? c->d_x : nullptr, c->stream);
   c->stats.kernel_launches += 2;
   c->stats.schur_applies++;
 }
 
-void schur_device(Ctx *c, const double *d_v2, double *d_y2)
+void schur_device(Ctx *c, const double *d_v2, double *d_y2, bool precond = false)
 {
   need_state(c);
   TcScope tcs(c);
   const tgpu::DevGeom &g = c->dg;
   const bool f32 = prod_f32(c);
   if (f32 && schur_store32_ok(c)) {
-    schur_device_store32(c, d_v2, d_y2);
+    schur_device_store32(c, d_v2, d_y2, precond);
     return;
   }
   const double *v2 = prolonged(c, d_v2, g.ncomp);
@@ -1214,6 +1262,7 @@ void schur_device(Ctx *c, const double *d_v2, double *d_y2)
   transpose_pass(c, c->pads.tr_jac, f32);
   tgpu::launch_schur_combine(c->d_x, c->d_vext, c->d_zero, v2, c->d_tr, c->d_ymf, d_y2, c->stream);
   if (c->coarse()) tgpu::launch_zero_nodes(d_y2, g.ncomp, g.N, c->cr, c->stream);
+  if (precond) tgpu::launch_precond(c->d_x, c->d_vext, c->d_zero, d_y2, d_y2, c->stream);
   c->stats.kernel_launches += 2;
   c->stats.schur_applies++;
 }
@@ -1463,24 +1512,25 @@ int gmres(Ctx *c, const double *d_rhs, double *d_x2, double tol, int maxit, int 
     gv[0] = beta;
     int k = 0;
     for (; k < m; k++) {
-      if (c->gmres_transpose) schur_t_device(c, V + (long)k * n, c->d_gw);
-      else schur_device(c, V + (long)k * n, c->d_gw);
-      tgpu::launch_precond(c->d_x, c->d_vext, c->d_zero, c->d_gw, c->d_gt, c->stream);
-      // classical Gram-Schmidt, two passes; h and the norm stay on the device
-      // until one copy per iteration
-      double *d_h1 = c->d_red, *d_h2 = c->d_red + (kdim + 1), *d_nrm = c->d_red + 2 * (kdim + 1);
-      tgpu::launch_multidot(V, n, k + 1, c->d_gt, n, c->d_partial, nb, d_h1, c->stream);
-      tgpu::launch_multiaxpy(c->d_gt, V, n, k + 1, d_h1, n, c->stream);
-      tgpu::launch_multidot(V, n, k + 1, c->d_gt, n, c->d_partial, nb, d_h2, c->stream);
-      tgpu::launch_multiaxpy(c->d_gt, V, n, k + 1, d_h2, n, c->stream);
-      tgpu::launch_norm2(c->d_gt, n, c->d_partial, nb, d_nrm, c->stream);
-      c->stats.kernel_launches += 6;
-      red_to_host(c, 2 * (kdim + 1) + 1);
-      const double hn = std::sqrt(c->h_red[2 * (kdim + 1)]);
+      if (c->gmres_transpose) {
+        schur_t_device(c, V + (long)k * n, c->d_gw);
+        tgpu::launch_precond(c->d_x, c->d_vext, c->d_zero, c->d_gw, c->d_gt, c->stream);
+      } else {
+        schur_device(c, V + (long)k * n, c->d_gt, true);
+      }
+      // classical Gram-Schmidt, two passes; h, the norm and the next basis vector stay on the device until one copy
+      // per iteration
+      double *d_nrm = c->d_red, *d_h1 = c->d_red + 1, *d_h2 = c->d_red + 1 + (k + 1);
+      tgpu::launch_gram_schmidt(0, c->d_gt, V, n, k + 1, n, nullptr, c->d_partial, d_h1, c->stream);
+      tgpu::launch_gram_schmidt(1, c->d_gt, V, n, k + 1, n, d_h1, c->d_partial, d_h2, c->stream);
+      tgpu::launch_gram_schmidt(2, c->d_gt, V, n, k + 1, n, d_h2, c->d_partial, d_nrm, c->stream);
+      tgpu::launch_normalize(V + (long)(k + 1) * n, c->d_gt, d_nrm, n, c->stream);
+      c->stats.kernel_launches += 5;
+      red_to_host(c, 1 + 2 * (k + 1));
+      const double hn = std::sqrt(c->h_red[0]);
       if (!std::isfinite(hn)) throw Error(TGPU_ERR_NONFINITE, "non-finite Krylov vector in the Schur solve");
-      for (int j = 0; j <= k; j++) H[(size_t)j * kdim + k] = c->h_red[j] + c->h_red[kdim + 1 + j];
+      for (int j = 0; j <= k; j++) H[(size_t)j * kdim + k] = c->h_red[1 + j] + c->h_red[2 + k + j];
       H[(size_t)(k + 1) * kdim + k] = hn;
-      if (hn > 0.0) tgpu::launch_scale(V + (long)(k + 1) * n, c->d_gt, 1.0 / hn, n, c->stream);
       for (int j = 0; j < k; j++) {
         const double a = H[(size_t)j * kdim + k], b = H[(size_t)(j + 1) * kdim + k];
         H[(size_t)j * kdim + k] = cs[j] * a + sn[j] * b;

@@ -318,15 +318,15 @@ __global__ void __launch_bounds__(lines_per_cta<C>() * HI) k_fft_lines(PassBatch
 // per FP32 inverse launch.)  Bound as the y and z passes; 128^3 workload, per launch of 1 and 5 or 6 lines' transforms:
 // forward 42 us in FP32 (47 with radix-4 stages), inverse 35 (33); FP64 271 (318) and 274 (338).
 template <class C>
-constexpr int x_pairs() { return std::is_same<C, float2>::value ? 16 : 8; }
+constexpr int x_pairs_max() { return std::is_same<C, float2>::value ? 16 : 8; }
 constexpr int kXBatch = 4;   // positions a lane loads before it stores them
 
 // shared pitch of the R2 values of one k1: odd, so that the R1 threads of a line read distinct banks
 __host__ __device__ __forceinline__ int pitch2(int R2) { return R2 | 1; }
 
 // the tile's transforms in place: sm[p * lp + x] -> sm[p * lp + k] (lp >= n and >= R1 pitch2(R2))
-template <int NP, int LO, int HI, bool INV, class C>
-__device__ __forceinline__ void tile_fft(C *sm, int lp, const Line1d<C> &ln)
+template <int LO, int HI, bool INV, class C>
+__device__ __forceinline__ void tile_fft(C *sm, int NP, int lp, const Line1d<C> &ln)
 {
   const int R1 = ln.R1, R2 = ln.R2, pr = pitch2(R2);
   __syncthreads();
@@ -367,10 +367,9 @@ __device__ __forceinline__ void tile_fft(C *sm, int lp, const Line1d<C> &ln)
 
 // forward: two real lines per complex line, split into two half-spectrum lines by Hermitian symmetry
 template <class T, class C, class Src, int LO, int HI>
-__global__ void __launch_bounds__((x_pairs<C>() * HI + 31) / 32 * 32) k_rfft_lines(SrcBatch<Src, C> sb, XGeom g,
-                                                                               Line1d<C> ln, int lp)
+__global__ void __launch_bounds__((x_pairs_max<C>() * HI + 31) / 32 * 32) k_rfft_lines(SrcBatch<Src, C> sb, XGeom g,
+                                                                               Line1d<C> ln, int NP, int lp)
 {
-  constexpr int NP = x_pairs<C>();
   const Src &src = sb.src[blockIdx.y];
   C *__restrict__ spec = sb.spec[blockIdx.y];
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -394,7 +393,7 @@ __global__ void __launch_bounds__((x_pairs<C>() * HI + 31) / 32 * 32) k_rfft_lin
         if (x0 + 32 * u < n) sm[p * lp + x0 + 32 * u] = C{a[u], b[u]};
     }
   }
-  tile_fft<NP, LO, HI, false, C>(sm, lp, ln);
+  tile_fft<LO, HI, false, C>(sm, NP, lp, ln);
   for (int p = warp; p < np; p += nw) {
     const long L = 2 * (long)(pair0 + p);
     const bool two = L + 1 < g.nlines;
@@ -428,11 +427,10 @@ __device__ __forceinline__ void write_line(const C *z, bool imag, O *o, int nx0,
 // inverse: two half-spectrum lines as one complex line Z = A + iB, whose inverse's real and imaginary parts are the
 // outputs of the interior nodes (out[node] = scale * value, or += when accumulate)
 template <class C, int LO, int HI>
-__global__ void __launch_bounds__((x_pairs<C>() * HI + 31) / 32 * 32) k_irfft_lines(OutBatch<C> ob, XGeom g,
-                                                                                Line1d<C> ln, int lp, double scale,
-                                                                                int accumulate)
+__global__ void __launch_bounds__((x_pairs_max<C>() * HI + 31) / 32 * 32) k_irfft_lines(OutBatch<C> ob, XGeom g,
+                                                                                Line1d<C> ln, int NP, int lp,
+                                                                                double scale, int accumulate)
 {
-  constexpr int NP = x_pairs<C>();
   using T = typename dft::Real<C>::T;
   const C *__restrict__ spec = ob.spec[blockIdx.y];
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -450,7 +448,7 @@ __global__ void __launch_bounds__((x_pairs<C>() * HI + 31) / 32 * 32) k_irfft_li
       if (k > 0 && 2 * k < n) sm[p * lp + n - k] = C{A.x + B.y, B.x - A.y};
     }
   }
-  tile_fft<NP, LO, HI, true, C>(sm, lp, ln);
+  tile_fft<LO, HI, true, C>(sm, NP, lp, ln);
   const int nx0 = g.nx[0];
   const T sc = (T)scale;
   for (int p = warp; p < np; p += nw) {
@@ -569,16 +567,22 @@ Line1d<C> line_of(const FftAxis &a)
 template <class C>
 size_t lines_smem(const FftAxis &a) { return sizeof(C) * (size_t)lines_per_cta<C>() * a.n; }
 template <class C>
-int x_threads(const FftAxis &a) { return (x_pairs<C>() * a.R1 + 31) / 32 * 32; }
+int x_pairs(long npairs, int nb)   // fewer pairs per CTA where whole tiles would leave SMs idle (2-D boxes)
+{
+  int np = x_pairs_max<C>();
+  while (np > 2 && (npairs + np - 1) / np * nb < 2 * 152) np /= 2;
+  return np;
+}
+int x_threads(const FftAxis &a, int np) { return (np * a.R1 + 31) / 32 * 32; }
 int x_pitch(const FftAxis &a) { return std::max(a.R1 * pitch2(a.R2), a.n) | 1; }   // of a line in the tile
 template <class C>
-size_t x_smem(const FftAxis &a) { return sizeof(C) * (size_t)x_pairs<C>() * x_pitch(a); }
+size_t x_smem(const FftAxis &a, int np) { return sizeof(C) * (size_t)np * x_pitch(a); }
 
 template <class T, class C>
 void set_smem_limits(const FftPlan &p)
 {
   const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  const int most_x = (int)(sizeof(C) * x_pairs<C>() * (kMaxRadix * (kMaxRadix | 1) + 1)), most = 128 * kFftMaxN;
+  const int most_x = (int)(sizeof(C) * x_pairs_max<C>() * (kMaxRadix * (kMaxRadix | 1) + 1)), most = 128 * kFftMaxN;
   with_range(p.ax[0].R1, [&](auto lo, auto hi) {
     constexpr int LO = decltype(lo)::value, HI = decltype(hi)::value;
     cudaFuncSetAttribute(k_rfft_lines<T, C, BoxSrc<T>, LO, HI>, attr, most_x);
@@ -662,10 +666,11 @@ void forward_x(const SrcBatch<Src, C> &sb, int nb, const XGeom &g, const FftPlan
 {
   const FftAxis &ax = p.ax[0];
   const long npairs = (g.nlines + 1) / 2;
-  const dim3 grid((unsigned)((npairs + x_pairs<C>() - 1) / x_pairs<C>()), (unsigned)nb);
+  const int np = x_pairs<C>(npairs, nb);
+  const dim3 grid((unsigned)((npairs + np - 1) / np), (unsigned)nb);
   with_range(ax.R1, [&](auto lo, auto hi) {
     constexpr int LO = decltype(lo)::value, HI = decltype(hi)::value;
-    k_rfft_lines<T, C, Src, LO, HI><<<grid, x_threads<C>(ax), x_smem<C>(ax), s>>>(sb, g, line_of<C>(ax), x_pitch(ax));
+    k_rfft_lines<T, C, Src, LO, HI><<<grid, x_threads(ax, np), x_smem<C>(ax, np), s>>>(sb, g, line_of<C>(ax), np, x_pitch(ax));
   });
 }
 
@@ -675,11 +680,12 @@ void inverse_x(const OutBatch<C> &ob, int nb, const FftPlan &p, double scale, bo
   const XGeom g = xgeom(p);
   const FftAxis &ax = p.ax[0];
   const long npairs = (g.nlines + 1) / 2;
-  const dim3 grid((unsigned)((npairs + x_pairs<C>() - 1) / x_pairs<C>()), (unsigned)nb);
+  const int np = x_pairs<C>(npairs, nb);
+  const dim3 grid((unsigned)((npairs + np - 1) / np), (unsigned)nb);
   with_range(ax.R1, [&](auto lo, auto hi) {
     constexpr int LO = decltype(lo)::value, HI = decltype(hi)::value;
-    k_irfft_lines<C, LO, HI><<<grid, x_threads<C>(ax), x_smem<C>(ax), s>>>(ob, g, line_of<C>(ax), x_pitch(ax), scale,
-                                                                        accumulate ? 1 : 0);
+    k_irfft_lines<C, LO, HI><<<grid, x_threads(ax, np), x_smem<C>(ax, np), s>>>(ob, g, line_of<C>(ax), np, x_pitch(ax),
+                                                                        scale, accumulate ? 1 : 0);
   });
 }
 

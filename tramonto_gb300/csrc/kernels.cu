@@ -214,10 +214,11 @@ __global__ void __launch_bounds__(kThreads) k_conv_split(const T *__restrict__ i
   }
 }
 
-// Split taps in 2-D and 3-D while k_conv's 256-node blocks would leave SMs idle or unevenly loaded, up to eight blocks
-// per SM (311 000 nodes; beyond, the last wave costs k_conv under 10% and it stages each tap for eight times the
-// nodes).  1-D problems keep k_conv (their solves run in gmres_line.h; a few hundred taps leave little to split).
-static bool conv_split(long N, int ndim) { return ndim >= 2 && N < 8L * 152 * kThreads; }
+// Split taps in 2-D while k_conv's 256-node blocks would leave SMs idle or unevenly loaded, up to eight blocks per SM
+// (311 000 nodes; beyond, the last wave costs k_conv under 10% and it stages each tap for eight times the nodes).  1-D
+// problems keep k_conv (their solves run in gmres_line.h; a few hundred taps leave little to split), and so do 3-D ones:
+// their sums of up to 1e5 terms follow the reference's order, tap by tap.
+static bool conv_split(long N, int ndim) { return ndim == 2 && N < 8L * 152 * kThreads; }
 
 template <typename T, typename Acc, int NIN, int NOUT>
 static void conv_dispatch(const T *in, long cstride, const int *loff, const T *coef, int L, const OutPtrs &out,
@@ -1169,9 +1170,10 @@ void launch_row_info32(const double *x, const double *vext, const signed char *z
 
 // k_schur_combine with the transposed sums and -u_MF in FP32 storage and the rows of k_row_info32 (no FP64 division
 // or comparison per product)
+// (x: also multiplied by the diagonal preconditioner, rho on rows with a logarithm)
 __global__ void k_schur_combine32(const double *__restrict__ inv, const signed char *__restrict__ kind,
                                   const double *__restrict__ v2, const float *__restrict__ tr,
-                                  const float *__restrict__ ymf, double *__restrict__ y2)
+                                  const float *__restrict__ ymf, double *__restrict__ y2, const double *__restrict__ x)
 {
   const long n = (long)c_g.ncomp * c_g.N;
   const bool att = c_g.attraction != 0;
@@ -1181,15 +1183,16 @@ __global__ void k_schur_combine32(const double *__restrict__ inv, const signed c
       y2[k] = v2[k];
     } else {
       const double t = v2[k] * inv[k];
-      y2[k] = kd == 0 ? t - (double)(att ? tr[k] + ymf[k] : tr[k]) : t;
+      const double r = kd == 0 ? t - (double)(att ? tr[k] + ymf[k] : tr[k]) : t;
+      y2[k] = x ? r * x[(long)c_g.first_rho * c_g.N + k] : r;
     }
   }
 }
 
 void launch_schur_combine32(const double *inv, const signed char *kind, const double *v2, const float *tr,
-                            const float *ymf, double *y2, cudaStream_t s)
+                            const float *ymf, double *y2, const double *x, cudaStream_t s)
 {
-  k_schur_combine32<<<1184, kThreads, 0, s>>>(inv, kind, v2, tr, ymf, y2);
+  k_schur_combine32<<<1184, kThreads, 0, s>>>(inv, kind, v2, tr, ymf, y2, x);
 }
 
 __global__ void k_jv_combine(const double *__restrict__ x, const double *__restrict__ vext,
@@ -1887,20 +1890,156 @@ __device__ void reduce_rows_last(const double *partial, int nb, int nrow, double
   if (threadIdx.x == 0) *counter = 0u;
 }
 
-// partial[j*nb + b] = sum over block b's chunk of V[j] . w; out[j] = sum over b (the last block)
-__global__ void k_multidot(const double *__restrict__ V, long ldv, int nvec, const double *__restrict__ w, long n,
-                           double *__restrict__ partial, double *__restrict__ out, unsigned *__restrict__ counter)
+// ---- classical Gram-Schmidt, twice (GMRES) -----------------------------------------------------------------------
+// Sums of eight values per lane over a warp, packed: lane l ends with the warp's sum of value l >> 2 (in the lanes with
+// l & 3 == 0), 9 additions instead of 40.
+__device__ __forceinline__ double warp_sum8(double *a)
 {
-  __shared__ double sh[32];
-  const long chunk = (n + gridDim.x - 1) / gridDim.x;
-  const long b0 = blockIdx.x * chunk, b1 = min(n, b0 + chunk);
-  for (int j = 0; j < nvec; j++) {
-    double s = 0.0;
-    for (long i = b0 + threadIdx.x; i < b1; i += blockDim.x) s = fma(V[(long)j * ldv + i], w[i], s);
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) partial[(long)j * gridDim.x + blockIdx.x] = s;
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const bool up = lane & 16;
+    const double send = up ? a[q] : a[q + 4], keep = up ? a[q + 4] : a[q];
+    a[q] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
   }
-  if (last_block_done(counter)) reduce_rows_last(partial, gridDim.x, nvec, out, sh, counter);
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const bool up = lane & 8;
+    const double send = up ? a[q] : a[q + 2], keep = up ? a[q + 2] : a[q];
+    a[q] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+  }
+  const bool up = lane & 4;
+  double v = (up ? a[1] : a[0]) + __shfl_xor_sync(0xffffffffu, up ? a[0] : a[1], 4);
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v;
+}
+
+// MODE 0: out[j] = V_j . w.  MODE 1: w -= sum_j hin[j] V_j, then out[j] = V_j . w.  MODE 2: w -= sum_j hin[j] V_j, then
+// out[0] = |w|^2.  One read of the basis per launch as long as it has at most eight vectors (MODE 1 keeps a node's eight
+// values in registers between the two uses).  Bound: the FP64 pipe (one FMA per 8 bytes of V and use: 3.4 us per vector
+// of 128^3 nodes) in the solves of large meshes, latency in small ones.  Per iteration of the 128^3 solve (4.7 vectors
+// on average) with dots, updates and norm as five launches: 215 us, as these three: 136 us; 40 401 nodes: 64 and 26 us.
+constexpr int kGsBlocks = 152 * 4;
+
+// one chunk of M vectors from V (the first chunk of MODE 1 and 2 also updates w, with all m vectors); M is a constant so
+// that a node's loads are all issued before their first use and no operation is spent on absent vectors
+template <int MODE, int M, bool FIRST>
+__device__ __forceinline__ void gs_chunk(double *__restrict__ w, const double *__restrict__ V, long ldv, int m, long n,
+                                         const double *hs, double *acc)
+{
+  const long stride = (long)gridDim.x * kThreads;
+#pragma unroll 2
+  for (long i = blockIdx.x * (long)kThreads + threadIdx.x; i < n; i += stride) {
+    double s = w[i], v[M];
+#pragma unroll
+    for (int q = 0; q < M; q++) v[q] = V[(long)q * ldv + i];
+    if (MODE > 0 && FIRST) {
+#pragma unroll
+      for (int q = 0; q < M; q++) s = fma(-hs[q], v[q], s);
+      if (M == 8) {
+#pragma unroll 4
+        for (int j = 8; j < m; j++) s = fma(-hs[j], V[(long)j * ldv + i], s);
+      }
+      w[i] = s;
+    }
+    if (MODE == 2) {
+      acc[0] = fma(s, s, acc[0]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < M; q++) acc[q] = fma(v[q], s, acc[q]);
+    }
+  }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kThreads) k_gram_schmidt(double *__restrict__ w, const double *__restrict__ V, long ldv,
+                                                            int m, long n, const double *__restrict__ hin,
+                                                            double *__restrict__ partial, double *__restrict__ out,
+                                                            unsigned *__restrict__ counter)
+{
+  constexpr int kWarps = kThreads / 32;
+  __shared__ double hs[512], red[kWarps][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (MODE > 0) {
+    for (int j = threadIdx.x; j < m; j += kThreads) hs[j] = hin[j];
+    __syncthreads();
+  }
+  const int rows = MODE == 2 ? 1 : m;
+  for (int c0 = 0; c0 < rows; c0 += 8) {
+    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    const double *Vc = V + (long)c0 * ldv;
+    if (c0 == 0) {
+      switch (min(m, 8)) {
+        case 1: gs_chunk<MODE, 1, true>(w, Vc, ldv, m, n, hs, acc); break;
+        case 2: gs_chunk<MODE, 2, true>(w, Vc, ldv, m, n, hs, acc); break;
+        case 3: gs_chunk<MODE, 3, true>(w, Vc, ldv, m, n, hs, acc); break;
+        case 4: gs_chunk<MODE, 4, true>(w, Vc, ldv, m, n, hs, acc); break;
+        case 5: gs_chunk<MODE, 5, true>(w, Vc, ldv, m, n, hs, acc); break;
+        case 6: gs_chunk<MODE, 6, true>(w, Vc, ldv, m, n, hs, acc); break;
+        case 7: gs_chunk<MODE, 7, true>(w, Vc, ldv, m, n, hs, acc); break;
+        default: gs_chunk<MODE, 8, true>(w, Vc, ldv, m, n, hs, acc); break;
+      }
+    } else {
+      switch (min(m - c0, 8)) {
+        case 1: gs_chunk<MODE, 1, false>(w, Vc, ldv, m, n, hs, acc); break;
+        case 2: gs_chunk<MODE, 2, false>(w, Vc, ldv, m, n, hs, acc); break;
+        case 3: gs_chunk<MODE, 3, false>(w, Vc, ldv, m, n, hs, acc); break;
+        case 4: gs_chunk<MODE, 4, false>(w, Vc, ldv, m, n, hs, acc); break;
+        case 5: gs_chunk<MODE, 5, false>(w, Vc, ldv, m, n, hs, acc); break;
+        case 6: gs_chunk<MODE, 6, false>(w, Vc, ldv, m, n, hs, acc); break;
+        case 7: gs_chunk<MODE, 7, false>(w, Vc, ldv, m, n, hs, acc); break;
+        default: gs_chunk<MODE, 8, false>(w, Vc, ldv, m, n, hs, acc); break;
+      }
+    }
+    const double v = warp_sum8(acc);
+    if ((lane & 3) == 0) red[warp][lane >> 2] = v;
+    __syncthreads();
+    if (threadIdx.x < 8 && c0 + (int)threadIdx.x < rows) {
+      double t = red[0][threadIdx.x];
+#pragma unroll
+      for (int q = 1; q < kWarps; q++) t += red[q][threadIdx.x];
+      partial[(long)(c0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
+    }
+    __syncthreads();
+  }
+  if (last_block_done(counter)) {   // a warp per row
+    for (int j = warp; j < rows; j += kWarps) {
+      double t = 0.0;
+#pragma unroll 4
+      for (int b = lane; b < (int)gridDim.x; b += 32) t += __ldcg(partial + (long)j * gridDim.x + b);
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) out[j] = t;
+    }
+    if (threadIdx.x == 0) *counter = 0u;
+  }
+}
+
+static int gs_blocks(long n) { return (int)std::min<long>(kGsBlocks, (n + kThreads - 1) / kThreads); }
+
+// partial: the base of a kPartialWords reduction buffer (its last word is the completion counter)
+void launch_gram_schmidt(int mode, double *w, const double *V, long ldv, int m, long n, const double *hin,
+                         double *partial, double *out, cudaStream_t s)
+{
+  unsigned *counter = reinterpret_cast<unsigned *>(partial + kPartialWords - 1);
+  const int grid = gs_blocks(n);
+  if (mode == 0) k_gram_schmidt<0><<<grid, kThreads, 0, s>>>(w, V, ldv, m, n, hin, partial, out, counter);
+  else if (mode == 1) k_gram_schmidt<1><<<grid, kThreads, 0, s>>>(w, V, ldv, m, n, hin, partial, out, counter);
+  else k_gram_schmidt<2><<<grid, kThreads, 0, s>>>(w, V, ldv, m, n, hin, partial, out, counter);
+}
+
+// y = x / sqrt(*norm2) (no host round trip between a norm and the next Krylov vector)
+__global__ void k_normalize(double *__restrict__ y, const double *__restrict__ x, const double *__restrict__ norm2, long n)
+{
+  __shared__ double inv;
+  if (threadIdx.x == 0) inv = 1.0 / sqrt(*norm2);
+  __syncthreads();
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) y[i] = inv * x[i];
+}
+
+void launch_normalize(double *y, const double *x, const double *norm2, long n, cudaStream_t s)
+{
+  k_normalize<<<(int)std::min<long>(1184, (n + kThreads - 1) / kThreads), kThreads, 0, s>>>(y, x, norm2, n);
 }
 
 __global__ void k_reduce_rows(const double *__restrict__ partial, int nb, int nrow, double *__restrict__ out)
@@ -1912,14 +2051,6 @@ __global__ void k_reduce_rows(const double *__restrict__ partial, int nb, int nr
     s = block_sum(s, sh);
     if (threadIdx.x == 0) out[j] = s;
   }
-}
-
-// partial: the base of a kPartialWords reduction buffer (its last word is the completion counter)
-void launch_multidot(const double *V, long ldv, int nvec, const double *w, long n, double *partial, int nblocks,
-                     double *result, cudaStream_t s)
-{
-  unsigned *counter = reinterpret_cast<unsigned *>(partial + kPartialWords - 1);
-  k_multidot<<<nblocks, kThreads, 0, s>>>(V, ldv, nvec, w, n, partial, result, counter);
 }
 
 __global__ void k_multiaxpy(double *__restrict__ w, const double *__restrict__ V, long ldv, int nvec,

@@ -533,7 +533,7 @@ void launch_rhs_combine32(const signed char *kind, const double *b, const float 
 void launch_row_info32(const double *x, const double *vext, const signed char *zero, double *inv, signed char *kind,
                        cudaStream_t s);
 void launch_schur_combine32(const double *inv, const signed char *kind, const double *v2, const float *tr,
-                            const float *ymf, double *y2, cudaStream_t s);
+                            const float *ymf, double *y2, const double *x, cudaStream_t s);
 void launch_schur_local(const double *x, const double *conv, double *chan, double *ymf, const double *coef,
                         cudaStream_t s, bool f32 = false);
 // f32: the per-node Hessian in FP32 arithmetic (FP32 products)
@@ -552,8 +552,10 @@ void launch_hw_correct_t(const double *w, const double *mfw, const DevStencil *t
                          const DevStencil *uatt, int ncomp, bool do_fmt, bool do_mf, const int *targets, int ntargets,
                          const signed char *zero, const int *bnodes, const short *fmask, double *out, cudaStream_t s);
 // Krylov helpers
-void launch_multidot(const double *V, long ldv, int nvec, const double *w, long n, double *partial, int nblocks,
-                     double *result, cudaStream_t s);
+// mode 0: out[j] = V_j . w; 1: w -= V hin, then out[j] = V_j . w; 2: w -= V hin, then out[0] = |w|^2 (m <= 512 vectors)
+void launch_gram_schmidt(int mode, double *w, const double *V, long ldv, int m, long n, const double *hin,
+                         double *partial, double *out, cudaStream_t s);
+void launch_normalize(double *y, const double *x, const double *norm2, long n, cudaStream_t s);
 void launch_multiaxpy(double *w, const double *V, long ldv, int nvec, const double *coef, long n, cudaStream_t s);
 void launch_scale(double *y, const double *x, double a, long n, cudaStream_t s);
 void launch_axpby(double *y, double a, const double *x, double b, long n, cudaStream_t s);
