@@ -1043,7 +1043,7 @@ void fill_arith(Ctx *c, const double *d_x, double *d_R, int mode, int arith)
   ck(cudaMemsetAsync(c->d_domain, 0, sizeof(unsigned), c->stream), "memset");
   if (arith == TGPU_FILL_REFINED) {
     ensure_refs(c);
-    tgpu::launch_fmt_local(x, c->d_chan, c->stream, c->d_domain);
+    tgpu::launch_fmt_local(g.ndim, g.functional, x, c->d_chan, c->stream, c->d_domain);
     bool refresh = !c->have_ref;
     if (!refresh) {
       const int nb = tgpu::reduce_blocks((long)nchan);
@@ -1082,12 +1082,12 @@ void fill_arith(Ctx *c, const double *d_x, double *d_R, int mode, int arith)
     c->fft_on = arith == TGPU_FILL_FFT;
     if (c->fft_on) ensure_fft(c);
     forward_pass(c, rho, c->pads.rho_res, f32);
-    tgpu::launch_fmt_local(x, c->d_chan, c->stream, c->d_domain);
+    tgpu::launch_fmt_local(g.ndim, g.functional, x, c->d_chan, c->stream, c->d_domain);
     transpose_pass(c, c->pads.tr_res, f32);
     c->ff_on = false;
     c->fft_on = false;
   }
-  tgpu::launch_assemble(x, c->d_vext, c->d_zero, c->d_conv, c->d_tr, d_R, c->stream, c->d_domain);
+  tgpu::launch_assemble(g.ndim, x, c->d_vext, c->d_zero, c->d_conv, c->d_tr, d_R, c->stream, c->d_domain);
   c->stats.kernel_launches += 2;
   if (c->coarse()) {   // the averaged rows of coarsened nodes
     tgpu::launch_coarse_rows(x, d_R, g.nunk, g.first_rho, g.ncomp, N, c->cr, c->d_cbulk, c->stream);
@@ -1159,7 +1159,7 @@ const double *hess_coef(Ctx *c)
   const int form = c->dg.jac_exact;
   if (c->hcoef_form == form) return c->d_hcoef;
   if (!c->d_hcoef) c->d_hcoef = dalloc<double>((size_t)tgpu::kHessCoef * c->dg.N);
-  tgpu::launch_hess_coef(c->d_x, c->d_hcoef, c->stream, c->d_hcoef32);   // with the FP32 table once it exists
+  tgpu::launch_hess_coef(c->dg.ndim, c->dg.functional, c->d_x, c->d_hcoef, c->stream, c->d_hcoef32);   // with the FP32 table once it exists
   c->stats.kernel_launches++;
   c->hcoef_form = form;
   if (c->d_hcoef32) {
@@ -1215,7 +1215,7 @@ void ensure_store32(Ctx *c)
     c->d_kind32 = dalloc<signed char>((size_t)g.ncomp * N);
   }
   if (c->hcoef32_form != g.jac_exact) {
-    tgpu::launch_hess_coef32(c->d_x, c->d_hcoef32, c->stream);
+    tgpu::launch_hess_coef32(g.ndim, g.functional, c->d_x, c->d_hcoef32, c->stream);
     tgpu::launch_row_info32(c->d_x, c->d_vext, c->d_zero, c->d_inv32, c->d_kind32, c->stream);
     c->stats.kernel_launches += 2;
     c->hcoef32_form = g.jac_exact;
@@ -1230,7 +1230,7 @@ void schur_device_store32(Ctx *c, const double *d_v2, double *d_y2, bool precond
   c->store32 = true;
   try {
     forward_pass(c, d_v2, c->pads.rho_jac, true);
-    tgpu::launch_schur_local32(g.ndim, c->d_conv32, c->d_hcoef32, c->d_chan32, c->d_ymf32, c->stream);
+    tgpu::launch_schur_local32(g.ndim, tgpu::fmt_alpha_form(g.functional), g.N, c->d_conv32, c->d_hcoef32, c->d_chan32, c->d_ymf32, c->stream);
     transpose_pass(c, c->pads.tr_jac, true);
   } catch (...) {
     c->store32 = false;
@@ -1289,7 +1289,7 @@ namespace tgpu {
 void launch_rhs_local(const double *x, const double *b, double *chan, double *ymf, const double *coef, cudaStream_t s);
 void launch_rhs_combine(const double *vext, const signed char *zero, const double *b, const double *tr,
                         const double *ymf, double *b2s, cudaStream_t s);
-void launch_x1(const double *b, const double *conv, const double *x2, double *dx, cudaStream_t s);
+void launch_x1(int nunk, long N, const double *b, const double *conv, const double *x2, double *dx, cudaStream_t s);
 }  // namespace tgpu
 
 namespace {
@@ -1307,7 +1307,7 @@ void schur_rhs_device(Ctx *c, const double *d_b, double *d_b2s)
   TcScope tcs(c);
   if (prod_f32(c) && schur_store32_ok(c)) {   // the FP32 products' right-hand side in FP32 storage
     ensure_store32(c);
-    tgpu::launch_rhs_local32(g.ndim, b, c->d_hcoef32, c->d_chan32, c->d_ymf32, c->stream);
+    tgpu::launch_rhs_local32(g.ndim, tgpu::fmt_alpha_form(g.functional), g.N, b, c->d_hcoef32, c->d_chan32, c->d_ymf32, c->stream);
     c->store32 = true;
     try {
       transpose_pass(c, c->pads.tr_jac, true);
@@ -1336,7 +1336,7 @@ void schur_x1_device(Ctx *c, const double *d_b, const double *d_x2, double *d_dx
   const tgpu::DevGeom &g = c->dg;
   const double *x2 = prolonged(c, d_x2, g.ncomp);
   forward_pass(c, x2, c->pads.rho_jac, prod_f32(c));
-  tgpu::launch_x1(d_b, c->d_conv, x2, d_dx, c->stream);
+  tgpu::launch_x1(g.nunk, g.N, d_b, c->d_conv, x2, d_dx, c->stream);
   if (c->coarse()) tgpu::launch_prolong(d_dx, 0, g.nunk, g.nunk, g.N, c->cr, nullptr, c->stream);
   c->stats.kernel_launches++;
 }
@@ -1613,7 +1613,7 @@ int newton_device(Ctx *c, double *d_x, double rel_tol, double abs_tol, double up
     tgpu::launch_newton_frac(d_x, d_dx, update_floor, c->d_partial, nb, c->d_red, c->stream);
     red_to_host(c, 1);
     const double frac = c->h_red[0];
-    tgpu::launch_newton_update(d_x, d_dx, frac, rel_tol, abs_tol, c->d_partial, nb, c->d_red, c->stream);
+    tgpu::launch_newton_update(d_x, d_dx, g.nunk, g.N, frac, rel_tol, abs_tol, c->d_partial, c->d_red, c->stream);
     coarse_state(c, d_x);
     red_to_host(c, 1);
     const double upd = std::sqrt(c->h_red[0]);
@@ -1695,7 +1695,7 @@ int newton_solve_device(Ctx *c, double *d_x, double resid_tol, int max_iter, dou
     red_to_host(c, 1);
     const double frac = c->h_red[0];
     // no update norm here (the stopping test is the next residual, whose norm also catches a non-finite update)
-    tgpu::launch_newton_update(d_x, d_dx, frac, 1.0, 1.0, nullptr, nb, nullptr, c->stream);
+    tgpu::launch_newton_update(d_x, d_dx, g.nunk, g.N, frac, 1.0, 1.0, nullptr, nullptr, c->stream);
     coarse_state(c, d_x);
     c->stats.kernel_launches += 5;
   }
@@ -1946,7 +1946,7 @@ void jtv_device(Ctx *c, const double *d_w_in, double *d_out)
         adj_conv(c, ic, 1, st, st.d_coef_fwd, o + nd + 1, 1);
       }
     }
-    tgpu::launch_jtv_local(c->d_x, c->d_vext, c->d_zero, d_w, c->d_adj_g, gst, 1, d_out, c->stream);
+    tgpu::launch_jtv_local(c->d_x, c->d_vext, c->d_zero, d_w, c->d_adj_g, gst, 1, d_out, hess_coef(c), c->stream);
     c->stats.kernel_launches += 4;
   }
   if (c->coarse()) {

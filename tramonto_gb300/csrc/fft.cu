@@ -97,8 +97,8 @@ struct XGeom {
 };
 
 // Sources of the forward x pass: element (x, y, z) of the real box (x < ext0, y < ext1, z < ext2; 0 beyond)
-// at padded position (x + off0, y + off1, z + off2).  A line's y and z are resolved once (line); load then takes the
-// elements x0, x0 + 32, ... of it, all loads issued before their values are used.
+// at padded position (x + off0, y + off1, z + off2).  A line's y and z are resolved once (line); load then takes its
+// elements first + x0, + 32, ..., all loads issued before their values are used, and at() any position around them.
 template <class T>
 struct BoxSrc {   // a padded channel, or a real box [F2][F1][F0] (off 0)
   const T *p;
@@ -108,12 +108,16 @@ struct BoxSrc {   // a padded channel, or a real box [F2][F1][F0] (off 0)
   {
     return p + (long)(z + g.off[2]) * sz + (long)(y + g.off[1]) * sy + g.off[0];
   }
+  // positions first .. first + count - 1 are the ones load reads: here all within the source's extent
+  __device__ __forceinline__ int first(const XGeom &) const { return 0; }
+  __device__ __forceinline__ int count(const XGeom &g) const { return g.ext[0]; }
   template <int NB>
-  __device__ __forceinline__ void load(const XGeom &g, const Line &L, int x0, T *v) const
+  __device__ __forceinline__ void load(const Line &L, bool use, int x0, int n, T *v) const
   {
 #pragma unroll
-    for (int u = 0; u < NB; u++) v[u] = x0 + 32 * u < g.ext[0] ? L[x0 + 32 * u] : (T)0;
+    for (int u = 0; u < NB; u++) v[u] = use && x0 + 32 * u < n ? L[x0 + 32 * u] : (T)0;
   }
+  __device__ __forceinline__ T at(const XGeom &, const Line &L, int x) const { return L[x]; }
 };
 template <class T>
 struct MappedSrc {   // the unpadded channel through the boundary maps (the padded box's values, computed)
@@ -161,50 +165,43 @@ struct MappedSrc {   // the unpadded channel through the boundary maps (the padd
     if (m.zc >= 0 && m.zero[(long)m.zc * m.N + node]) return (T)0;
     return (__popc(refl & m.signmask) & 1) ? -val : val;
   }
+  // the mesh's nodes: the box holds node i at x = e[0] + i, with no map to read
+  __device__ __forceinline__ int first(const XGeom &g) const { return g.e[0]; }
+  __device__ __forceinline__ int count(const XGeom &) const { return m.nx[0]; }
+  // nodes x0, x0 + 32, ... of a line; a line outside the mesh reads its sentinel's value
   template <int NB>
-  __device__ __forceinline__ void load(const XGeom &g, const Line &L, int x0, T *v) const
+  __device__ __forceinline__ void load(const Line &L, bool use, int x0, int n, T *v) const
   {
-    // nodes of the mesh need no map (the box's x = e[0] + node); the positions beyond them do
-    const int i0 = x0 - g.e[0];
-    bool in[NB];
+    if (!use || L.sent) {
+      const T c = use ? sentinel(L.sent) : (T)0;
 #pragma unroll
-    for (int u = 0; u < NB; u++) {
-      in[u] = !L.sent && (unsigned)(i0 + 32 * u) < (unsigned)m.nx[0];
-      v[u] = 0;
+      for (int u = 0; u < NB; u++) v[u] = c;
+      return;
     }
     if (m.src32) {
-      const float *s = m.src32 + L.base + i0;
+      const float *s = m.src32 + L.base;
 #pragma unroll
-      for (int u = 0; u < NB; u++)
-        if (in[u]) v[u] = (T)s[32 * u];
+      for (int u = 0; u < NB; u++) v[u] = x0 + 32 * u < n ? (T)s[x0 + 32 * u] : (T)0;
     } else {
-      const double *s = m.src + L.base + i0;
+      const double *s = m.src + L.base;
       double t[NB];
 #pragma unroll
-      for (int u = 0; u < NB; u++) {
-        t[u] = 0.0;
-        if (in[u]) t[u] = s[32 * u];
-      }
+      for (int u = 0; u < NB; u++) t[u] = x0 + 32 * u < n ? s[x0 + 32 * u] : 0.0;
 #pragma unroll
       for (int u = 0; u < NB; u++) v[u] = to_arith<T>(t[u]);
     }
     if (m.zc >= 0) {
-      const signed char *z = m.zero + (long)m.zc * m.N + L.base + i0;
+      const signed char *z = m.zero + (long)m.zc * m.N + L.base;
       signed char f[NB];
 #pragma unroll
-      for (int u = 0; u < NB; u++) {
-        f[u] = 0;
-        if (in[u]) f[u] = z[32 * u];
-      }
+      for (int u = 0; u < NB; u++) f[u] = x0 + 32 * u < n ? z[x0 + 32 * u] : (signed char)0;
 #pragma unroll
       for (int u = 0; u < NB; u++)
         if (f[u]) v[u] = 0;
     }
-    const bool neg = __popc(L.refl & m.signmask) & 1;
+    if (__popc(L.refl & m.signmask) & 1) {
 #pragma unroll
-    for (int u = 0; u < NB; u++) {
-      if (neg) v[u] = -v[u];
-      if (!in[u] && x0 + 32 * u < g.ext[0]) v[u] = at(g, L, x0 + 32 * u);
+      for (int u = 0; u < NB; u++) v[u] = -v[u];
     }
   }
 };
@@ -370,7 +367,7 @@ template <class T, class C, class Src, int LO, int HI>
 __global__ void __launch_bounds__((x_pairs_max<C>() * HI + 31) / 32 * 32) k_rfft_lines(SrcBatch<Src, C> sb, XGeom g,
                                                                                Line1d<C> ln, int NP, int lp)
 {
-  const Src &src = sb.src[blockIdx.y];
+  const Src src = sb.src[blockIdx.y];
   C *__restrict__ spec = sb.spec[blockIdx.y];
   extern __shared__ __align__(16) unsigned char smraw[];
   C *sm = reinterpret_cast<C *>(smraw);
@@ -384,13 +381,25 @@ __global__ void __launch_bounds__((x_pairs_max<C>() * HI + 31) / 32 * 32) k_rfft
     const bool r1 = L + 1 < g.nlines && y1 < g.ext[1] && z1 < g.ext[2];
     const typename Src::Line l0 = r0 ? src.line(g, y0, z0) : typename Src::Line{};
     const typename Src::Line l1 = r1 ? src.line(g, y1, z1) : typename Src::Line{};
-    for (int x0 = lane; x0 < n; x0 += 32 * kXBatch) {
-      T a[kXBatch] = {}, b[kXBatch] = {};
-      if (r0) src.template load<kXBatch>(g, l0, x0, a);
-      if (r1) src.template load<kXBatch>(g, l1, x0, b);
+    // the mesh's nodes of both lines, with no test per node but the zero-density flag, then the positions around them
+    const int e0 = src.first(g), nn = src.count(g);
+    C *row = sm + p * lp;
+    for (int x0 = lane; x0 < nn; x0 += 32 * kXBatch) {
+      T a[kXBatch], b[kXBatch];
+      src.template load<kXBatch>(l0, r0, x0, nn, a);
+      src.template load<kXBatch>(l1, r1, x0, nn, b);
 #pragma unroll
       for (int u = 0; u < kXBatch; u++)
-        if (x0 + 32 * u < n) sm[p * lp + x0 + 32 * u] = C{a[u], b[u]};
+        if (x0 + 32 * u < nn) row[e0 + x0 + 32 * u] = C{a[u], b[u]};
+    }
+    for (int t = lane; t < n - nn; t += 32) {
+      const int x = t < e0 ? t : t + nn;
+      C v = C{0, 0};
+      if (x < g.ext[0]) {
+        if (r0) v.x = src.at(g, l0, x);
+        if (r1) v.y = src.at(g, l1, x);
+      }
+      row[x] = v;
     }
   }
   tile_fft<LO, HI, false, C>(sm, NP, lp, ln);

@@ -804,6 +804,136 @@ __device__ __forceinline__ void hess_apply_node_t(const double *x, const double 
   fmt_hess_apply_coef(c, n, y, z, nd, false);
 }
 
+// ---- 3-D forms of the FMT functions --------------------------------------------------------------------------------
+// fmt_dphi_at and fmt_hess_coef_at with the functional and the dimension as constants and the divisions by constants
+// and by powers of one number as products: the per-node kernels of 3-D problems are bound by the FP64 pipe (two
+// operations per SM and clock; a division costs about ten).  1-D and 2-D meshes, bound by launches, keep the general
+// functions, which the host checks share.
+template <int FN>
+__device__ __forceinline__ FmtF fmt_f_t(double n3, double a)
+{
+  constexpr double pi = 3.141592653589793238462643383279502884197;
+  FmtF r;
+  const double a2 = a * a, a3 = a2 * a;
+  if (FN == TGPU_FMT1 || FN == TGPU_FMT2) {
+    constexpr double c0 = 1.0 / (24.0 * pi), c1 = 1.0 / (12.0 * pi), c2 = 1.0 / (4.0 * pi);
+    r.f = a2 * c0;
+    r.f1 = a3 * c1;
+    r.f2 = a2 * a2 * c2;
+  } else {
+    constexpr double c = 1.0 / (36.0 * pi);
+    const double t = n3, one = 1.0 - n3, it = 1.0 / t, it2 = it * it, it3 = it2 * it;
+    const double lg = log(one);
+    const double F = t + one * one * lg, F1 = t - 2.0 * one * lg, F2 = 3.0 + 2.0 * lg;
+    const double G = a2 * it2, G1 = 2.0 * (a3 * it2 - a2 * it3);
+    const double G2 = 6.0 * a2 * it2 * it2 - 8.0 * a3 * it3 + 6.0 * a2 * a2 * it2;
+    r.f = F * G * c;
+    r.f1 = (F1 * G + F * G1) * c;
+    r.f2 = (F2 * G + 2.0 * F1 * G1 + F * G2) * c;
+  }
+  return r;
+}
+
+template <int FN>
+__device__ __forceinline__ void fmt_dphi_3d(const double *n, double *dphi)
+{
+  const double a = 1.0 / (1.0 - n[3]);
+  dphi[0] = log(a);
+  dphi[1] = n[2] * a;
+#pragma unroll
+  for (int d = 0; d < 3; d++) dphi[4 + d] = -n[7 + d] * a;
+  if (fmt_white_bear(FN) && !(n[3] > 1.e-10)) {
+    dphi[2] = dphi[3] = dphi[7] = dphi[8] = dphi[9] = 0.0;
+    return;
+  }
+  const double dot22 = n[7] * n[7] + n[8] * n[8] + n[9] * n[9], dot12 = n[4] * n[7] + n[5] * n[8] + n[6] * n[9];
+  const FmtG g = fmt_g(n[2], dot22, FN);
+  const FmtF f = fmt_f_t<FN>(n[3], a);
+  const double gvf = g.gv * f.f;
+  dphi[2] = n[1] * a + g.g2 * f.f;
+  dphi[3] = n[0] * a + (n[1] * n[2] - dot12) * (a * a) + g.g * f.f1;
+#pragma unroll
+  for (int d = 0; d < 3; d++) dphi[7 + d] = gvf * n[7 + d] - n[4 + d] * a;
+}
+
+template <int FN>
+__device__ __forceinline__ HessCoef fmt_hess_coef_3d(const double *n, bool exact)
+{
+  if (FN == TGPU_FMT2 || FN == TGPU_FMT4) return fmt_hess_coef_at(n, 3, FN, exact);
+  HessCoef c;
+  if (fmt_white_bear(FN) && !(n[3] > 1.e-10)) {
+    c.a = c.a2 = c.h13 = c.h22 = c.h23 = c.h33 = c.ff = c.gvf1 = c.g2vr_f = c.g2vc_f = c.gvv = c.gvv_out = 0.0;
+    return c;
+  }
+  const double Q = n[7] * n[7] + n[8] * n[8] + n[9] * n[9], Pd = n[4] * n[7] + n[5] * n[8] + n[6] * n[9];
+  const double a = 1.0 / (1.0 - n[3]), a2 = a * a;
+  const FmtG g = fmt_g(n[2], Q, FN);
+  const FmtF f = fmt_f_t<FN>(n[3], a);
+  c.a = a;
+  c.a2 = a2;
+  c.h13 = n[2] * a2;
+  c.h22 = g.g22 * f.f;
+  c.h23 = n[1] * a2 + g.g2 * f.f1;
+  c.h33 = n[0] * a2 + 2.0 * (n[1] * n[2] - Pd) * (a2 * a) + g.g * f.f2;
+  c.ff = f.f;
+  c.gvf1 = g.gv * f.f1;
+  c.g2vr_f = c.g2vc_f = g.g2v * f.f;
+  c.gvv = g.gvv;
+  c.gvv_out = g.gvv_out;
+  return c;
+}
+
+// kernel launches by functional in 3-D, the general kernel otherwise
+#define TGPU_BY_FUNCTIONAL(ndim, fn, k3, general)      \
+  do {                                                 \
+    if ((ndim) != 3) { general; }                      \
+    else switch (fn) {                                 \
+      case TGPU_FMT1: { constexpr int FN = TGPU_FMT1; k3; } break; \
+      case TGPU_FMT2: { constexpr int FN = TGPU_FMT2; k3; } break; \
+      case TGPU_FMT3: { constexpr int FN = TGPU_FMT3; k3; } break; \
+      default: { constexpr int FN = TGPU_FMT4; k3; } break;        \
+    }                                                  \
+  } while (0)
+
+__device__ __forceinline__ void load_n3(const double *x, long i, double *n)
+{
+  const long N = c_g.N;
+  const double *rb = x + (long)c_g.first_rb * N + i;
+  n[3] = rb[0];
+  n[2] = rb[N];
+  n[1] = rb[2 * N];
+  n[0] = rb[3 * N];
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    n[7 + d] = rb[(4 + d) * N];
+    n[4 + d] = rb[(7 + d) * N];
+  }
+}
+
+// k_hess_coef and k_hess_coef32 (coef or coef32 may be null) in 3-D: 339 -> 228 us at 128^3 for the FP32 table alone
+template <int FN>
+__global__ void __launch_bounds__(kThreads) k_hess_coef_3d(const double *__restrict__ x, double *__restrict__ coef,
+                                                            float *__restrict__ coef32)
+{
+  const long N = c_g.N;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < N; i += (long)gridDim.x * blockDim.x) {
+    double n[10];
+    load_n3(x, i, n);
+    const HessCoef c = fmt_hess_coef_3d<FN>(n, c_g.jac_exact != 0);
+    const double v[kHessCoef] = {c.a, c.a2, c.h13, c.h22, c.h23, c.h33, c.ff, c.gvf1, c.g2vr_f, c.g2vc_f, c.gvv,
+                                 c.gvv_out};
+    if (coef)
+#pragma unroll
+      for (int k = 0; k < kHessCoef; k++) coef[(long)k * N + i] = v[k];
+    if (coef32) {
+#pragma unroll
+      for (int k = 0; k < kHessCoef; k++) coef32[(long)k * N + i] = (float)v[k];
+#pragma unroll
+      for (int k = 0; k < 10; k++) coef32[(long)(kHessCoef + k) * N + i] = (float)n[k];
+    }
+  }
+}
+
 // coef32, when given, receives the FP32 table of k_hess_coef32 in the same pass
 __global__ void k_hess_coef(const double *__restrict__ x, double *__restrict__ coef, float *__restrict__ coef32)
 {
@@ -822,9 +952,10 @@ __global__ void k_hess_coef(const double *__restrict__ x, double *__restrict__ c
   }
 }
 
-void launch_hess_coef(const double *x, double *coef, cudaStream_t s, float *coef32)
+void launch_hess_coef(int ndim, int fn, const double *x, double *coef, cudaStream_t s, float *coef32)
 {
-  k_hess_coef<<<1184, kThreads, 0, s>>>(x, coef, coef32);
+  TGPU_BY_FUNCTIONAL(ndim, fn, (k_hess_coef_3d<FN><<<1184, kThreads, 0, s>>>(x, coef, coef32)),
+                     (k_hess_coef<<<1184, kThreads, 0, s>>>(x, coef, coef32)));
 }
 
 // Transpose-convolution channels from a weighted-density-shaped vector q (n ordering):
@@ -856,9 +987,32 @@ __global__ void k_fmt_local(const double *__restrict__ x, double *__restrict__ c
   }
 }
 
-void launch_fmt_local(const double *x, double *chan, cudaStream_t s, unsigned *domain)
+// k_fmt_local in 3-D (128^3: 394 -> 338 us, FP64 pipe: a logarithm, a division and about 45 other operations)
+template <int FN>
+__global__ void __launch_bounds__(kThreads) k_fmt_local_3d(const double *__restrict__ x, double *__restrict__ chan,
+                                                            unsigned *__restrict__ domain)
 {
-  k_fmt_local<<<1184, kThreads, 0, s>>>(x, chan, domain);
+  const long N = c_g.N;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < N; i += (long)gridDim.x * blockDim.x) {
+    double n[10], q[10];
+    load_n3(x, i, n);
+    if (domain && n[3] >= 1.0) atomicOr(domain, kDomainN3);
+    fmt_dphi_3d<FN>(n, q);
+    for (int ic = 0; ic < c_g.ncomp; ic++) {
+      const double f = c_g.fac[ic], i4pr = c_g.inv_4pir[ic], i4pr2 = c_g.inv_4pirsq[ic];
+      double *o = chan + (long)ic * 5 * N + i;
+      o[0] = f * (q[0] * i4pr2 + q[1] * i4pr + q[2]);
+#pragma unroll
+      for (int d = 0; d < 3; d++) o[(1 + d) * N] = f * (q[4 + d] * i4pr + q[7 + d]);
+      o[4 * N] = f * q[3];
+    }
+  }
+}
+
+void launch_fmt_local(int ndim, int fn, const double *x, double *chan, cudaStream_t s, unsigned *domain)
+{
+  TGPU_BY_FUNCTIONAL(ndim, fn, (k_fmt_local_3d<FN><<<1184, kThreads, 0, s>>>(x, chan, domain)),
+                     (k_fmt_local<<<1184, kThreads, 0, s>>>(x, chan, domain)));
 }
 
 // The pinned density of a constrained interface: R = ln rho - ln pin_value, J = 1/rho on the diagonal
@@ -867,13 +1021,20 @@ __device__ __forceinline__ bool pin_row(int ic, long i) { return ic == 0 && i ==
 
 __device__ __forceinline__ int row_kind(long i) { return c_g.rowkind ? c_g.rowkind[i] : 0; }
 
+// v == vext_max on the integer pipe (an FP64 comparison takes a slot of the FP64 pipe; no NaN: the field has none)
+__device__ __forceinline__ bool at_vext_max(double v)
+{
+  const long long a = __double_as_longlong(v), b = __double_as_longlong(c_g.vext_max);
+  return a == b || ((a | b) << 1) == 0;
+}
+
 // Euler-Lagrange rows without nonlocal couplings: zero-density rows (R = rho, J = 1), the pinned row and
 // the rows of BULK_ZONE / PB_ZONE nodes
 __device__ __forceinline__ bool zero_row(const double *vext, const signed char *zero, int ic, long i)
 {
   if (pin_row(ic, i)) return true;
   const long k = (long)ic * c_g.N + i;
-  return zero[k] || vext[k] == c_g.vext_max || row_kind(i) != 0;
+  return zero[k] || at_vext_max(vext[k]) || row_kind(i) != 0;
 }
 
 // Of those, the rows R = ln rho - ln c with J = 1/rho: the pinned row (c = pin_value), a BULK_ZONE node's
@@ -884,7 +1045,7 @@ __device__ __forceinline__ bool log_row(const double *vext, const signed char *z
 {
   if (pin_row(ic, i)) return true;
   const long k = (long)ic * c_g.N + i;
-  return !(zero[k] || vext[k] == c_g.vext_max) && row_kind(i) != 0;
+  return !(zero[k] || at_vext_max(vext[k])) && row_kind(i) != 0;
 }
 
 __device__ __forceinline__ double log_row_c(const double *vext, int ic, long i)
@@ -916,13 +1077,42 @@ __device__ __forceinline__ bool dep_rb(int k, int *src, double *c)
   return false;
 }
 
-// domain: when non-null, bit kDomainRho is set where a live Euler-Lagrange row takes log(rho) of rho <= 0
-__global__ void k_assemble(const double *__restrict__ x, const double *__restrict__ vext,
-                           const signed char *__restrict__ zero, const double *__restrict__ conv,
-                           const double *__restrict__ tr, double *__restrict__ R, unsigned *__restrict__ domain)
+// domain: when non-null, bit kDomainRho is set where a live Euler-Lagrange row takes log(rho) of rho <= 0.  ND: the
+// dimension, so that a node's rows are loaded together; the components' chemical potentials are formed once per thread
+// (their logarithm per node cost as much as the row's own).  128^3: 374 -> 241 us, FP64 pipe and memory.
+template <int ND>
+__global__ void __launch_bounds__(kThreads) k_assemble(const double *__restrict__ x, const double *__restrict__ vext,
+                                                        const signed char *__restrict__ zero,
+                                                        const double *__restrict__ conv, const double *__restrict__ tr,
+                                                        double *__restrict__ R, unsigned *__restrict__ domain)
 {
+  constexpr int NRB = 4 + 2 * ND;
+  __shared__ double s_mu[kMaxC];
   const long N = c_g.N;
+  if (threadIdx.x < c_g.ncomp) {
+    const int ic = threadIdx.x;
+    double mu;
+    if (c_g.interface) {
+      mu = -c_g.betamu_if[ic];
+    } else {
+      mu = -log(c_g.rho_b[ic]) - c_g.betamu_hs_ex[ic];
+      if (c_g.attraction) mu -= c_g.betamu_att[ic];
+    }
+    s_mu[ic] = mu;
+  }
+  __syncthreads();
+  int src[NRB];
+  double cd[NRB];
+  bool dep[NRB];
+#pragma unroll
+  for (int k = 0; k < NRB; k++) dep[k] = dep_rb(k, &src[k], &cd[k]);
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < N; i += (long)gridDim.x * blockDim.x) {
+    double rb[NRB], cv[NRB];
+#pragma unroll
+    for (int k = 0; k < NRB; k++) {
+      rb[k] = x[(long)(c_g.first_rb + k) * N + i];
+      cv[k] = dep[k] ? 0.0 : conv[(long)k * N + i];
+    }
     for (int ic = 0; ic < c_g.ncomp; ic++) {
       const int iu = c_g.first_rho + ic;
       const double xi = x[(long)iu * N + i];
@@ -935,27 +1125,18 @@ __global__ void k_assemble(const double *__restrict__ x, const double *__restric
           r = xi;
         }
       } else {
-        double mu;
-        if (c_g.interface) {
-          mu = -c_g.betamu_if[ic];
-        } else {
-          mu = -log(c_g.rho_b[ic]) - c_g.betamu_hs_ex[ic];
-          if (c_g.attraction) mu -= c_g.betamu_att[ic];
-        }
         if (domain && xi <= 0.0) atomicOr(domain, kDomainRho);
-        r = log(xi) + mu + vext[(long)ic * N + i] + tr[(long)ic * N + i];
+        r = log(xi) + s_mu[ic] + vext[(long)ic * N + i] + tr[(long)ic * N + i];
         if (c_g.attraction) r += x[(long)(c_g.first_mf + ic) * N + i];
       }
       R[(long)iu * N + i] = r;
     }
-    for (int k = 0; k < c_g.nrb; k++) {
-      const int iu = c_g.first_rb + k;
-      int src;
-      double c;
-      double r = -x[(long)iu * N + i];
-      if (dep_rb(k, &src, &c)) r += x[(long)(c_g.first_rb + src) * N + i] * c;
-      else r += conv[(long)k * N + i];
-      R[(long)iu * N + i] = r;
+#pragma unroll
+    for (int k = 0; k < NRB; k++) {
+      double r = -rb[k];
+      if (dep[k]) r += rb[k == 2 || k == 3 ? 1 : k >= 4 + ND ? k - ND : k] * cd[k];
+      else r += cv[k];
+      R[(long)(c_g.first_rb + k) * N + i] = r;
     }
     if (c_g.attraction)
       for (int ic = 0; ic < c_g.ncomp; ic++) {
@@ -965,10 +1146,12 @@ __global__ void k_assemble(const double *__restrict__ x, const double *__restric
   }
 }
 
-void launch_assemble(const double *x, const double *vext, const signed char *zero, const double *conv,
+void launch_assemble(int ndim, const double *x, const double *vext, const signed char *zero, const double *conv,
                      const double *tr, double *R, cudaStream_t s, unsigned *domain)
 {
-  k_assemble<<<1184, kThreads, 0, s>>>(x, vext, zero, conv, tr, R, domain);
+  if (ndim == 3) k_assemble<3><<<1184, kThreads, 0, s>>>(x, vext, zero, conv, tr, R, domain);
+  else if (ndim == 2) k_assemble<2><<<1184, kThreads, 0, s>>>(x, vext, zero, conv, tr, R, domain);
+  else k_assemble<1><<<1184, kThreads, 0, s>>>(x, vext, zero, conv, tr, R, domain);
 }
 
 // Schur local step: y1 = A11^-1 u (u = A12 v in conv), then the EL-side
@@ -1024,72 +1207,139 @@ __global__ void k_hess_coef32(const double *__restrict__ x, float *__restrict__ 
   }
 }
 
-void launch_hess_coef32(const double *x, float *coef, cudaStream_t s)
+void launch_hess_coef32(int ndim, int fn, const double *x, float *coef, cudaStream_t s)
 {
-  k_hess_coef32<<<1184, kThreads, 0, s>>>(x, coef);
+  TGPU_BY_FUNCTIONAL(ndim, fn, (k_hess_coef_3d<FN><<<1184, kThreads, 0, s>>>(x, nullptr, coef)),
+                     (k_hess_coef32<<<1184, kThreads, 0, s>>>(x, coef)));
+}
+
+// H y from a node's rows of the FP32 table (state's scalars, V1 and V2 per dimension) in the n ordering.  ALPHA: the
+// functionals whose third term has the alpha form; for the others (FMT1, FMT3) g2v f = -6 f, g_vv f = -h22, no outer
+// product, and a^2 is formed: seven scalars are read instead of twelve.
+template <int ND, bool ALPHA>
+struct Hess32 {
+  float a, h13, h22, h23, h33, ff, gvf1, a2, g2vr, g2vc, gvv, gvvo, V1[ND], V2[ND];
+  __device__ __forceinline__ void load(const float *__restrict__ coef, long N, long i)
+  {
+    const float *c = coef + i;
+    a = c[0];
+    h13 = c[2 * N];
+    h22 = c[3 * N];
+    h23 = c[4 * N];
+    h33 = c[5 * N];
+    ff = c[6 * N];
+    gvf1 = c[7 * N];
+    if (ALPHA) {
+      a2 = c[N];
+      g2vr = c[8 * N];
+      g2vc = c[9 * N];
+      gvv = c[10 * N];
+      gvvo = c[11 * N];
+    }
+#pragma unroll
+    for (int d = 0; d < ND; d++) {
+      V1[d] = c[(long)(kHessCoef + 4 + d) * N];
+      V2[d] = c[(long)(kHessCoef + 4 + ND + d) * N];
+    }
+  }
+  __device__ __forceinline__ void apply(const float *y, float *z) const
+  {
+    const float aa = ALPHA ? a2 : a * a, row = ALPHA ? g2vr : -6.0f * ff, col = ALPHA ? g2vc : row;
+    float Vy = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+    for (int d = 0; d < ND; d++) Vy += V2[d] * y[4 + ND + d];
+#pragma unroll
+    for (int d = 0; d < ND; d++) {
+      const float h3v2 = gvf1 * V2[d] - V1[d] * aa;
+      s3 += h3v2 * y[4 + ND + d] - V2[d] * aa * y[4 + d];
+      z[4 + d] = -V2[d] * aa * y[3] - a * y[4 + ND + d];
+      const float vv = ALPHA ? ff * (gvv * y[4 + ND + d] + gvvo * V2[d] * Vy) : -h22 * y[4 + ND + d];
+      z[4 + ND + d] = col * V2[d] * y[2] + h3v2 * y[3] - a * y[4 + d] + vv;
+    }
+    s2 = row * Vy;
+    z[0] = a * y[3];
+    z[1] = a * y[2] + h13 * y[3];
+    z[2] = a * y[1] + h22 * y[2] + h23 * y[3] + s2;
+    z[3] = a * y[0] + h13 * y[1] + h23 * y[2] + h33 * y[3] + s3;
+  }
+};
+
+// per-component constants of the channels, converted once per block
+__device__ __forceinline__ void local32_constants(float (*s_c)[3])
+{
+  if (threadIdx.x < c_g.ncomp) {
+    s_c[threadIdx.x][0] = (float)c_g.fac[threadIdx.x];
+    s_c[threadIdx.x][1] = (float)c_g.inv_4pir[threadIdx.x];
+    s_c[threadIdx.x][2] = (float)c_g.inv_4pirsq[threadIdx.x];
+  }
+  __syncthreads();
+}
+
+// the channels of H y at node i
+template <int ND>
+__device__ __forceinline__ void write_chan32(const float *z, const float (*s_c)[3], float *__restrict__ chan, long N, long i)
+{
+  for (int ic = 0; ic < c_g.ncomp; ic++) {
+    const float fc = s_c[ic][0], i4pr = s_c[ic][1], i4pr2 = s_c[ic][2];
+    float *o = chan + (long)ic * (ND + 2) * N + i;
+    o[0] = fc * (z[0] * i4pr2 + z[1] * i4pr + z[2]);
+#pragma unroll
+    for (int d = 0; d < ND; d++) o[(long)(1 + d) * N] = fc * (z[4 + d] * i4pr + z[4 + ND + d]);
+    o[(long)(ND + 1) * N] = fc * z[3];
+  }
 }
 
 // k_schur_local with every operand in FP32 storage (conv [nrb + ncomp][N] the stencil sums of A12 v, chan the
-// transposed-sum channels, ymf = -u_MF); ND the dimension, so that the per-node arrays stay in registers, and the
-// per-component constants converted once per thread
-template <int ND>
-__global__ void k_schur_local32(const float *__restrict__ conv, const float *__restrict__ coef,
-                                float *__restrict__ chan, float *__restrict__ ymf)
+// transposed-sum channels, ymf = -u_MF); ND the dimension, so that the per-node arrays stay in registers and a node's
+// loads are issued together.  Bound: memory latency and bandwidth, 100 bytes read and written per node (128^3: 73 ->
+// 38 us with the rows that the functional needs, 5.5 TB/s).
+template <int ND, bool ALPHA>
+__global__ void __launch_bounds__(kThreads) k_schur_local32(const float *__restrict__ conv, const float *__restrict__ coef,
+                                                             float *__restrict__ chan, float *__restrict__ ymf)
 {
   constexpr int NRB = 4 + 2 * ND;
+  __shared__ float s_c[kMaxC][3];
+  local32_constants(s_c);
   const long N = c_g.N;
-  int src_k[NRB];
-  float dep_c[NRB];
-  bool dep[NRB];
-#pragma unroll
-  for (int k = 0; k < NRB; k++) {
-    double cd = 0.0;
-    dep[k] = dep_rb(k, &src_k[k], &cd);
-    dep_c[k] = (float)cd;
-  }
-  const int ncomp = c_g.ncomp;
+  const bool single = c_g.single_size != 0;
+  const float r1 = s_c[0][1], r2 = s_c[0][2];
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < N; i += (long)gridDim.x * blockDim.x) {
-    float ysv[NRB], y[NRB], z[NRB], n[NRB];
+    Hess32<ND, ALPHA> h;
+    h.load(coef, N, i);
+    float u[NRB], y[NRB], z[NRB];
 #pragma unroll
     for (int k = 0; k < NRB; k++)
-      ysv[k] = dep[k] ? -dep_c[k] * conv[(long)src_k[k] * N + i] : -conv[(long)k * N + i];   // -u_dep - B u_ind
-    y[0] = ysv[3]; y[1] = ysv[2]; y[2] = ysv[1]; y[3] = ysv[0];
+      u[k] = single && (k == 2 || k == 3 || k >= 4 + ND) ? 0.f : conv[(long)k * N + i];
+    if (single) {   // -u_dep - B u_ind of the copies n1, n0, V1
+      u[2] = r1 * u[1];
+      u[3] = r2 * u[1];
 #pragma unroll
-    for (int d = 0; d < ND; d++) { y[4 + d] = ysv[4 + ND + d]; y[4 + ND + d] = ysv[4 + d]; }
-#pragma unroll
-    for (int k = 0; k < NRB; k++) n[k] = coef[(long)(kHessCoef + k) * N + i];
-    HessCoefT<float> hc;
-    hc.a = coef[i];
-    hc.a2 = coef[N + i];
-    hc.h13 = coef[2 * N + i];
-    hc.h22 = coef[3 * N + i];
-    hc.h23 = coef[4 * N + i];
-    hc.h33 = coef[5 * N + i];
-    hc.ff = coef[6 * N + i];
-    hc.gvf1 = coef[7 * N + i];
-    hc.g2vr_f = coef[8 * N + i];
-    hc.g2vc_f = coef[9 * N + i];
-    hc.gvv = coef[10 * N + i];
-    hc.gvv_out = coef[11 * N + i];
-    fmt_hess_apply_coef(hc, n, y, z, ND, false);
-    for (int ic = 0; ic < ncomp; ic++) {
-      const float fc = (float)c_g.fac[ic], i4pr = (float)c_g.inv_4pir[ic], i4pr2 = (float)c_g.inv_4pirsq[ic];
-      const long base = (long)ic * (ND + 2);
-      chan[base * N + i] = fc * (z[0] * i4pr2 + z[1] * i4pr + z[2]);
-#pragma unroll
-      for (int d = 0; d < ND; d++) chan[(base + 1 + d) * N + i] = fc * (z[4 + d] * i4pr + z[4 + ND + d]);
-      chan[(base + ND + 1) * N + i] = fc * z[3];
+      for (int d = 0; d < ND; d++) u[4 + ND + d] = r1 * u[4 + d];
     }
+    y[0] = -u[3]; y[1] = -u[2]; y[2] = -u[1]; y[3] = -u[0];
+#pragma unroll
+    for (int d = 0; d < ND; d++) { y[4 + d] = -u[4 + ND + d]; y[4 + ND + d] = -u[4 + d]; }
+    h.apply(y, z);
+    write_chan32<ND>(z, s_c, chan, N, i);
     if (c_g.attraction)
-      for (int ic = 0; ic < ncomp; ic++) ymf[(long)ic * N + i] = -conv[(long)(NRB + ic) * N + i];
+      for (int ic = 0; ic < c_g.ncomp; ic++) ymf[(long)ic * N + i] = -conv[(long)(NRB + ic) * N + i];
   }
 }
 
-void launch_schur_local32(int ndim, const float *conv, const float *coef, float *chan, float *ymf, cudaStream_t s)
+// whole waves of blocks that all have work
+static int node_blocks(long N) { return (int)std::min<long>((N + kThreads - 1) / kThreads, 152L * 8); }
+
+void launch_schur_local32(int ndim, bool alpha, long N, const float *conv, const float *coef, float *chan, float *ymf,
+                          cudaStream_t s)
 {
-  if (ndim == 3) k_schur_local32<3><<<1184, kThreads, 0, s>>>(conv, coef, chan, ymf);
-  else if (ndim == 2) k_schur_local32<2><<<1184, kThreads, 0, s>>>(conv, coef, chan, ymf);
-  else k_schur_local32<1><<<1184, kThreads, 0, s>>>(conv, coef, chan, ymf);
+  const int grid = node_blocks(N);
+  if (ndim == 3) {
+    if (alpha) k_schur_local32<3, true><<<grid, kThreads, 0, s>>>(conv, coef, chan, ymf);
+    else k_schur_local32<3, false><<<grid, kThreads, 0, s>>>(conv, coef, chan, ymf);
+  } else {
+    if (alpha) k_schur_local32<2, true><<<grid, kThreads, 0, s>>>(conv, coef, chan, ymf);
+    else k_schur_local32<2, false><<<grid, kThreads, 0, s>>>(conv, coef, chan, ymf);
+  }
 }
 
 // J v local step: channels of H v_rb for the EL rows.
@@ -1268,67 +1518,50 @@ void launch_rhs_local(const double *x, const double *b, double *chan, double *ym
 
 // k_rhs_local in FP32 storage (the FP32 products' right-hand side b2 - A21 A11^-1 b1: FP32 arithmetic on the FP32
 // table of the state, FP32 channels for the FP32 transposed sums; ymf = -b_MF)
-template <int ND>
-__global__ void k_rhs_local32(const double *__restrict__ b, const float *__restrict__ coef, float *__restrict__ chan,
-                              float *__restrict__ ymf)
+template <int ND, bool ALPHA>
+__global__ void __launch_bounds__(kThreads) k_rhs_local32(const double *__restrict__ b, const float *__restrict__ coef,
+                                                           float *__restrict__ chan, float *__restrict__ ymf)
 {
   constexpr int NRB = 4 + 2 * ND;
+  __shared__ float s_c[kMaxC][3];
+  local32_constants(s_c);
   const long N = c_g.N;
-  int src_k[NRB];
-  float dep_c[NRB];
-  bool dep[NRB];
-#pragma unroll
-  for (int k = 0; k < NRB; k++) {
-    double cd = 0.0;
-    dep[k] = dep_rb(k, &src_k[k], &cd);
-    dep_c[k] = (float)cd;
-  }
-  const int ncomp = c_g.ncomp;
+  const bool single = c_g.single_size != 0;
+  const float r1 = s_c[0][1], r2 = s_c[0][2];
   const double *brb = b + (long)c_g.first_rb * N;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < N; i += (long)gridDim.x * blockDim.x) {
-    float ysv[NRB], y[NRB], z[NRB], n[NRB];
+    Hess32<ND, ALPHA> h;
+    h.load(coef, N, i);
+    float u[NRB], y[NRB], z[NRB];
 #pragma unroll
-    for (int k = 0; k < NRB; k++) {
-      const float bk = (float)brb[(long)k * N + i];
-      ysv[k] = dep[k] ? -bk - dep_c[k] * (float)brb[(long)src_k[k] * N + i] : -bk;
+    for (int k = 0; k < NRB; k++) u[k] = (float)brb[(long)k * N + i];
+    if (single) {
+      u[2] += r1 * u[1];
+      u[3] += r2 * u[1];
+#pragma unroll
+      for (int d = 0; d < ND; d++) u[4 + ND + d] += r1 * u[4 + d];
     }
-    y[0] = ysv[3]; y[1] = ysv[2]; y[2] = ysv[1]; y[3] = ysv[0];
+    y[0] = -u[3]; y[1] = -u[2]; y[2] = -u[1]; y[3] = -u[0];
 #pragma unroll
-    for (int d = 0; d < ND; d++) { y[4 + d] = ysv[4 + ND + d]; y[4 + ND + d] = ysv[4 + d]; }
-#pragma unroll
-    for (int k = 0; k < NRB; k++) n[k] = coef[(long)(kHessCoef + k) * N + i];
-    HessCoefT<float> hc;
-    hc.a = coef[i];
-    hc.a2 = coef[N + i];
-    hc.h13 = coef[2 * N + i];
-    hc.h22 = coef[3 * N + i];
-    hc.h23 = coef[4 * N + i];
-    hc.h33 = coef[5 * N + i];
-    hc.ff = coef[6 * N + i];
-    hc.gvf1 = coef[7 * N + i];
-    hc.g2vr_f = coef[8 * N + i];
-    hc.g2vc_f = coef[9 * N + i];
-    hc.gvv = coef[10 * N + i];
-    hc.gvv_out = coef[11 * N + i];
-    fmt_hess_apply_coef(hc, n, y, z, ND, false);
-    for (int ic = 0; ic < ncomp; ic++) {
-      const float fc = (float)c_g.fac[ic], i4pr = (float)c_g.inv_4pir[ic], i4pr2 = (float)c_g.inv_4pirsq[ic];
-      const long base = (long)ic * (ND + 2);
-      chan[base * N + i] = fc * (z[0] * i4pr2 + z[1] * i4pr + z[2]);
-#pragma unroll
-      for (int d = 0; d < ND; d++) chan[(base + 1 + d) * N + i] = fc * (z[4 + d] * i4pr + z[4 + ND + d]);
-      chan[(base + ND + 1) * N + i] = fc * z[3];
-    }
+    for (int d = 0; d < ND; d++) { y[4 + d] = -u[4 + ND + d]; y[4 + ND + d] = -u[4 + d]; }
+    h.apply(y, z);
+    write_chan32<ND>(z, s_c, chan, N, i);
     if (c_g.attraction)
-      for (int ic = 0; ic < ncomp; ic++) ymf[(long)ic * N + i] = -(float)b[(long)(c_g.first_mf + ic) * N + i];
+      for (int ic = 0; ic < c_g.ncomp; ic++) ymf[(long)ic * N + i] = -(float)b[(long)(c_g.first_mf + ic) * N + i];
   }
 }
 
-void launch_rhs_local32(int ndim, const double *b, const float *coef, float *chan, float *ymf, cudaStream_t s)
+void launch_rhs_local32(int ndim, bool alpha, long N, const double *b, const float *coef, float *chan, float *ymf,
+                        cudaStream_t s)
 {
-  if (ndim == 3) k_rhs_local32<3><<<1184, kThreads, 0, s>>>(b, coef, chan, ymf);
-  else if (ndim == 2) k_rhs_local32<2><<<1184, kThreads, 0, s>>>(b, coef, chan, ymf);
-  else k_rhs_local32<1><<<1184, kThreads, 0, s>>>(b, coef, chan, ymf);
+  const int grid = node_blocks(N);
+  if (ndim == 3) {
+    if (alpha) k_rhs_local32<3, true><<<grid, kThreads, 0, s>>>(b, coef, chan, ymf);
+    else k_rhs_local32<3, false><<<grid, kThreads, 0, s>>>(b, coef, chan, ymf);
+  } else {
+    if (alpha) k_rhs_local32<2, true><<<grid, kThreads, 0, s>>>(b, coef, chan, ymf);
+    else k_rhs_local32<2, false><<<grid, kThreads, 0, s>>>(b, coef, chan, ymf);
+  }
 }
 
 // b2s = b2 - A21 y1 on full Euler-Lagrange rows (the rows' kinds from k_row_info32), b2 elsewhere
@@ -1375,36 +1608,36 @@ void launch_rhs_combine(const double *vext, const signed char *zero, const doubl
 
 // Back substitution x1 = A11^-1 (b1 - A12 x2) (ComputeX1, src/dft_Schur_Epetra_Operator.cpp:135-147);
 // writes the full Newton step dx = [x1; x2].
-__global__ void k_x1(const double *__restrict__ b, const double *__restrict__ conv, const double *__restrict__ x2,
-                     double *__restrict__ dx)
+// One row of unknowns per blockIdx.y, as in k_newton_update (128^3: 132 -> 100 us).
+__global__ void __launch_bounds__(kThreads) k_x1(const double *__restrict__ b, const double *__restrict__ conv,
+                                                  const double *__restrict__ x2, double *__restrict__ dx)
 {
   const long N = c_g.N;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < N; i += (long)gridDim.x * blockDim.x) {
-    double y[kMaxRb];
-    const double *brb = b + (long)c_g.first_rb * N;
-    for (int k = 0; k < c_g.nrb; k++) {
-      int src;
-      double c;
-      y[k] = dep_rb(k, &src, &c) ? brb[(long)k * N + i] : brb[(long)k * N + i] - conv[(long)k * N + i];
-    }
-    for (int k = 0; k < c_g.nrb; k++) {
-      int src;
-      double c;
-      double v = dep_rb(k, &src, &c) ? (-y[k] - c * y[src]) : -y[k];
-      dx[(long)(c_g.first_rb + k) * N + i] = v;
-    }
-    for (int ic = 0; ic < c_g.ncomp; ic++) dx[(long)(c_g.first_rho + ic) * N + i] = x2[(long)ic * N + i];
-    if (c_g.attraction)
-      for (int ic = 0; ic < c_g.ncomp; ic++) {
-        const long k = (long)(c_g.first_mf + ic) * N + i;
-        dx[k] = -(b[k] - conv[(long)(c_g.nrb + ic) * N + i]);
-      }
+  const int iu = blockIdx.y, k = iu - c_g.first_rb;
+  const bool rho = iu < c_g.ncomp, mf = !rho && k >= c_g.nrb;   // (densities, weighted densities, mean fields)
+  int src = 0;
+  double cd = 0.0;
+  const bool dep = !rho && !mf && dep_rb(k, &src, &cd);
+  const double *br = b + (long)iu * N, *bs = b + (long)(c_g.first_rb + src) * N, *cs = conv + (long)src * N;
+  const double *cr = conv + (long)(mf ? c_g.nrb + iu - c_g.first_mf : rho ? 0 : k) * N, *xr = x2 + (long)(rho ? iu : 0) * N;
+  double *o = dx + (long)iu * N;
+  const long i0 = blockIdx.x * (long)blockDim.x + threadIdx.x, st = (long)gridDim.x * blockDim.x;
+  if (rho) {
+#pragma unroll 4
+    for (long i = i0; i < N; i += st) o[i] = xr[i];
+  } else if (dep) {
+#pragma unroll 4
+    for (long i = i0; i < N; i += st) o[i] = -br[i] - cd * (bs[i] - cs[i]);
+  } else {
+#pragma unroll 4
+    for (long i = i0; i < N; i += st) o[i] = -(br[i] - cr[i]);
   }
 }
 
-void launch_x1(const double *b, const double *conv, const double *x2, double *dx, cudaStream_t s)
+void launch_x1(int nunk, long N, const double *b, const double *conv, const double *x2, double *dx, cudaStream_t s)
 {
-  k_x1<<<1184, kThreads, 0, s>>>(b, conv, x2, dx);
+  const dim3 grid((unsigned)std::min<long>((N + kThreads - 1) / kThreads, 1024), (unsigned)nunk);
+  k_x1<<<grid, kThreads, 0, s>>>(b, conv, x2, dx);
 }
 
 // ---------------------------------------------------------------------------
@@ -1420,12 +1653,12 @@ void launch_x1(const double *b, const double *conv, const double *x2, double *dx
 __global__ void k_jtv_local(const double *__restrict__ x, const double *__restrict__ vext,
                             const signed char *__restrict__ zero, const double *__restrict__ w,
                             const double *__restrict__ gel, int gstride_ic, int v2_first,
-                            double *__restrict__ out)
+                            double *__restrict__ out, const double *__restrict__ coef)
 {
   const long N = c_g.N;
   const int nd = c_g.ndim;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < N; i += (long)gridDim.x * blockDim.x) {
-    double g[kMaxRb], n[kMaxRb], z[kMaxRb];
+    double g[kMaxRb], z[kMaxRb];
     for (int k = 0; k < 4 + 2 * nd; k++) g[k] = 0.0;
     for (int ic = 0; ic < c_g.ncomp; ic++) {
       const double *G = gel + (long)ic * gstride_ic * N;
@@ -1440,8 +1673,7 @@ __global__ void k_jtv_local(const double *__restrict__ x, const double *__restri
         g[4 + d] -= c_g.inv_4pir[ic] * gd;
       }
     }
-    load_n(x, i, n);
-    fmt_hess_apply(n, g, z, true);
+    hess_apply_node(x, coef, i, g, z, true);
     // rb columns in solution-vector order: -w_rb + B^T w_dep + z
     double wrb[kMaxRb];
     for (int k = 0; k < c_g.nrb; k++) wrb[k] = w[(long)(c_g.first_rb + k) * N + i];
@@ -1474,9 +1706,9 @@ __global__ void k_jtv_local(const double *__restrict__ x, const double *__restri
 }
 
 void launch_jtv_local(const double *x, const double *vext, const signed char *zero, const double *w,
-                      const double *gel, int gstride_ic, int v2_first, double *out, cudaStream_t s)
+                      const double *gel, int gstride_ic, int v2_first, double *out, const double *coef, cudaStream_t s)
 {
-  k_jtv_local<<<1184, kThreads, 0, s>>>(x, vext, zero, w, gel, gstride_ic, v2_first, out);
+  k_jtv_local<<<1184, kThreads, 0, s>>>(x, vext, zero, w, gel, gstride_ic, v2_first, out, coef);
 }
 
 // Adjoint channels from the rb and MF rows of w, per component jc ([jc][ndim+2][N]):
@@ -2144,45 +2376,50 @@ void launch_newton_frac(const double *x, const double *dx, double floor_frac, do
   k_min_final<<<1, kThreads, 0, s>>>(partial, nblocks, result);
 }
 
+// One row of unknowns per blockIdx.y (a thread keeps one row's loads in flight: 257 -> 105 us at 128^3, 5.8 TB/s).
 // partial != null: also the weighted update norm (a convergence test, <= 1): its quotients in FP32 and its squares
 // summed in FP32 per thread (FP64 divisions per unknown made this kernel FP64-bound); the residual-targeted Newton
 // needs no norm and skips it
-__global__ void k_newton_update(double *__restrict__ x, const double *__restrict__ dx, double frac, double rel,
-                                double abs_tol, double *__restrict__ partial)
+__global__ void __launch_bounds__(kThreads) k_newton_update(double *__restrict__ x, const double *__restrict__ dx,
+                                                             double frac, double rel, double abs_tol,
+                                                             double *__restrict__ partial)
 {
   __shared__ double sh[32];
   const long N = c_g.N;
   const bool norm = partial != nullptr;
+  const int iu = blockIdx.y;
+  const bool is_rho = iu >= c_g.first_rho && iu < c_g.first_rho + c_g.ncomp, is_n3 = iu == c_g.first_rb;
   float s = 0.0f;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < N; i += (long)gridDim.x * blockDim.x)
-    for (int iu = 0; iu < c_g.nunk; iu++) {
-      const long k = (long)iu * N + i;
-      const double xo = x[k], d = dx[k];
-      const double xn = fma(frac, d, xo);
-      if (norm) {
-        float t = (float)(frac * d) / (float)fma(rel, xo, abs_tol);
-        if (fabsf(t) > 1.0e18f) t = 1.0e18f;   // any term above 1 fails the test; NaN passes through to the check
-        s = fmaf(t, t, s);
-      }
-      const bool is_rho = iu >= c_g.first_rho && iu < c_g.first_rho + c_g.ncomp;
-      if (is_rho && xn < 1.e-99) x[k] = 0.1 * xo;
-      else if (iu == c_g.first_rb && xn > 1.0) x[k] = xo + 0.5 * (1.0 - xo);
-      else x[k] = xn;
+  double *xr = x + (long)iu * N;
+  const double *dr = dx + (long)iu * N;
+#pragma unroll 4
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < N; i += (long)gridDim.x * blockDim.x) {
+    const double xo = xr[i], d = dr[i];
+    const double xn = fma(frac, d, xo);
+    if (norm) {
+      float t = (float)(frac * d) / (float)fma(rel, xo, abs_tol);
+      if (fabsf(t) > 1.0e18f) t = 1.0e18f;   // any term above 1 fails the test; NaN passes through to the check
+      s = fmaf(t, t, s);
     }
+    double v = xn;
+    if (is_rho) {
+      if (xn < 1.e-99) v = 0.1 * xo;
+    } else if (is_n3) {
+      if (xn > 1.0) v = xo + 0.5 * (1.0 - xo);
+    }
+    xr[i] = v;
+  }
   if (!norm) return;
   const double sb = block_sum((double)s, sh);
-  if (threadIdx.x == 0) partial[blockIdx.x] = sb;
+  if (threadIdx.x == 0) partial[(long)blockIdx.y * gridDim.x + blockIdx.x] = sb;
 }
 
-void launch_newton_update(double *x, const double *dx, double frac, double rel, double abs_tol, double *partial,
-                          int nblocks, double *result, cudaStream_t s)
+void launch_newton_update(double *x, const double *dx, int nunk, long N, double frac, double rel, double abs_tol,
+                          double *partial, double *result, cudaStream_t s)
 {
-  if (!partial) {
-    k_newton_update<<<nblocks, kThreads, 0, s>>>(x, dx, frac, rel, abs_tol, nullptr);
-    return;
-  }
-  k_newton_update<<<nblocks, kThreads, 0, s>>>(x, dx, frac, rel, abs_tol, partial);
-  k_reduce_rows<<<1, kThreads, 0, s>>>(partial, nblocks, 1, result);
+  const dim3 grid((unsigned)std::min<long>((N + kThreads - 1) / kThreads, 1024), (unsigned)nunk);
+  k_newton_update<<<grid, kThreads, 0, s>>>(x, dx, frac, rel, abs_tol, partial);
+  if (partial) k_reduce_rows<<<1, kThreads, 0, s>>>(partial, (int)(grid.x * grid.y), 1, result);
 }
 
 __global__ void k_norm2(const double *__restrict__ x, long n, double *__restrict__ partial, double *__restrict__ out,

@@ -518,16 +518,18 @@ void launch_conv_slab_ff(const float *in_hi, const float *in_lo, long in_total, 
 constexpr int kSlabTileX = 128, kSlabTileY = 16;
 // domain flags of a fill (launch_fmt_local / launch_assemble with a non-null flag word)
 constexpr unsigned kDomainN3 = 1u, kDomainRho = 2u;
-void launch_fmt_local(const double *x, double *chan, cudaStream_t s, unsigned *domain = nullptr);
-void launch_assemble(const double *x, const double *vext, const signed char *zero, const double *conv,
+void launch_fmt_local(int ndim, int fn, const double *x, double *chan, cudaStream_t s, unsigned *domain = nullptr);
+void launch_assemble(int ndim, const double *x, const double *vext, const signed char *zero, const double *conv,
                      const double *tr, double *R, cudaStream_t s, unsigned *domain = nullptr);
 // coef: the state's Hessian scalars ([kHessCoef][N], launch_hess_coef) or null to evaluate them in place
-void launch_hess_coef(const double *x, double *coef, cudaStream_t s, float *coef32 = nullptr);
+void launch_hess_coef(int ndim, int fn, const double *x, double *coef, cudaStream_t s, float *coef32 = nullptr);
 // FP32 storage variants of the FP32 Schur product: the state's Hessian scalars and weighted densities as FP32 rows
 // [kHessCoef + nrb][N]; the local step and the combination on FP32 sums, channels and transposed sums
-void launch_hess_coef32(const double *x, float *coef, cudaStream_t s);
-void launch_schur_local32(int ndim, const float *conv, const float *coef, float *chan, float *ymf, cudaStream_t s);
-void launch_rhs_local32(int ndim, const double *b, const float *coef, float *chan, float *ymf, cudaStream_t s);
+void launch_hess_coef32(int ndim, int fn, const double *x, float *coef, cudaStream_t s);
+void launch_schur_local32(int ndim, bool alpha, long N, const float *conv, const float *coef, float *chan, float *ymf,
+                          cudaStream_t s);
+void launch_rhs_local32(int ndim, bool alpha, long N, const double *b, const float *coef, float *chan, float *ymf,
+                        cudaStream_t s);
 void launch_rhs_combine32(const signed char *kind, const double *b, const float *tr, const float *ymf, double *b2s,
                           cudaStream_t s);
 void launch_row_info32(const double *x, const double *vext, const signed char *zero, double *inv, signed char *kind,
@@ -563,12 +565,13 @@ void launch_precond(const double *x, const double *vext, const signed char *zero
                     cudaStream_t s);
 void launch_newton_frac(const double *x, const double *dx, double floor_frac, double *partial, int nblocks,
                         double *result, cudaStream_t s);
-void launch_newton_update(double *x, const double *dx, double frac, double rel, double abs, double *partial,
-                          int nblocks, double *result, cudaStream_t s);
+void launch_newton_update(double *x, const double *dx, int nunk, long N, double frac, double rel, double abs,
+                          double *partial, double *result, cudaStream_t s);
 void launch_norm2(const double *x, long n, double *partial, int nblocks, double *result, cudaStream_t s);
 // J^T w local step: A22, A11^T (with B^T), the MF coupling and H g for the rb columns
 void launch_jtv_local(const double *x, const double *vext, const signed char *zero, const double *w,
-                      const double *gel, int gstride_ic, int v2_first, double *out, cudaStream_t s);
+                      const double *gel, int gstride_ic, int v2_first, double *out, const double *coef,
+                      cudaStream_t s);
 void launch_objectives(const double *x, const double *vext, const double *satt, const double *wf, const double *wb,
                        const ObjConst &oc, int ncomp, double *partial, int nblocks, double *result, cudaStream_t s);
 void launch_objective_grad(const double *x, const double *vext, const double *satt, const double *wf,
