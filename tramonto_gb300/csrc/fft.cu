@@ -294,17 +294,19 @@ __global__ void __launch_bounds__(lines_per_cta<C>() * HI) k_fft_lines(PassBatch
       for (int r = 0; r < R; r++) sm[(r * R2 + q) * kLines + l] = v[r];
     });
   __syncthreads();
-  if (q < R1 && live)
+  if (live)
     with_radix<0, HI>(R2, [&](auto rc) {
       constexpr int R = decltype(rc)::value;
-      C v[R];
-#pragma unroll
-      for (int r = 0; r < R; r++) v[r] = sm[(q * R + r) * kLines + l];
-      dft::run<R, INV, C>(v);
-      C *p = out + base + q * es;
       const long step = R1 * es;
+      for (int k = q; k < R1; k += blockDim.x / kLines) {
+        C v[R];
 #pragma unroll
-      for (int r = 0; r < R; r++) p[r * step] = v[r];
+        for (int r = 0; r < R; r++) v[r] = sm[(k * R + r) * kLines + l];
+        dft::run<R, INV, C>(v);
+        C *p = out + base + k * es;
+#pragma unroll
+        for (int r = 0; r < R; r++) p[r * step] = v[r];
+      }
     });
 }
 
@@ -573,6 +575,14 @@ Line1d<C> line_of(const FftAxis &a)
   else return Line1d<C>{a.R1, a.R2, a.d_tw};
 }
 
+// Threads per line of a y or z pass: R2 (every thread has a first step, a few take two second steps) unless that leaves
+// over a quarter of the second step's rounds idle, else R1.  128 = 16 x 8 with eight: twice the CTAs per SM, all of their
+// warps loading (five FP32 forward transforms 26 -> 22 us).
+int line_threads(const FftAxis &a)
+{
+  const int rounds = (a.R1 + a.R2 - 1) / a.R2, slots = rounds * a.R2;
+  return 4 * (slots - a.R1) <= slots ? a.R2 : a.R1;
+}
 template <class C>
 size_t lines_smem(const FftAxis &a) { return sizeof(C) * (size_t)lines_per_cta<C>() * a.n; }
 template <class C>
@@ -655,9 +665,9 @@ void strided_pass_batch(const PassBatch<C> &pb, int nb, const FftPlan &p, int d,
   with_range(ax.R1, [&](auto lo, auto hi) {
     constexpr int LO = decltype(lo)::value, HI = decltype(hi)::value;
     if (inverse)
-      k_fft_lines<C, LO, HI, true><<<grid, kLines * ax.R1, lines_smem<C>(ax), s>>>(pb, X, line_of<C>(ax), es, outer);
+      k_fft_lines<C, LO, HI, true><<<grid, kLines * line_threads(ax), lines_smem<C>(ax), s>>>(pb, X, line_of<C>(ax), es, outer);
     else
-      k_fft_lines<C, LO, HI, false><<<grid, kLines * ax.R1, lines_smem<C>(ax), s>>>(pb, X, line_of<C>(ax), es, outer);
+      k_fft_lines<C, LO, HI, false><<<grid, kLines * line_threads(ax), lines_smem<C>(ax), s>>>(pb, X, line_of<C>(ax), es, outer);
   });
   if (timed) {
     cudaEventRecord(e1, s);
