@@ -395,6 +395,62 @@ void plan_geometry_args(const Ctx *c, int P[3], int nx[3], int h[3], int per[3])
   }
 }
 
+// dimensions whose ends read one boundary value (walls or uniform bulk on both sides); along x a wall and a bulk, or
+// the two bulks of an interface, may differ (the sums' profiles make up for it)
+void share_args(const Ctx *c, int share[3])
+{
+  for (int d = 0; d < 3; d++) {
+    share[d] = 0;
+    if (d >= c->dg.ndim) continue;
+    const int l = c->g.bc[d][0], r = c->g.bc[d][1];
+    const bool flat = (l == TGPU_BC_IN_WALL || l == TGPU_BC_IN_BULK) && (r == TGPU_BC_IN_WALL || r == TGPU_BC_IN_BULK);
+    const bool same = l == r && !(l == TGPU_BC_IN_BULK && c->g.interface == 2);
+    share[d] = flat && (d == 0 || same);
+  }
+}
+
+// [nq][nx0]: the weight of each coefficient's points beyond the low x end, per node (profile of the shared boundary value)
+double *low_end_profile(Ctx *c, const DevStencil &st, const double *d_coef, int nq)
+{
+  const int n = c->dg.nx[0], nd = c->dg.ndim;
+  std::vector<double> coef((size_t)st.L * nq), s((size_t)nq * n, 0.0);
+  ck(cudaMemcpyAsync(coef.data(), d_coef, coef.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "d2h");
+  ck(cudaStreamSynchronize(c->stream), "sync");
+  const int h = c->dg.h[0];
+  std::vector<double> col((size_t)nq * (h + 1), 0.0);   // summed weight per offset -ox
+  for (int k = 0; k < st.L; k++) {
+    const int ox = st.off[(size_t)k * nd];
+    if (ox < 0)
+      for (int q = 0; q < nq; q++) col[(size_t)q * (h + 1) - ox] += coef[(size_t)k * nq + q];
+  }
+  for (int q = 0; q < nq; q++) {
+    double t = 0.0;
+    for (int ix = h - 1; ix >= 0; ix--) {   // offsets -ox > ix
+      t += col[(size_t)q * (h + 1) + ix + 1];
+      if (ix < n) s[(size_t)q * n + ix] = t;
+    }
+  }
+  return upload(s, c->stream);
+}
+
+// value beyond an x end of channel ch of the last pad()
+double x_end_value(const Ctx *c, int ch, int side)
+{
+  return c->g.bc[0][side] == TGPU_BC_IN_BULK ? c->pad_pp->h_bulk[side * c->pad_pp->nch + ch] : 0.0;
+}
+
+// adds channel ch's term to an output's profile: coefficient q of the stencil's forward or transposed table
+void add_profile(const Ctx *c, tgpu::FftProfile &p, const DevStencil &st, bool tr, int q, int ch)
+{
+  if (!c->fft.shared[0]) return;
+  const double d = x_end_value(c, ch, 0) - x_end_value(c, ch, 1);
+  if (d == 0.0) return;
+  const double *s = tr ? st.d_prof_tr : st.d_prof_fwd;
+  if (!s || p.n >= 2) throw Error(TGPU_ERR_STATE, "profile of a shared boundary value");
+  p.s[p.n] = s + (long)q * c->dg.nx[0];
+  p.c[p.n++] = d;
+}
+
 // spectrum (FP64 half spectrum) of coefficient q of a stencil's forward (side 0) or transposed (side 1) table
 void kernel_spectrum(Ctx *c, const DevStencil &st, int side, int q, double *rbox, double2 *spec)
 {
@@ -411,10 +467,18 @@ void ensure_fft(Ctx *c)
   c->fft_state = -1;
   const tgpu::DevGeom &dg = c->dg;
   if (dg.ndim < 2) return;
-  int P[3], nx[3], h[3], per[3];
+  int P[3], nx[3], h[3], per[3], share[3];
   plan_geometry_args(c, P, nx, h, per);
-  if (!tgpu::fft_make_plan(c->fft, P, nx, h, per, dg.ndim, c->stream)) return;
+  share_args(c, share);
+  if (!tgpu::fft_make_plan(c->fft, P, nx, h, per, share, dg.ndim, c->stream)) return;
   c->fft_plan_ok = true;
+  if (share[0] && (c->g.bc[0][0] != c->g.bc[0][1] || c->g.interface == 2))
+    for (int t = 0; t < 3; t++)
+      for (auto &st : c->sten[t]) {
+        if (st.L == 0) continue;
+        if (!st.d_prof_fwd) st.d_prof_fwd = low_end_profile(c, st, st.d_coef_fwd, st.nout_fwd);
+        if (!st.d_prof_tr && st.d_coef_tr) st.d_prof_tr = low_end_profile(c, st, st.d_coef_tr, st.nin_tr);
+      }
   if (dg.ndim != 3) return;   // in 2-D the accurate fills keep the direct FP64 sums
   const long NH = c->fft.NS, NR = c->fft.NR;   // stored half-spectrum points
   // device memory: three work spectra and one spectrum per stencil coefficient
@@ -521,7 +585,8 @@ std::vector<float2 *> &tr_boxes<float2>(Ctx *c) { return c->d_trbox32; }
 // transposed sum: out (+)= the inverse of sum_t (spectrum of channel chs[t]) * kern[t], over channels of the last
 // pad(), in one inverse transform
 template <class C>
-void fft_tr_sum(Ctx *c, const int *chs, const C *const *kern, int n, double *out, bool accumulate = true)
+void fft_tr_sum(Ctx *c, const int *chs, const C *const *kern, int n, double *out, const tgpu::FftProfile &prof,
+                bool accumulate = true)
 {
   if (n > tgpu::fft_max_terms()) throw Error(TGPU_ERR_UNSUPPORTED, "too many channels for one FFT transposed sum");
   std::vector<C *> &boxes = tr_boxes<C>(c);
@@ -544,7 +609,7 @@ void fft_tr_sum(Ctx *c, const int *chs, const C *const *kern, int n, double *out
       return;
     }
   }
-  tgpu::rfft_inverse_products(a.data(), kern, n, work, c->fft, 1.0 / (double)c->fft.NR, out, accumulate, c->stream);
+  tgpu::rfft_inverse_products(a.data(), kern, n, work, c->fft, 1.0 / (double)c->fft.NR, out, accumulate, c->stream, prof);
   c->stats.kernel_launches += 3;
   c->stats.conv_launches++;
 }
@@ -552,16 +617,18 @@ void fft_tr_sum(Ctx *c, const int *chs, const C *const *kern, int n, double *out
 // FFT sums with the stencil's spectra `spec` (FP32 or FP64): forward, one inverse per output of the field's spectrum
 // times the output's kernel; transposed, one inverse of the channels' spectra times their kernels
 template <class C>
-void fft_conv_impl(Ctx *c, int ch0, int nin, const std::vector<C *> &spec, bool tr, double *const *outs, int nout,
-                   C *const *fbox, const C *(*channel)(Ctx *, int))
+void fft_conv_impl(Ctx *c, int ch0, int nin, const DevStencil &st, const std::vector<C *> &spec, bool tr,
+                   double *const *outs, int nout, C *const *fbox, const C *(*channel)(Ctx *, int))
 {
   if (!tr) {
     const C *F = channel(c, ch0);
     {   // every output in one launch per pass
       std::vector<C *> &work = tr_boxes<C>(c);
       while ((int)work.size() < nout) work.push_back(dalloc<C>((size_t)c->fft.NS));
+      std::vector<tgpu::FftProfile> prof(nout, tgpu::FftProfile{});
+      for (int q = 0; q < nout; q++) add_profile(c, prof[q], st, false, q, ch0);
       tgpu::rfft_inverse_batch(F, spec.data(), nout, work.data(), c->fft, 1.0 / (double)c->fft.NR, outs, true,
-                               c->stream);
+                               c->stream, prof.data());
       c->stats.kernel_launches += 3;
     }
     c->stats.conv_launches++;
@@ -572,13 +639,15 @@ void fft_conv_impl(Ctx *c, int ch0, int nin, const std::vector<C *> &spec, bool 
       chs[t] = ch0 + t;
       k[t] = spec[t];
     }
-    fft_tr_sum<C>(c, chs.data(), k.data(), nin, outs[0]);
+    tgpu::FftProfile prof{};
+    for (int t = 0; t < nin; t++) add_profile(c, prof, st, true, t, ch0 + t);
+    fft_tr_sum<C>(c, chs.data(), k.data(), nin, outs[0], prof);
   }
 }
 
 void fft_conv32(Ctx *c, int ch0, int nin, const DevStencil &st, bool tr, double *const *outs, int nout)
 {
-  fft_conv_impl<float2>(c, ch0, nin, tr ? st.spec_tr32 : st.spec_fwd32, tr, outs, nout, c->d_fbox32, fft_channel32);
+  fft_conv_impl<float2>(c, ch0, nin, st, tr ? st.spec_tr32 : st.spec_fwd32, tr, outs, nout, c->d_fbox32, fft_channel32);
 }
 
 // FP32 FFT for this sum: the attraction stencil by its context's choice (tensor-core products or FP32 slab
@@ -594,7 +663,7 @@ bool use_fft32(const Ctx *c, const DevStencil &st, bool tr, int nin, int nout)
 
 void fft_conv(Ctx *c, int ch0, int nin, const DevStencil &st, bool tr, double *const *outs, int nout)
 {
-  fft_conv_impl<double2>(c, ch0, nin, tr ? st.spec_tr : st.spec_fwd, tr, outs, nout, c->d_fbox, fft_channel);
+  fft_conv_impl<double2>(c, ch0, nin, st, tr ? st.spec_tr : st.spec_fwd, tr, outs, nout, c->d_fbox, fft_channel);
 }
 
 void conv(Ctx *c, int ch0, int nin, const DevStencil &st, bool tr, double *const *outs, int nout, bool f32)
@@ -805,7 +874,10 @@ void forward_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, boo
       std::vector<const double2 *> ks;
       std::vector<const float2 *> ks32;
       std::vector<double *> os;
+      std::vector<tgpu::FftProfile> prof;
       auto add = [&](const DevStencil &st, int q, double *o) {
+        prof.push_back(tgpu::FftProfile{});
+        add_profile(c, prof.back(), st, false, q, jc);
         if (f32) ks32.push_back(st.spec_fwd32[q]);
         else ks.push_back(st.spec_fwd[q]);
         os.push_back(o);
@@ -826,13 +898,13 @@ void forward_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, boo
           for (double *o : os) os32.push_back(c->d_conv32 + (o - c->d_conv));
           tgpu::rfft_inverse_batch(F, ks32.data(), n, work.data(), c->fft, scale, os32.data(), acc, c->stream);
         } else {
-          tgpu::rfft_inverse_batch(F, ks32.data(), n, work.data(), c->fft, scale, os.data(), acc, c->stream);
+          tgpu::rfft_inverse_batch(F, ks32.data(), n, work.data(), c->fft, scale, os.data(), acc, c->stream, prof.data());
         }
       } else {
         const double2 *F = fft_channel(c, jc);
         std::vector<double2 *> &work = tr_boxes<double2>(c);
         while ((int)work.size() < n) work.push_back(dalloc<double2>((size_t)c->fft.NS));
-        tgpu::rfft_inverse_batch(F, ks.data(), n, work.data(), c->fft, scale, os.data(), acc, c->stream);
+        tgpu::rfft_inverse_batch(F, ks.data(), n, work.data(), c->fft, scale, os.data(), acc, c->stream, prof.data());
       }
       c->stats.kernel_launches += 3 * ((n + tgpu::fft_max_batch() - 1) / tgpu::fft_max_batch());
       c->stats.conv_launches++;
@@ -872,16 +944,19 @@ void transpose_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, b
     int chs[tgpu::kMaxRb];
     for (int t = 0; t < nd + 2; t++) chs[t] = base + t;
     if (sten == c->sten && tr_all_fft(c, ic, f32)) {
+      tgpu::FftProfile prof{};
+      for (int t = 0; t <= nd; t++) add_profile(c, prof, sd, true, t, chs[t]);
+      add_profile(c, prof, st, true, 0, chs[nd + 1]);
       if (f32) {
         const float2 *k[tgpu::kMaxRb];
         for (int t = 0; t <= nd; t++) k[t] = sd.spec_tr32[t];
         k[nd + 1] = st.spec_tr32[0];
-        fft_tr_sum<float2>(c, chs, k, nd + 2, o[0], !fresh);
+        fft_tr_sum<float2>(c, chs, k, nd + 2, o[0], prof, !fresh);
       } else {
         const double2 *k[tgpu::kMaxRb];
         for (int t = 0; t <= nd; t++) k[t] = sd.spec_tr[t];
         k[nd + 1] = st.spec_tr[0];
-        fft_tr_sum<double2>(c, chs, k, nd + 2, o[0], !fresh);
+        fft_tr_sum<double2>(c, chs, k, nd + 2, o[0], prof, !fresh);
       }
       continue;
     }
@@ -2900,6 +2975,7 @@ int tgpu_destroy(tgpu_handle h)
       for (auto &st : c->sten[t]) {
         dfree(st.d_loff); dfree(st.d_loff_neg); dfree(st.d_off); dfree(st.d_w); dfree(st.d_hw);
         dfree(st.d_coef_fwd); dfree(st.d_coef_fwd32); dfree(st.d_coef_tr); dfree(st.d_coef_tr32); dfree(st.d_coef_adj);
+        dfree(st.d_prof_fwd); dfree(st.d_prof_tr);
         for (auto *L : {&st.lines_fwd, &st.lines_tr}) {
           dfree(L->d_planes); dfree(L->d_lines); dfree(L->d_w); dfree(L->d_w_lo);
         }

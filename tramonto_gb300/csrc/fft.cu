@@ -5,8 +5,11 @@
 // correlation.  Along a periodic dimension of n nodes it is exactly the circular correlation of period n; along
 // any other dimension the padded channel (the field extended by the boundary rules over the stencil's reach h)
 // is transformed on a length F >= P = n + 2h, where the circular correlation equals the sum for every interior
-// output.  So the transform box is [F2][F1][F0] with F_d = n_d on periodic dimensions (when n_d is a product of
-// 2, 3, 5 and 7) and the smallest such F_d >= P_d elsewhere; with the correlation kernel g[(-o) mod F] = c(o)
+// output.  Where the field has one boundary value beyond both ends (walls, bulk), F >= n + h is enough: the positions
+// from n on hold that value and serve the reads beyond either end.  Along x the two ends may differ (a wall and a bulk):
+// the box holds the high end's value and the outputs next to the low end take the difference times the stencil's weight
+// beyond it, a profile in x.  So the transform box is [F2][F1][F0] with F_d = n_d on periodic dimensions (when n_d is a
+// product of 2, 3, 5 and 7) and the smallest such F_d >= P_d elsewhere; with the correlation kernel g[(-o) mod F] = c(o)
 // (points that wrap onto the same position add up, as the reference folds a stencil wider than a periodic box),
 // one forward transform of the field, a product with the kernel's spectrum and one inverse transform give the
 // sum at a cost that does not depend on the stencil's length.  At 128^3 with the attraction reach of 25 nodes
@@ -94,13 +97,15 @@ struct XGeom {
   int off[3], ext[3];
   // inverse destination: box position p holds output node p - e (interior nodes only)
   int e[3], nx[3];
+  int last[3];               // last padded position (box positions past it read the same boundary value)
+  int flat0;                 // x holds the nodes, then one boundary value to the end
 };
 
 // Sources of the forward x pass: element (x, y, z) of the real box (x < ext0, y < ext1, z < ext2; 0 beyond)
 // at padded position (x + off0, y + off1, z + off2).  A line's y and z are resolved once (line); load then takes its
 // elements first + x0, + 32, ..., all loads issued before their values are used, and at() any position around them.
 template <class T>
-struct BoxSrc {   // a padded channel, or a real box [F2][F1][F0] (off 0)
+struct BoxSrc {   // a real box [F2][F1][F0] (off 0)
   const T *p;
   long sy, sz;
   using Line = const T *;
@@ -118,6 +123,7 @@ struct BoxSrc {   // a padded channel, or a real box [F2][F1][F0] (off 0)
     for (int u = 0; u < NB; u++) v[u] = use && x0 + 32 * u < n ? L[x0 + 32 * u] : (T)0;
   }
   __device__ __forceinline__ T at(const XGeom &, const Line &L, int x) const { return L[x]; }
+  __device__ __forceinline__ T flat(const XGeom &) const { return (T)0; }
 };
 template <class T>
 struct MappedSrc {   // the unpadded channel through the boundary maps (the padded box's values, computed)
@@ -134,7 +140,7 @@ struct MappedSrc {   // the unpadded channel through the boundary maps (the padd
   __device__ __forceinline__ Line line(const XGeom &g, int y, int z) const
   {
     Line L{0, 0, 0};
-    const int q[3] = {0, y + g.off[1], z + g.off[2]};
+    const int q[3] = {0, min(y + g.off[1], g.last[1]), min(z + g.off[2], g.last[2])};
     long idx[3] = {0, 0, 0};
     for (int d = 1; d < m.ndim; d++) {
       const int v = m.map[d][q[d]];
@@ -157,7 +163,7 @@ struct MappedSrc {   // the unpadded channel through the boundary maps (the padd
   }
   __device__ __forceinline__ T at(const XGeom &g, const Line &L, int x) const
   {
-    const int v = m.map[0][x + g.off[0]], out = v < 0 ? v : L.sent;
+    const int v = m.map[0][min(x + g.off[0], g.last[0])], out = v < 0 ? v : L.sent;
     if (out) return sentinel(out);
     const int refl = L.refl | ((v & kReflBit) ? 1 : 0);
     const long node = L.base + (v & ~kReflBit);
@@ -165,6 +171,8 @@ struct MappedSrc {   // the unpadded channel through the boundary maps (the padd
     if (m.zc >= 0 && m.zero[(long)m.zc * m.N + node]) return (T)0;
     return (__popc(refl & m.signmask) & 1) ? -val : val;
   }
+  // the boundary value that follows the nodes of a flat x (x decides first: also on lines outside the mesh)
+  __device__ __forceinline__ T flat(const XGeom &g) const { return sentinel(m.map[0][g.last[0]]); }
   // the mesh's nodes: the box holds node i at x = e[0] + i, with no map to read
   __device__ __forceinline__ int first(const XGeom &g) const { return g.e[0]; }
   __device__ __forceinline__ int count(const XGeom &) const { return m.nx[0]; }
@@ -235,6 +243,7 @@ struct OutBatch {
   const C *spec[kMaxBatch];
   double *out[kMaxBatch];
   float *out32[kMaxBatch];   // FP32 outputs (the FP32 transforms; used instead of out when set)
+  FftProfile prof[kMaxBatch];
 };
 
 // ---- y and z passes ---------------------------------------------------------------------------------------------
@@ -246,8 +255,8 @@ struct OutBatch {
 // writes `out` (in place when out == in: a CTA has read its lines before it writes them).  R1 in (LO, HI]: one kernel
 // per range of radices, so that short ones do not carry the registers of long ones.
 template <class C, int LO, int HI, bool INV>
-__global__ void __launch_bounds__(lines_per_cta<C>() * HI) k_fft_lines(PassBatch<C> pb, int X, Line1d<C> ln, long es,
-                                                         long outer_stride)
+__global__ void __launch_bounds__(lines_per_cta<C>() * HI) k_fft_lines(PassBatch<C> pb, int X, unsigned nlines,
+                                                                           Line1d<C> ln, long es, long outer_stride)
 {
   extern __shared__ __align__(16) unsigned char smraw[];
   constexpr int kLines = lines_per_cta<C>();
@@ -256,10 +265,23 @@ __global__ void __launch_bounds__(lines_per_cta<C>() * HI) k_fft_lines(PassBatch
   C *out = pb.out[blockIdx.y];
   const int l = threadIdx.x & (kLines - 1), q = threadIdx.x / kLines;
   const int R1 = ln.R1, R2 = ln.R2;
-  const int xblocks = (X + kLines - 1) / kLines;
-  const int x0 = (blockIdx.x % xblocks) * kLines;
-  const long base = (long)(blockIdx.x / xblocks) * outer_stride + x0 + l;
-  const bool live = x0 + l < X;
+  // FP64 (bound by its arithmetic): lines numbered through the outer indices, so that only the last CTA has idle ones.
+  // FP32 (bound by its accesses): CTAs start at multiples of 16 in x, on 128-byte boundaries (81 x 128 x 128 points, a
+  // forward pass of one and five transforms: 12.6 us; numbered through 14.0; FP64 172 and 161 us).
+  unsigned o, x;
+  bool live;
+  if constexpr (std::is_same<C, double2>::value) {
+    const unsigned line = blockIdx.x * kLines + l;
+    o = line / (unsigned)X;
+    x = line - o * X;
+    live = line < nlines;
+  } else {
+    const unsigned xblocks = (X + kLines - 1) / kLines;
+    o = blockIdx.x / xblocks;
+    x = (blockIdx.x - o * xblocks) * kLines + l;
+    live = x < (unsigned)X;
+  }
+  const long base = (long)o * outer_stride + x;
   if (q < R2 && live)
     with_radix<LO, HI>(R1, [&](auto rc) {
       constexpr int R = decltype(rc)::value;
@@ -375,6 +397,7 @@ __global__ void __launch_bounds__((x_pairs_max<C>() * HI + 31) / 32 * 32) k_rfft
   C *sm = reinterpret_cast<C *>(smraw);
   const int n = g.F0, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int npairs = (int)((g.nlines + 1) / 2), pair0 = blockIdx.x * NP, np = min(NP, npairs - pair0);
+  const T beyond = g.flat0 ? src.flat(g) : (T)0;
   for (int p = warp; p < np; p += nw) {
     const int L = 2 * (pair0 + p);
     const int z0 = L / g.F1, y0 = L - z0 * g.F1, y1 = y0 + 1 < g.F1 ? y0 + 1 : 0, z1 = y0 + 1 < g.F1 ? z0 : z0 + 1;
@@ -393,6 +416,11 @@ __global__ void __launch_bounds__((x_pairs_max<C>() * HI + 31) / 32 * 32) k_rfft
 #pragma unroll
       for (int u = 0; u < kXBatch; u++)
         if (x0 + 32 * u < nn) row[e0 + x0 + 32 * u] = C{a[u], b[u]};
+    }
+    if (g.flat0) {
+      const C v = C{r0 ? beyond : (T)0, r1 ? beyond : (T)0};
+      for (int x = nn + lane; x < n; x += 32) row[x] = v;
+      continue;
     }
     for (int t = lane; t < n - nn; t += 32) {
       const int x = t < e0 ? t : t + nn;
@@ -419,7 +447,8 @@ __global__ void __launch_bounds__((x_pairs_max<C>() * HI + 31) / 32 * 32) k_rfft
 
 // one output line: out = scale * value (+ out when accumulate), every load before the stores
 template <class T, class O, class C>
-__device__ __forceinline__ void write_line(const C *z, bool imag, O *o, int nx0, T sc, bool accumulate, int lane)
+__device__ __forceinline__ void write_line(const C *z, bool imag, O *o, int nx0, T sc, bool accumulate,
+                                           const FftProfile &prof, int lane)
 {
   for (int x0 = lane; x0 < nx0; x0 += 32 * kXBatch) {
     O old[kXBatch];
@@ -429,7 +458,9 @@ __device__ __forceinline__ void write_line(const C *z, bool imag, O *o, int nx0,
     for (int u = 0; u < kXBatch; u++)
       if (x0 + 32 * u < nx0) {
         const C r = z[x0 + 32 * u];
-        const O v = (O)(sc * (imag ? r.y : r.x));   // scaled in the transform's arithmetic
+        O v = (O)(sc * (imag ? r.y : r.x));   // scaled in the transform's arithmetic
+        if (prof.n > 0) v += (O)(prof.c[0] * prof.s[0][x0 + 32 * u]);
+        if (prof.n > 1) v += (O)(prof.c[1] * prof.s[1][x0 + 32 * u]);
         o[x0 + 32 * u] = accumulate ? old[u] + v : v;
       }
   }
@@ -462,6 +493,7 @@ __global__ void __launch_bounds__((x_pairs_max<C>() * HI + 31) / 32 * 32) k_irff
   tile_fft<LO, HI, true, C>(sm, NP, lp, ln);
   const int nx0 = g.nx[0];
   const T sc = (T)scale;
+  const FftProfile prof = ob.prof[blockIdx.y];
   for (int p = warp; p < np; p += nw) {
     const int L = 2 * (pair0 + p);
 #pragma unroll
@@ -472,9 +504,9 @@ __global__ void __launch_bounds__((x_pairs_max<C>() * HI + 31) / 32 * 32) k_irff
       const long row = ((long)z * g.nx[1] + y) * nx0;
       const C *zl = sm + p * lp + g.e[0];
       if (std::is_same<C, float2>::value && ob.out32[blockIdx.y])
-        write_line<T, float>(zl, h != 0, ob.out32[blockIdx.y] + row, nx0, sc, accumulate != 0, lane);
+        write_line<T, float>(zl, h != 0, ob.out32[blockIdx.y] + row, nx0, sc, accumulate != 0, prof, lane);
       else
-        write_line<T, double>(zl, h != 0, ob.out[blockIdx.y] + row, nx0, sc, accumulate != 0, lane);
+        write_line<T, double>(zl, h != 0, ob.out[blockIdx.y] + row, nx0, sc, accumulate != 0, prof, lane);
     }
   }
 }
@@ -629,7 +661,9 @@ XGeom xgeom(const FftPlan &p)
     g.ext[d] = p.ext[d];
     g.e[d] = p.h[d] - p.off[d];
     g.nx[d] = p.nx[d];
+    g.last[d] = p.P[d] - 1;
   }
+  g.flat0 = p.shared[0];
   return g;
 }
 
@@ -654,7 +688,9 @@ void strided_pass_batch(const PassBatch<C> &pb, int nb, const FftPlan &p, int d,
   const long nouter = d == 1 ? p.F[2] : p.F[1];
   const FftAxis &ax = p.ax[d];
   constexpr int kLines = lines_per_cta<C>();
-  const dim3 grid((unsigned)((X + kLines - 1) / kLines * nouter), (unsigned)nb);
+  const long nlines = X * nouter;
+  const long blocks = std::is_same<C, double2>::value ? (nlines + kLines - 1) / kLines : (X + kLines - 1) / kLines * nouter;
+  const dim3 grid((unsigned)blocks, (unsigned)nb);
   const bool timed = std::is_same<C, float2>::value && g_pass_timer.on;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (timed) {
@@ -665,9 +701,9 @@ void strided_pass_batch(const PassBatch<C> &pb, int nb, const FftPlan &p, int d,
   with_range(ax.R1, [&](auto lo, auto hi) {
     constexpr int LO = decltype(lo)::value, HI = decltype(hi)::value;
     if (inverse)
-      k_fft_lines<C, LO, HI, true><<<grid, kLines * line_threads(ax), lines_smem<C>(ax), s>>>(pb, X, line_of<C>(ax), es, outer);
+      k_fft_lines<C, LO, HI, true><<<grid, kLines * line_threads(ax), lines_smem<C>(ax), s>>>(pb, X, (unsigned)nlines, line_of<C>(ax), es, outer);
     else
-      k_fft_lines<C, LO, HI, false><<<grid, kLines * line_threads(ax), lines_smem<C>(ax), s>>>(pb, X, line_of<C>(ax), es, outer);
+      k_fft_lines<C, LO, HI, false><<<grid, kLines * line_threads(ax), lines_smem<C>(ax), s>>>(pb, X, (unsigned)nlines, line_of<C>(ax), es, outer);
   });
   if (timed) {
     cudaEventRecord(e1, s);
@@ -720,13 +756,15 @@ void strided_pass(const C *in, C *out, const Terms<C> &terms, const FftPlan &p, 
 }
 
 template <class T, class C, class Src>
-void rfft_forward_impl(const Src &src, bool padded, C *spec, const FftPlan &p, cudaStream_t s)
+void rfft_forward_impl(const Src &src, bool mapped, C *spec, const FftPlan &p, cudaStream_t s)
 {
   XGeom g = xgeom(p);
-  if (!padded)   // a real box [F2][F1][F0]
+  if (!mapped)   // a real box [F2][F1][F0]
     for (int d = 0; d < 3; d++) {
       g.off[d] = 0;
       g.ext[d] = p.F[d];
+      g.last[d] = p.F[d] - 1;
+      g.flat0 = 0;
     }
   SrcBatch<Src, C> sb{};
   sb.src[0] = src;
@@ -740,7 +778,7 @@ void rfft_forward_impl(const Src &src, bool padded, C *spec, const FftPlan &p, c
 // inverse of the products in `terms`, formed by the first inverse pass into `spec` (the work box)
 template <class C>
 void rfft_inverse_impl(const Terms<C> &terms, C *spec, const FftPlan &p, double scale, double *out, float *out32,
-                       bool accumulate, cudaStream_t s)
+                       bool accumulate, const FftProfile &prof, cudaStream_t s)
 {
   const Terms<C> none{};
   // A sum of several FP32 products is formed by a pass of its own (five terms at 128^3: 24 + 9 us; 70 us inside the
@@ -756,6 +794,7 @@ void rfft_inverse_impl(const Terms<C> &terms, C *spec, const FftPlan &p, double 
   ob.spec[0] = spec;
   ob.out[0] = out;
   ob.out32[0] = out32;
+  ob.prof[0] = prof;
   inverse_x<C>(ob, 1, p, scale, accumulate, s);
 }
 
@@ -779,7 +818,8 @@ void rfft_forward_mapped_batch_impl(const MapSrc *m, int nb, C *const *spec, con
 // nb inverse transforms, output b the inverse of a * k[b] (formed by the first inverse pass in work[b])
 template <class C>
 void rfft_inverse_batch_impl(const C *a, const C *const *k, int nb, C *const *work, const FftPlan &p, double scale,
-                             double *const *out, float *const *out32, bool accumulate, cudaStream_t s)
+                             double *const *out, float *const *out32, bool accumulate, const FftProfile *prof,
+                             cudaStream_t s)
 {
   PassBatch<C> pb{}, plain{};
   OutBatch<C> ob{};
@@ -792,6 +832,7 @@ void rfft_inverse_batch_impl(const C *a, const C *const *k, int nb, C *const *wo
     ob.spec[b] = work[b];
     ob.out[b] = out ? out[b] : nullptr;
     ob.out32[b] = out32 ? out32[b] : nullptr;
+    if (prof) ob.prof[b] = prof[b];
   }
   bool pending = true;
   for (int d = 2; d >= 1; d--) {
@@ -806,12 +847,13 @@ void rfft_inverse_batch_impl(const C *a, const C *const *k, int nb, C *const *wo
 
 }  // namespace
 
-bool fft_make_plan(FftPlan &p, const int P[3], const int nx[3], const int h[3], const int periodic[3], int ndim,
-                   cudaStream_t s)
+bool fft_make_plan(FftPlan &p, const int P[3], const int nx[3], const int h[3], const int periodic[3],
+                   const int share[3], int ndim, cudaStream_t s)
 {
   p.NR = 1;
   for (int d = 0; d < 3; d++) {
     FftAxis &a = p.ax[d];
+    p.shared[d] = 0;
     p.P[d] = d < ndim ? P[d] : 1;
     p.nx[d] = d < ndim ? nx[d] : 1;
     p.h[d] = d < ndim ? h[d] : 0;
@@ -833,6 +875,13 @@ bool fft_make_plan(FftPlan &p, const int P[3], const int nx[3], const int h[3], 
       p.F[d] = F;
       p.off[d] = 0;
       p.ext[d] = P[d];
+      if (share[d]) {   // node i at box position i, the shared boundary value from nx on
+        F = p.nx[d] + p.h[d];
+        while (!radices_of(F, a.R1, a.R2)) F++;
+        p.F[d] = p.ext[d] = F;
+        p.off[d] = p.h[d];
+        p.shared[d] = 1;
+      }
     }
     a.n = p.F[d];
     std::vector<double2> tw(a.n);
@@ -869,16 +918,6 @@ void fft_free_plan(FftPlan &p)
   }
 }
 
-void rfft_forward(const double *pad, double2 *spec, const FftPlan &p, cudaStream_t s)
-{
-  rfft_forward_impl<double, double2>(BoxSrc<double>{pad, p.P[0], (long)p.P[0] * p.P[1]}, true, spec, p, s);
-}
-
-void rfft_forward(const float *pad, float2 *spec, const FftPlan &p, cudaStream_t s)
-{
-  rfft_forward_impl<float, float2>(BoxSrc<float>{pad, p.P[0], (long)p.P[0] * p.P[1]}, true, spec, p, s);
-}
-
 void rfft_forward_mapped(const MapSrc &m, double2 *spec, const FftPlan &p, cudaStream_t s)
 {
   rfft_forward_impl<double, double2>(MappedSrc<double>(m), true, spec, p, s);
@@ -907,21 +946,23 @@ Terms<C> make_terms(const C *const *a, const C *const *k, int n)
 }
 
 void rfft_inverse_products(const double2 *const *a, const double2 *const *k, int nterms, double2 *work,
-                           const FftPlan &p, double scale, double *out, bool accumulate, cudaStream_t s)
+                           const FftPlan &p, double scale, double *out, bool accumulate, cudaStream_t s,
+                           const FftProfile &prof)
 {
-  rfft_inverse_impl<double2>(make_terms(a, k, nterms), work, p, scale, out, nullptr, accumulate, s);
+  rfft_inverse_impl<double2>(make_terms(a, k, nterms), work, p, scale, out, nullptr, accumulate, prof, s);
 }
 
 void rfft_inverse_products(const float2 *const *a, const float2 *const *k, int nterms, float2 *work,
-                           const FftPlan &p, double scale, double *out, bool accumulate, cudaStream_t s)
+                           const FftPlan &p, double scale, double *out, bool accumulate, cudaStream_t s,
+                           const FftProfile &prof)
 {
-  rfft_inverse_impl<float2>(make_terms(a, k, nterms), work, p, scale, out, nullptr, accumulate, s);
+  rfft_inverse_impl<float2>(make_terms(a, k, nterms), work, p, scale, out, nullptr, accumulate, prof, s);
 }
 
 void rfft_inverse_products(const float2 *const *a, const float2 *const *k, int nterms, float2 *work,
                            const FftPlan &p, double scale, float *out, bool accumulate, cudaStream_t s)
 {
-  rfft_inverse_impl<float2>(make_terms(a, k, nterms), work, p, scale, nullptr, out, accumulate, s);
+  rfft_inverse_impl<float2>(make_terms(a, k, nterms), work, p, scale, nullptr, out, accumulate, FftProfile{}, s);
 }
 
 int fft_max_terms() { return kMaxTerms; }
@@ -940,11 +981,11 @@ void rfft_forward_mapped_batch(const MapSrc *m, int nb, double2 *const *spec, co
 }
 
 void rfft_inverse_batch(const float2 *a, const float2 *const *k, int nb, float2 *const *work, const FftPlan &p,
-                        double scale, double *const *out, bool accumulate, cudaStream_t s)
+                        double scale, double *const *out, bool accumulate, cudaStream_t s, const FftProfile *prof)
 {
   for (int b0 = 0; b0 < nb; b0 += kMaxBatch)
     rfft_inverse_batch_impl<float2>(a, k + b0, std::min(kMaxBatch, nb - b0), work + b0, p, scale, out + b0, nullptr,
-                                    accumulate, s);
+                                    accumulate, prof ? prof + b0 : nullptr, s);
 }
 
 void rfft_inverse_batch(const float2 *a, const float2 *const *k, int nb, float2 *const *work, const FftPlan &p,
@@ -952,15 +993,15 @@ void rfft_inverse_batch(const float2 *a, const float2 *const *k, int nb, float2 
 {
   for (int b0 = 0; b0 < nb; b0 += kMaxBatch)
     rfft_inverse_batch_impl<float2>(a, k + b0, std::min(kMaxBatch, nb - b0), work + b0, p, scale, nullptr, out + b0,
-                                    accumulate, s);
+                                    accumulate, nullptr, s);
 }
 
 void rfft_inverse_batch(const double2 *a, const double2 *const *k, int nb, double2 *const *work, const FftPlan &p,
-                        double scale, double *const *out, bool accumulate, cudaStream_t s)
+                        double scale, double *const *out, bool accumulate, cudaStream_t s, const FftProfile *prof)
 {
   for (int b0 = 0; b0 < nb; b0 += kMaxBatch)
     rfft_inverse_batch_impl<double2>(a, k + b0, std::min(kMaxBatch, nb - b0), work + b0, p, scale, out + b0, nullptr,
-                                     accumulate, s);
+                                     accumulate, prof ? prof + b0 : nullptr, s);
 }
 
 void fft_pass(double2 *spec, const FftPlan &p, int d, bool inverse, cudaStream_t s)

@@ -66,7 +66,8 @@ constexpr double kDensityMin = 1.e-20;   // integrands vanish at or below this d
 // betamu and the bulk integrand rho_b(ln rho_b - 1) - rho_b betamu [+ rho_b betamu_att / 2],
 // and the hard-sphere energy density of the bulk weighted densities.
 // 3-D real-to-complex FFTs for the stencil sums (fft.cu): real box [F2][F1][F0] with F_d = n_d on periodic
-// dimensions (no padding) and F_d >= the padded extent elsewhere, half spectrum [F2][F1][F0/2 + 1]; each axis's
+// dimensions (no padding) and F_d >= the padded extent elsewhere
+// (n_d + h_d where one boundary value serves both ends), half spectrum [F2][F1][F0/2 + 1]; each axis's
 // length is a product of radices 2, 3, 4, 5
 struct FftAxis {
   int n = 1, R1 = 1, R2 = 1;   // length and its two radices
@@ -79,12 +80,21 @@ struct FftPlan {
   int P[3] = {1, 1, 1}, nx[3] = {1, 1, 1}, h[3] = {0, 0, 0};
   int off[3] = {0, 0, 0};    // first padded index the box holds along d (h on an unpadded periodic dimension)
   int ext[3] = {1, 1, 1};    // padded extent the box holds (zeros beyond it)
+  int shared[3] = {0, 0, 0}; // node i at position i, one boundary value from n to F (both ends read it)
   long NR = 0;               // real box points
   long NH = 0, NS = 0;       // half-spectrum points, points stored (pitch included)
   FftAxis ax[3];
 };
-bool fft_make_plan(FftPlan &p, const int P[3], const int nx[3], const int h[3], const int periodic[3], int ndim,
-                   cudaStream_t s);
+// share[d]: one boundary value beyond both ends of d (or, along x, the low end's corrected by a profile): F_d >= n_d + h_d
+bool fft_make_plan(FftPlan &p, const int P[3], const int nx[3], const int h[3], const int periodic[3],
+                   const int share[3], int ndim, cudaStream_t s);
+// What an output along x takes on top of its inverse transform: sum_k c[k] s[k][ix], k < n (the low boundary's value less
+// the high one's, times the stencil's weight beyond the low boundary)
+struct FftProfile {
+  const double *s[2];
+  double c[2];
+  int n;
+};
 // One channel of a field read through the per-dimension boundary maps (the values a padded box would hold:
 // bulk values at bulk sentinels, 0 inside walls, mirrored nodes with the sign flips of signmask, 0 at the
 // zero-density nodes of component zc >= 0)
@@ -101,17 +111,16 @@ struct MapSrc {
 void rfft_forward_mapped(const MapSrc &m, double2 *spec, const FftPlan &p, cudaStream_t s);
 void rfft_forward_mapped(const MapSrc &m, float2 *spec, const FftPlan &p, cudaStream_t s);
 void fft_free_plan(FftPlan &p);
-// half spectrum of a padded channel [P2][P1][P0]
-void rfft_forward(const double *pad, double2 *spec, const FftPlan &p, cudaStream_t s);
-void rfft_forward(const float *pad, float2 *spec, const FftPlan &p, cudaStream_t s);
 // half spectrum of a real box [F2][F1][F0]
 void rfft_forward_box(const double *box, double2 *spec, const FftPlan &p, cudaStream_t s);
 // out[node] (+)= scale * inverse transform of sum_t a_t k_t (nterms <= fft_max_terms() spectral products, formed by
 // the first inverse pass) at the interior nodes; work holds the half spectrum in between
 void rfft_inverse_products(const double2 *const *a, const double2 *const *k, int nterms, double2 *work,
-                           const FftPlan &p, double scale, double *out, bool accumulate, cudaStream_t s);
+                           const FftPlan &p, double scale, double *out, bool accumulate, cudaStream_t s,
+                           const FftProfile &prof = FftProfile{});
 void rfft_inverse_products(const float2 *const *a, const float2 *const *k, int nterms, float2 *work,
-                           const FftPlan &p, double scale, double *out, bool accumulate, cudaStream_t s);
+                           const FftPlan &p, double scale, double *out, bool accumulate, cudaStream_t s,
+                           const FftProfile &prof = FftProfile{});
 void rfft_inverse_products(const float2 *const *a, const float2 *const *k, int nterms, float2 *work,
                            const FftPlan &p, double scale, float *out, bool accumulate, cudaStream_t s);
 int fft_max_terms();
@@ -121,11 +130,13 @@ int fft_max_batch();
 void rfft_forward_mapped_batch(const MapSrc *m, int nb, float2 *const *spec, const FftPlan &p, cudaStream_t s);
 void rfft_forward_mapped_batch(const MapSrc *m, int nb, double2 *const *spec, const FftPlan &p, cudaStream_t s);
 void rfft_inverse_batch(const float2 *a, const float2 *const *k, int nb, float2 *const *work, const FftPlan &p,
-                        double scale, double *const *out, bool accumulate, cudaStream_t s);
+                        double scale, double *const *out, bool accumulate, cudaStream_t s,
+                        const FftProfile *prof = nullptr);
 void rfft_inverse_batch(const float2 *a, const float2 *const *k, int nb, float2 *const *work, const FftPlan &p,
                         double scale, float *const *out, bool accumulate, cudaStream_t s);
 void rfft_inverse_batch(const double2 *a, const double2 *const *k, int nb, double2 *const *work, const FftPlan &p,
-                        double scale, double *const *out, bool accumulate, cudaStream_t s);
+                        double scale, double *const *out, bool accumulate, cudaStream_t s,
+                        const FftProfile *prof = nullptr);
 // per-launch CUDA-event timing of the FP32 y/z FFT passes (off unless enabled; collect reads and resets)
 void pass_timer_enable(bool on);
 void pass_timer_collect(long *launches, double *ms_total, double *bytes_total, long *fields_total);
@@ -434,6 +445,7 @@ struct DevStencil {
   // FFT spectra of the correlation kernels (FP64 fills by FFT): per forward output, per transpose input;
   // FP32 copies of the forward ones for the FP32 sums (products, FP32 fills)
   std::vector<double2 *> spec_fwd, spec_tr;
+  double *d_prof_fwd = nullptr, *d_prof_tr = nullptr;   // [coefficients][nx]: weight beyond the low x end per node
   std::vector<double2 *> spec_adj;      // of the adjoint's transposed sums (offsets negated): delta 1 + ndim, others 1
   std::vector<float2 *> spec_fwd32, spec_tr32;
   int fft32_fwd = 0, fft32_tr = 0;      // short stencils: FP32 FFT (1) or slab (-1) sums, 0 undecided
