@@ -883,10 +883,35 @@ void forward_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, boo
         os.push_back(o);
       };
       add(sten[TGPU_STEN_THETA][jc], 0, out);
-      for (size_t q = 0; q < o_de.size(); q++) add(sten[TGPU_STEN_DELTA][jc], (int)q, o_de[q]);
+      // of the delta shell's sums n1, n0 and V1 are multiples of n2 and V2: with several particle sizes the transforms
+      // of n2 and V2 write them too (binary pore 96 x 96 x 64: 10 inverse transforms per density become 5)
+      std::vector<tgpu::FftCopies> copies;
+      const int nsum = 1 + nd;   // n2, V2
+      for (int q = 0; q < nsum; q++) {
+        const int t = q == 0 ? 0 : (g.single_size ? q : 2 + q);
+        add(sten[TGPU_STEN_DELTA][jc], t, o_de[t]);
+      }
+      copies.assign(os.size(), tgpu::FftCopies{});
+      if (!g.single_size)
+        for (int q = 0; q < nsum; q++) {
+          tgpu::FftCopies &cp = copies[1 + q];
+          auto copy = [&](int row, double f) {
+            double *o = out + (long)row * N;
+            cp.out[cp.n] = o;
+            cp.out32[cp.n] = c->store32 ? c->d_conv32 + (o - c->d_conv) : nullptr;
+            cp.f[cp.n++] = f;
+          };
+          if (q == 0) {
+            copy(2, g.inv_4pir[jc]);
+            copy(3, g.inv_4pirsq[jc]);
+          } else {
+            copy(4 + nd + q - 1, g.inv_4pir[jc]);
+          }
+        }
       if (g.attraction)
         for (int ic = 0; ic < g.ncomp; ic++)
           add(sten[TGPU_STEN_UATT][ic + g.ncomp * jc], 0, out + (long)(g.nrb + ic) * N);
+      copies.resize(os.size(), tgpu::FftCopies{});
       const int n = (int)os.size();
       const double scale = 1.0 / (double)c->fft.NR;
       if (f32) {
@@ -896,15 +921,17 @@ void forward_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, boo
         if (c->store32) {   // the FP32 shadows of the sums
           std::vector<float *> os32;
           for (double *o : os) os32.push_back(c->d_conv32 + (o - c->d_conv));
-          tgpu::rfft_inverse_batch(F, ks32.data(), n, work.data(), c->fft, scale, os32.data(), acc, c->stream);
+          tgpu::rfft_inverse_batch(F, ks32.data(), n, work.data(), c->fft, scale, os32.data(), acc, c->stream, copies.data());
         } else {
-          tgpu::rfft_inverse_batch(F, ks32.data(), n, work.data(), c->fft, scale, os.data(), acc, c->stream, prof.data());
+          tgpu::rfft_inverse_batch(F, ks32.data(), n, work.data(), c->fft, scale, os.data(), acc, c->stream, prof.data(),
+                                   copies.data());
         }
       } else {
         const double2 *F = fft_channel(c, jc);
         std::vector<double2 *> &work = tr_boxes<double2>(c);
         while ((int)work.size() < n) work.push_back(dalloc<double2>((size_t)c->fft.NS));
-        tgpu::rfft_inverse_batch(F, ks.data(), n, work.data(), c->fft, scale, os.data(), acc, c->stream, prof.data());
+        tgpu::rfft_inverse_batch(F, ks.data(), n, work.data(), c->fft, scale, os.data(), acc, c->stream, prof.data(),
+                                   copies.data());
       }
       c->stats.kernel_launches += 3 * ((n + tgpu::fft_max_batch() - 1) / tgpu::fft_max_batch());
       c->stats.conv_launches++;

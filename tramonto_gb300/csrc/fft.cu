@@ -244,6 +244,7 @@ struct OutBatch {
   double *out[kMaxBatch];
   float *out32[kMaxBatch];   // FP32 outputs (the FP32 transforms; used instead of out when set)
   FftProfile prof[kMaxBatch];
+  FftCopies copies[kMaxBatch];
 };
 
 // ---- y and z passes ---------------------------------------------------------------------------------------------
@@ -445,9 +446,10 @@ __global__ void __launch_bounds__((x_pairs_max<C>() * HI + 31) / 32 * 32) k_rfft
   }
 }
 
-// one output line: out = scale * value (+ out when accumulate), every load before the stores
-template <class T, class O, class C>
-__device__ __forceinline__ void write_line(const C *z, bool imag, O *o, int nx0, T sc, bool accumulate,
+// one output line: out = scale * value (+ out when accumulate), every load before the stores; times is a further factor of
+// an output that is a multiple of the transform's (TIMES)
+template <bool TIMES, class T, class O, class C>
+__device__ __forceinline__ void write_line(const C *z, bool imag, O *o, double times, int nx0, T sc, bool accumulate,
                                            const FftProfile &prof, int lane)
 {
   for (int x0 = lane; x0 < nx0; x0 += 32 * kXBatch) {
@@ -461,6 +463,7 @@ __device__ __forceinline__ void write_line(const C *z, bool imag, O *o, int nx0,
         O v = (O)(sc * (imag ? r.y : r.x));   // scaled in the transform's arithmetic
         if (prof.n > 0) v += (O)(prof.c[0] * prof.s[0][x0 + 32 * u]);
         if (prof.n > 1) v += (O)(prof.c[1] * prof.s[1][x0 + 32 * u]);
+        if (TIMES) v *= (O)times;
         o[x0 + 32 * u] = accumulate ? old[u] + v : v;
       }
   }
@@ -494,6 +497,7 @@ __global__ void __launch_bounds__((x_pairs_max<C>() * HI + 31) / 32 * 32) k_irff
   const int nx0 = g.nx[0];
   const T sc = (T)scale;
   const FftProfile prof = ob.prof[blockIdx.y];
+  const int copies = ob.copies[blockIdx.y].n;
   for (int p = warp; p < np; p += nw) {
     const int L = 2 * (pair0 + p);
 #pragma unroll
@@ -503,10 +507,18 @@ __global__ void __launch_bounds__((x_pairs_max<C>() * HI + 31) / 32 * 32) k_irff
       if (y < 0 || y >= g.nx[1] || z < 0 || z >= g.nx[2]) continue;
       const long row = ((long)z * g.nx[1] + y) * nx0;
       const C *zl = sm + p * lp + g.e[0];
-      if (std::is_same<C, float2>::value && ob.out32[blockIdx.y])
-        write_line<T, float>(zl, h != 0, ob.out32[blockIdx.y] + row, nx0, sc, accumulate != 0, prof, lane);
-      else
-        write_line<T, double>(zl, h != 0, ob.out[blockIdx.y] + row, nx0, sc, accumulate != 0, prof, lane);
+      const bool acc = accumulate != 0;
+      if (std::is_same<C, float2>::value && ob.out32[blockIdx.y]) {
+        write_line<false, T, float>(zl, h != 0, ob.out32[blockIdx.y] + row, 1.0, nx0, sc, acc, prof, lane);
+        for (int q = 0; q < copies; q++)
+          write_line<true, T, float>(zl, h != 0, ob.copies[blockIdx.y].out32[q] + row, ob.copies[blockIdx.y].f[q], nx0, sc,
+                                     acc, prof, lane);
+      } else {
+        write_line<false, T, double>(zl, h != 0, ob.out[blockIdx.y] + row, 1.0, nx0, sc, acc, prof, lane);
+        for (int q = 0; q < copies; q++)
+          write_line<true, T, double>(zl, h != 0, ob.copies[blockIdx.y].out[q] + row, ob.copies[blockIdx.y].f[q], nx0, sc,
+                                      acc, prof, lane);
+      }
     }
   }
 }
@@ -819,7 +831,7 @@ void rfft_forward_mapped_batch_impl(const MapSrc *m, int nb, C *const *spec, con
 template <class C>
 void rfft_inverse_batch_impl(const C *a, const C *const *k, int nb, C *const *work, const FftPlan &p, double scale,
                              double *const *out, float *const *out32, bool accumulate, const FftProfile *prof,
-                             cudaStream_t s)
+                             const FftCopies *copies, cudaStream_t s)
 {
   PassBatch<C> pb{}, plain{};
   OutBatch<C> ob{};
@@ -833,6 +845,7 @@ void rfft_inverse_batch_impl(const C *a, const C *const *k, int nb, C *const *wo
     ob.out[b] = out ? out[b] : nullptr;
     ob.out32[b] = out32 ? out32[b] : nullptr;
     if (prof) ob.prof[b] = prof[b];
+    if (copies) ob.copies[b] = copies[b];
   }
   bool pending = true;
   for (int d = 2; d >= 1; d--) {
@@ -981,27 +994,29 @@ void rfft_forward_mapped_batch(const MapSrc *m, int nb, double2 *const *spec, co
 }
 
 void rfft_inverse_batch(const float2 *a, const float2 *const *k, int nb, float2 *const *work, const FftPlan &p,
-                        double scale, double *const *out, bool accumulate, cudaStream_t s, const FftProfile *prof)
+                        double scale, double *const *out, bool accumulate, cudaStream_t s, const FftProfile *prof,
+                        const FftCopies *copies)
 {
   for (int b0 = 0; b0 < nb; b0 += kMaxBatch)
     rfft_inverse_batch_impl<float2>(a, k + b0, std::min(kMaxBatch, nb - b0), work + b0, p, scale, out + b0, nullptr,
-                                    accumulate, prof ? prof + b0 : nullptr, s);
+                                    accumulate, prof ? prof + b0 : nullptr, copies ? copies + b0 : nullptr, s);
 }
 
 void rfft_inverse_batch(const float2 *a, const float2 *const *k, int nb, float2 *const *work, const FftPlan &p,
-                        double scale, float *const *out, bool accumulate, cudaStream_t s)
+                        double scale, float *const *out, bool accumulate, cudaStream_t s, const FftCopies *copies)
 {
   for (int b0 = 0; b0 < nb; b0 += kMaxBatch)
     rfft_inverse_batch_impl<float2>(a, k + b0, std::min(kMaxBatch, nb - b0), work + b0, p, scale, nullptr, out + b0,
-                                    accumulate, nullptr, s);
+                                    accumulate, nullptr, copies ? copies + b0 : nullptr, s);
 }
 
 void rfft_inverse_batch(const double2 *a, const double2 *const *k, int nb, double2 *const *work, const FftPlan &p,
-                        double scale, double *const *out, bool accumulate, cudaStream_t s, const FftProfile *prof)
+                        double scale, double *const *out, bool accumulate, cudaStream_t s, const FftProfile *prof,
+                        const FftCopies *copies)
 {
   for (int b0 = 0; b0 < nb; b0 += kMaxBatch)
     rfft_inverse_batch_impl<double2>(a, k + b0, std::min(kMaxBatch, nb - b0), work + b0, p, scale, out + b0, nullptr,
-                                     accumulate, prof ? prof + b0 : nullptr, s);
+                                     accumulate, prof ? prof + b0 : nullptr, copies ? copies + b0 : nullptr, s);
 }
 
 void fft_pass(double2 *spec, const FftPlan &p, int d, bool inverse, cudaStream_t s)

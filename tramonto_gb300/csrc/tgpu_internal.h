@@ -88,6 +88,13 @@ struct FftPlan {
 // share[d]: one boundary value beyond both ends of d (or, along x, the low end's corrected by a profile): F_d >= n_d + h_d
 bool fft_make_plan(FftPlan &p, const int P[3], const int nx[3], const int h[3], const int periodic[3],
                    const int share[3], int ndim, cudaStream_t s);
+// Further outputs that are multiples of a transform's: out[k] (or out32[k]) (+)= f[k] times it, k < n
+struct FftCopies {
+  double *out[2];
+  float *out32[2];
+  double f[2];
+  int n;
+};
 // What an output along x takes on top of its inverse transform: sum_k c[k] s[k][ix], k < n (the low boundary's value less
 // the high one's, times the stencil's weight beyond the low boundary)
 struct FftProfile {
@@ -131,12 +138,13 @@ void rfft_forward_mapped_batch(const MapSrc *m, int nb, float2 *const *spec, con
 void rfft_forward_mapped_batch(const MapSrc *m, int nb, double2 *const *spec, const FftPlan &p, cudaStream_t s);
 void rfft_inverse_batch(const float2 *a, const float2 *const *k, int nb, float2 *const *work, const FftPlan &p,
                         double scale, double *const *out, bool accumulate, cudaStream_t s,
-                        const FftProfile *prof = nullptr);
+                        const FftProfile *prof = nullptr, const FftCopies *copies = nullptr);
 void rfft_inverse_batch(const float2 *a, const float2 *const *k, int nb, float2 *const *work, const FftPlan &p,
-                        double scale, float *const *out, bool accumulate, cudaStream_t s);
+                        double scale, float *const *out, bool accumulate, cudaStream_t s,
+                        const FftCopies *copies = nullptr);
 void rfft_inverse_batch(const double2 *a, const double2 *const *k, int nb, double2 *const *work, const FftPlan &p,
                         double scale, double *const *out, bool accumulate, cudaStream_t s,
-                        const FftProfile *prof = nullptr);
+                        const FftProfile *prof = nullptr, const FftCopies *copies = nullptr);
 // per-launch CUDA-event timing of the FP32 y/z FFT passes (off unless enabled; collect reads and resets)
 void pass_timer_enable(bool on);
 void pass_timer_collect(long *launches, double *ms_total, double *bytes_total, long *fields_total);
