@@ -1037,6 +1037,31 @@ void decide_fft32_2d(Ctx *c, bool tr)
   for (int *f : flags) *f = t[1] < t[0] + bias ? 1 : -1;
 }
 
+// a 1-D pass's sums in one launch, all rows of the output written (one quadrature zone)
+bool line_sums(Ctx *c, const double *src, const PadParams &pp, bool f32, bool transposed)
+{
+  const tgpu::DevGeom &g = c->dg;
+  if (c->nzone != 1 || !tgpu::line_sums_ok(g.ndim, g.N, g.h[0])) return false;
+  tgpu::LineSumsCall q{};
+  q.sten = c->sten;
+  q.ncomp = g.ncomp;
+  q.attraction = g.attraction;
+  q.h = g.h[0];
+  q.nch = pp.nch;
+  q.transposed = transposed;
+  q.f32 = f32;
+  q.N = g.N;
+  q.src = src;
+  q.bulk = pp.bulk;
+  q.sign = pp.sign;
+  q.zero = c->d_zero;
+  q.out = transposed ? c->d_tr : c->d_conv;
+  tgpu::launch_line_sums(q, c->stream);
+  c->stats.kernel_launches++;
+  c->stats.conv_launches++;
+  return true;
+}
+
 // Weighted-density (and mean-field) sums of a density-shaped field
 // (`field` points at the first density row, rows N apart) into d_conv.
 void forward_pass(Ctx *c, const double *field, const PadParams &pp, bool f32, bool zero_first = true)
@@ -1044,28 +1069,31 @@ void forward_pass(Ctx *c, const double *field, const PadParams &pp, bool f32, bo
   const tgpu::DevGeom &g = c->dg;
   const long N = g.N;
   const size_t nrows = (size_t)(g.nrb + g.ncomp);
-  pad(c, field, pp, f32);
-  if (f32 && g.ndim == 2) decide_fft32_2d(c, false);
-  if (f32 && g.attraction && g.ndim == 3) decide_fft32(c);
-  if (f32 && g.ndim == 3)
-    for (int jc = 0; jc < g.ncomp; jc++) {
-      decide_fft32_sten(c, c->sten[TGPU_STEN_THETA][jc], false, jc, 1, 1);
-      decide_fft32_sten(c, c->sten[TGPU_STEN_DELTA][jc], false, jc, 1, c->sten[TGPU_STEN_DELTA][jc].nout_fwd);
+  const bool line = zero_first && line_sums(c, field, pp, f32, false);
+  if (!line) {
+    pad(c, field, pp, f32);
+    if (f32 && g.ndim == 2) decide_fft32_2d(c, false);
+    if (f32 && g.attraction && g.ndim == 3) decide_fft32(c);
+    if (f32 && g.ndim == 3)
+      for (int jc = 0; jc < g.ncomp; jc++) {
+        decide_fft32_sten(c, c->sten[TGPU_STEN_THETA][jc], false, jc, 1, 1);
+        decide_fft32_sten(c, c->sten[TGPU_STEN_DELTA][jc], false, jc, 1, c->sten[TGPU_STEN_DELTA][jc].nout_fwd);
+      }
+    // sums that all take the FFT need no zeroed rows (the copies' rows n1, n0, V1 of one particle size are not read)
+    bool fresh = zero_first && c->nzone == 1 && !c->coarse() && c->hw_targets.empty();
+    for (int jc = 0; jc < g.ncomp; jc++) fresh = fresh && fwd_all_fft(c, jc, f32);
+    if (zero_first && !fresh) {
+      if (c->store32) ck(cudaMemsetAsync(c->d_conv32, 0, sizeof(float) * nrows * N, c->stream), "memset");
+      else ck(cudaMemsetAsync(c->d_conv, 0, sizeof(double) * nrows * N, c->stream), "memset");
     }
-  // sums that all take the FFT need no zeroed rows (the copies' rows n1, n0, V1 of one particle size are not read)
-  bool fresh = zero_first && c->nzone == 1 && !c->coarse() && c->hw_targets.empty();
-  for (int jc = 0; jc < g.ncomp; jc++) fresh = fresh && fwd_all_fft(c, jc, f32);
-  if (zero_first && !fresh) {
-    if (c->store32) ck(cudaMemsetAsync(c->d_conv32, 0, sizeof(float) * nrows * N, c->stream), "memset");
-    else ck(cudaMemsetAsync(c->d_conv, 0, sizeof(double) * nrows * N, c->stream), "memset");
-  }
-  forward_convs(c, c->sten, c->d_conv, f32, fresh);
-  // nodes of the coarser quadrature zones keep their own zone's sums (zero_first holds with zones)
-  for (int z = 1; z < c->nzone; z++) {
-    ck(cudaMemsetAsync(c->d_zbuf, 0, sizeof(double) * nrows * N, c->stream), "memset");
-    forward_convs(c, c->zsten[z], c->d_zbuf, f32);
-    tgpu::launch_zone_merge(c->d_zbuf, c->d_conv, (int)nrows, N, c->d_zone, z, c->stream);
-    c->stats.kernel_launches++;
+    forward_convs(c, c->sten, c->d_conv, f32, fresh);
+    // nodes of the coarser quadrature zones keep their own zone's sums (zero_first holds with zones)
+    for (int z = 1; z < c->nzone; z++) {
+      ck(cudaMemsetAsync(c->d_zbuf, 0, sizeof(double) * nrows * N, c->stream), "memset");
+      forward_convs(c, c->zsten[z], c->d_zbuf, f32);
+      tgpu::launch_zone_merge(c->d_zbuf, c->d_conv, (int)nrows, N, c->d_zone, z, c->stream);
+      c->stats.kernel_launches++;
+    }
   }
   if (g.hard_surf && !c->hw_targets.empty()) {
     tgpu::launch_hw_correct(field, N, 0, c->sten[TGPU_STEN_THETA].data(), c->sten[TGPU_STEN_DELTA].data(),
@@ -1081,6 +1109,7 @@ void transpose_pass(Ctx *c, const PadParams &pp, bool f32, const double *chan = 
 {
   const tgpu::DevGeom &g = c->dg;
   const long N = g.N;
+  if (zero_first && line_sums(c, chan ? chan : c->d_chan, pp, f32, true)) return;
   if (c->store32) pad32(c, c->d_chan32, pp);
   else pad(c, chan ? chan : c->d_chan, pp, f32);
   if (f32 && g.ndim == 2) decide_fft32_2d(c, true);

@@ -2634,5 +2634,6 @@ void launch_vext_sens(const double *lam, const double *gv, const double *vext, c
 }
 
 #include "gmres_line.h"
+#include "line_sums.h"
 
 }  // namespace tgpu

@@ -648,6 +648,19 @@ struct LineCall {
   unsigned *bar;        // two words, zero before the launch; the second is set when a barrier gave up
   LineResult *res;
 };
+// the point sums of a pass of a 1-D problem in one launch (line_sums.h)
+struct LineSumsCall {
+  const std::vector<DevStencil> *sten;   // [3]
+  int ncomp, attraction, h, nch;
+  bool transposed, f32;
+  long N;
+  const double *src, *bulk;
+  const int *sign;
+  const signed char *zero;
+  double *out;
+};
+bool line_sums_ok(int ndim, long N, int h);
+void launch_line_sums(const LineSumsCall &q, cudaStream_t s);
 int gmres_line_per(long N, int nsm);   // nodes per CTA, 0: the mesh is too large
 size_t gmres_line_smem(int nc, bool tr, bool f32, int kdim, int per, int h);
 cudaError_t launch_gmres_line(const LineCall &q, cudaStream_t s);
