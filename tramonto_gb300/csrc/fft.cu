@@ -334,13 +334,14 @@ __global__ void __launch_bounds__(lines_per_cta<C>() * HI) k_fft_lines(PassBatch
 }
 
 // ---- x passes ---------------------------------------------------------------------------------------------------
-// A CTA takes x_pairs complex lines (pairs of real ones).  A line's values lie along x, so they are staged through
+// A CTA takes up to kXPairs complex lines (pairs of real ones).  A line's values lie along x, so they are staged through
 // shared memory: one warp reads or writes a line with consecutive lanes, and the two register steps work on the tile.
 // (Register steps that read and wrote global memory themselves, in runs of R1 or R2 elements, took 87 instead of 36 us
 // per FP32 inverse launch.)  Bound as the y and z passes; 128^3 workload, per launch of 1 and 5 or 6 lines' transforms:
 // forward 42 us in FP32 (47 with radix-4 stages), inverse 35 (33); FP64 271 (318) and 274 (338).
-template <class C>
-constexpr int x_pairs_max() { return std::is_same<C, float2>::value ? 16 : 8; }
+// Eight pairs per CTA: more and smaller CTAs than sixteen overlap one's loads with another's steps in FP32 (forward 37.3
+// -> 35.0 us, inverse 29.1 -> 27.7 on the 160 x 128 x 128 box; four: the same).
+constexpr int kXPairs = 8;
 constexpr int kXBatch = 4;   // positions a lane loads before it stores them
 
 // shared pitch of the R2 values of one k1: odd, so that the R1 threads of a line read distinct banks
@@ -389,7 +390,7 @@ __device__ __forceinline__ void tile_fft(C *sm, int NP, int lp, const Line1d<C> 
 
 // forward: two real lines per complex line, split into two half-spectrum lines by Hermitian symmetry
 template <class T, class C, class Src, int LO, int HI>
-__global__ void __launch_bounds__((x_pairs_max<C>() * HI + 31) / 32 * 32) k_rfft_lines(SrcBatch<Src, C> sb, XGeom g,
+__global__ void __launch_bounds__((kXPairs * HI + 31) / 32 * 32) k_rfft_lines(SrcBatch<Src, C> sb, XGeom g,
                                                                                Line1d<C> ln, int NP, int lp)
 {
   const Src src = sb.src[blockIdx.y];
@@ -472,7 +473,7 @@ __device__ __forceinline__ void write_line(const C *z, bool imag, O *o, double t
 // inverse: two half-spectrum lines as one complex line Z = A + iB, whose inverse's real and imaginary parts are the
 // outputs of the interior nodes (out[node] = scale * value, or += when accumulate)
 template <class C, int LO, int HI>
-__global__ void __launch_bounds__((x_pairs_max<C>() * HI + 31) / 32 * 32) k_irfft_lines(OutBatch<C> ob, XGeom g,
+__global__ void __launch_bounds__((kXPairs * HI + 31) / 32 * 32) k_irfft_lines(OutBatch<C> ob, XGeom g,
                                                                                 Line1d<C> ln, int NP, int lp,
                                                                                 double scale, int accumulate)
 {
@@ -629,10 +630,9 @@ int line_threads(const FftAxis &a)
 }
 template <class C>
 size_t lines_smem(const FftAxis &a) { return sizeof(C) * (size_t)lines_per_cta<C>() * a.n; }
-template <class C>
 int x_pairs(long npairs, int nb)   // fewer pairs per CTA where whole tiles would leave SMs idle (2-D boxes)
 {
-  int np = x_pairs_max<C>();
+  int np = kXPairs;
   while (np > 2 && (npairs + np - 1) / np * nb < 2 * 152) np /= 2;
   return np;
 }
@@ -645,7 +645,7 @@ template <class T, class C>
 void set_smem_limits(const FftPlan &p)
 {
   const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  const int most_x = (int)(sizeof(C) * x_pairs_max<C>() * (kMaxRadix * (kMaxRadix | 1) + 1)), most = 128 * kFftMaxN;
+  const int most_x = (int)(sizeof(C) * kXPairs * (kMaxRadix * (kMaxRadix | 1) + 1)), most = 128 * kFftMaxN;
   with_range(p.ax[0].R1, [&](auto lo, auto hi) {
     constexpr int LO = decltype(lo)::value, HI = decltype(hi)::value;
     cudaFuncSetAttribute(k_rfft_lines<T, C, BoxSrc<T>, LO, HI>, attr, most_x);
@@ -733,7 +733,7 @@ void forward_x(const SrcBatch<Src, C> &sb, int nb, const XGeom &g, const FftPlan
 {
   const FftAxis &ax = p.ax[0];
   const long npairs = (g.nlines + 1) / 2;
-  const int np = x_pairs<C>(npairs, nb);
+  const int np = x_pairs(npairs, nb);
   const dim3 grid((unsigned)((npairs + np - 1) / np), (unsigned)nb);
   with_range(ax.R1, [&](auto lo, auto hi) {
     constexpr int LO = decltype(lo)::value, HI = decltype(hi)::value;
@@ -747,7 +747,7 @@ void inverse_x(const OutBatch<C> &ob, int nb, const FftPlan &p, double scale, bo
   const XGeom g = xgeom(p);
   const FftAxis &ax = p.ax[0];
   const long npairs = (g.nlines + 1) / 2;
-  const int np = x_pairs<C>(npairs, nb);
+  const int np = x_pairs(npairs, nb);
   const dim3 grid((unsigned)((npairs + np - 1) / np), (unsigned)nb);
   with_range(ax.R1, [&](auto lo, auto hi) {
     constexpr int LO = decltype(lo)::value, HI = decltype(hi)::value;
