@@ -1174,7 +1174,7 @@ void fill_arith(Ctx *c, const double *d_x, double *d_R, int mode, int arith)
   ck(cudaMemsetAsync(c->d_domain, 0, sizeof(unsigned), c->stream), "memset");
   if (arith == TGPU_FILL_REFINED) {
     ensure_refs(c);
-    tgpu::launch_fmt_local(g.ndim, g.functional, x, c->d_chan, c->stream, c->d_domain);
+    tgpu::launch_fmt_local(c->dg.N, g.ndim, g.functional, x, c->d_chan, c->stream, c->d_domain);
     bool refresh = !c->have_ref;
     if (!refresh) {
       const int nb = tgpu::reduce_blocks((long)nchan);
@@ -1213,12 +1213,12 @@ void fill_arith(Ctx *c, const double *d_x, double *d_R, int mode, int arith)
     c->fft_on = arith == TGPU_FILL_FFT;
     if (c->fft_on) ensure_fft(c);
     forward_pass(c, rho, c->pads.rho_res, f32);
-    tgpu::launch_fmt_local(g.ndim, g.functional, x, c->d_chan, c->stream, c->d_domain);
+    tgpu::launch_fmt_local(c->dg.N, g.ndim, g.functional, x, c->d_chan, c->stream, c->d_domain);
     transpose_pass(c, c->pads.tr_res, f32);
     c->ff_on = false;
     c->fft_on = false;
   }
-  tgpu::launch_assemble(g.ndim, x, c->d_vext, c->d_zero, c->d_conv, c->d_tr, d_R, c->stream, c->d_domain);
+  tgpu::launch_assemble(c->dg.N, g.ndim, x, c->d_vext, c->d_zero, c->d_conv, c->d_tr, d_R, c->stream, c->d_domain);
   c->stats.kernel_launches += 2;
   if (c->coarse()) {   // the averaged rows of coarsened nodes
     tgpu::launch_coarse_rows(x, d_R, g.nunk, g.first_rho, g.ncomp, N, c->cr, c->d_cbulk, c->stream);
@@ -1290,7 +1290,7 @@ const double *hess_coef(Ctx *c)
   const int form = c->dg.jac_exact;
   if (c->hcoef_form == form) return c->d_hcoef;
   if (!c->d_hcoef) c->d_hcoef = dalloc<double>((size_t)tgpu::kHessCoef * c->dg.N);
-  tgpu::launch_hess_coef(c->dg.ndim, c->dg.functional, c->d_x, c->d_hcoef, c->stream, c->d_hcoef32);   // with the FP32 table once it exists
+  tgpu::launch_hess_coef(c->dg.N, c->dg.ndim, c->dg.functional, c->d_x, c->d_hcoef, c->stream, c->d_hcoef32);   // with the FP32 table once it exists
   c->stats.kernel_launches++;
   c->hcoef_form = form;
   if (c->d_hcoef32) {
@@ -1346,7 +1346,7 @@ void ensure_store32(Ctx *c)
     c->d_kind32 = dalloc<signed char>((size_t)g.ncomp * N);
   }
   if (c->hcoef32_form != g.jac_exact) {
-    tgpu::launch_hess_coef32(g.ndim, g.functional, c->d_x, c->d_hcoef32, c->stream);
+    tgpu::launch_hess_coef32(c->dg.N, g.ndim, g.functional, c->d_x, c->d_hcoef32, c->stream);
     tgpu::launch_row_info32(c->d_x, c->d_vext, c->d_zero, c->d_inv32, c->d_kind32, c->stream);
     c->stats.kernel_launches += 2;
     c->hcoef32_form = g.jac_exact;
@@ -1389,7 +1389,7 @@ void schur_device(Ctx *c, const double *d_v2, double *d_y2, bool precond = false
   const double *v2 = prolonged(c, d_v2, g.ncomp);
   forward_pass(c, v2, c->pads.rho_jac, f32);
   if (c->coarse()) tgpu::launch_prolong(c->d_conv, 0, g.nrb + g.ncomp, g.nunk, g.N, c->cr, nullptr, c->stream);
-  tgpu::launch_schur_local(c->d_x, c->d_conv, c->d_chan, c->d_ymf, hess_coef(c), c->stream, f32);
+  tgpu::launch_schur_local(c->dg.N, c->d_x, c->d_conv, c->d_chan, c->d_ymf, hess_coef(c), c->stream, f32);
   transpose_pass(c, c->pads.tr_jac, f32);
   tgpu::launch_schur_combine(c->d_x, c->d_vext, c->d_zero, v2, c->d_tr, c->d_ymf, d_y2, c->stream);
   if (c->coarse()) tgpu::launch_zero_nodes(d_y2, g.ncomp, g.N, c->cr, c->stream);
@@ -1405,7 +1405,7 @@ void jv_device(Ctx *c, const double *d_v, double *d_out)
   const long N = c->dg.N;
   const bool f32 = prod_f32(c);
   forward_pass(c, d_v + (long)c->dg.first_rho * N, c->pads.rho_jac, f32);
-  tgpu::launch_jv_local(c->d_x, d_v, c->d_chan, hess_coef(c), c->stream, f32);
+  tgpu::launch_jv_local(c->dg.N, c->d_x, d_v, c->d_chan, hess_coef(c), c->stream, f32);
   transpose_pass(c, c->pads.tr_jac, f32);
   tgpu::launch_jv_combine(c->d_x, c->d_vext, c->d_zero, d_v, c->d_conv, c->d_tr, d_out, c->stream);
   c->stats.kernel_launches += 2;
@@ -1417,7 +1417,7 @@ void jv_device(Ctx *c, const double *d_v, double *d_out)
 
 // ---- kernels used only by the Schur rhs / back-substitution ------------------
 namespace tgpu {
-void launch_rhs_local(const double *x, const double *b, double *chan, double *ymf, const double *coef, cudaStream_t s);
+void launch_rhs_local(long N, const double *x, const double *b, double *chan, double *ymf, const double *coef, cudaStream_t s);
 void launch_rhs_combine(const double *vext, const signed char *zero, const double *b, const double *tr,
                         const double *ymf, double *b2s, cudaStream_t s);
 void launch_x1(int nunk, long N, const double *b, const double *conv, const double *x2, double *dx, cudaStream_t s);
@@ -1453,7 +1453,7 @@ void schur_rhs_device(Ctx *c, const double *d_b, double *d_b2s)
     c->stats.kernel_launches += 2;
     return;
   }
-  tgpu::launch_rhs_local(c->d_x, b, c->d_chan, c->d_ymf, hess_coef(c), c->stream);
+  tgpu::launch_rhs_local(c->dg.N, c->d_x, b, c->d_chan, c->d_ymf, hess_coef(c), c->stream);
   transpose_pass(c, c->pads.tr_jac, prod_f32(c));
   tgpu::launch_rhs_combine(c->d_vext, c->d_zero, b, c->d_tr, c->d_ymf, d_b2s, c->stream);
   if (c->coarse()) tgpu::launch_zero_nodes(d_b2s, g.ncomp, g.N, c->cr, c->stream);
@@ -2077,7 +2077,7 @@ void jtv_device(Ctx *c, const double *d_w_in, double *d_out)
         adj_conv(c, ic, 1, st, st.d_coef_fwd, o + nd + 1, 1);
       }
     }
-    tgpu::launch_jtv_local(c->d_x, c->d_vext, c->d_zero, d_w, c->d_adj_g, gst, 1, d_out, hess_coef(c), c->stream);
+    tgpu::launch_jtv_local(c->dg.N, c->d_x, c->d_vext, c->d_zero, d_w, c->d_adj_g, gst, 1, d_out, hess_coef(c), c->stream);
     c->stats.kernel_launches += 4;
   }
   if (c->coarse()) {
@@ -2114,7 +2114,7 @@ void schur_t_device(Ctx *c, const double *d_v2, double *d_y2)
   copy_d(c, full + (long)g.first_rho * N, d_v2, (size_t)g.ncomp * N);
   jtv_reduced(c, full, t);
   copy_d(c, d_y2, t + (long)g.first_rho * N, (size_t)g.ncomp * N);   // A22^T v2 - nothing else yet
-  tgpu::launch_a11inv_t(t, full, c->stream);                           // y1 in block-1 rows, density rows 0
+  tgpu::launch_a11inv_t(c->dg.N, t, full, c->stream);                           // y1 in block-1 rows, density rows 0
   jtv_reduced(c, full, t);                                             // t_rho = A12^T y1
   tgpu::launch_axpby(d_y2, -1.0, t + (long)g.first_rho * N, 1.0, (long)g.ncomp * N, c->stream);
   c->stats.schur_applies++;
@@ -2138,7 +2138,7 @@ int adjoint_solve_device(Ctx *c, const double *d_g_in, double *d_lam, double tol
     d_g = c->d_cscr2;
   }
   // rhs2 = g2 - A12^T A11^-T g1
-  tgpu::launch_a11inv_t(d_g, full, c->stream);
+  tgpu::launch_a11inv_t(c->dg.N, d_g, full, c->stream);
   jtv_reduced(c, full, t);
   copy_d(c, c->d_b2s, d_g + (long)g.first_rho * N, (size_t)g.ncomp * N);
   tgpu::launch_axpby(c->d_b2s, -1.0, t + (long)g.first_rho * N, 1.0, (long)g.ncomp * N, c->stream);
@@ -2156,7 +2156,7 @@ int adjoint_solve_device(Ctx *c, const double *d_g_in, double *d_lam, double tol
   copy_d(c, full + (long)g.first_rho * N, c->d_gx, (size_t)g.ncomp * N);
   jtv_reduced(c, full, t);                                  // block-1 rows: A21^T lambda2
   tgpu::launch_axpby(t, 1.0, d_g, -1.0, (long)n, c->stream);  // t = g - J^T[0; lambda2] (block-1 rows used)
-  tgpu::launch_a11inv_t(t, d_lam, c->stream);
+  tgpu::launch_a11inv_t(c->dg.N, t, d_lam, c->stream);
   copy_d(c, d_lam + (long)g.first_rho * N, c->d_gx, (size_t)g.ncomp * N);
   return st;
 }

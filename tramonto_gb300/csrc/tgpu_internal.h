@@ -538,14 +538,14 @@ void launch_conv_slab_ff(const float *in_hi, const float *in_lo, long in_total, 
 constexpr int kSlabTileX = 128, kSlabTileY = 16;
 // domain flags of a fill (launch_fmt_local / launch_assemble with a non-null flag word)
 constexpr unsigned kDomainN3 = 1u, kDomainRho = 2u;
-void launch_fmt_local(int ndim, int fn, const double *x, double *chan, cudaStream_t s, unsigned *domain = nullptr);
-void launch_assemble(int ndim, const double *x, const double *vext, const signed char *zero, const double *conv,
+void launch_fmt_local(long N, int ndim, int fn, const double *x, double *chan, cudaStream_t s, unsigned *domain = nullptr);
+void launch_assemble(long N, int ndim, const double *x, const double *vext, const signed char *zero, const double *conv,
                      const double *tr, double *R, cudaStream_t s, unsigned *domain = nullptr);
 // coef: the state's Hessian scalars ([kHessCoef][N], launch_hess_coef) or null to evaluate them in place
-void launch_hess_coef(int ndim, int fn, const double *x, double *coef, cudaStream_t s, float *coef32 = nullptr);
+void launch_hess_coef(long N, int ndim, int fn, const double *x, double *coef, cudaStream_t s, float *coef32 = nullptr);
 // FP32 storage variants of the FP32 Schur product: the state's Hessian scalars and weighted densities as FP32 rows
 // [kHessCoef + nrb][N]; the local step and the combination on FP32 sums, channels and transposed sums
-void launch_hess_coef32(int ndim, int fn, const double *x, float *coef, cudaStream_t s);
+void launch_hess_coef32(long N, int ndim, int fn, const double *x, float *coef, cudaStream_t s);
 void launch_schur_local32(int ndim, bool alpha, long N, const float *conv, const float *coef, float *chan, float *ymf,
                           cudaStream_t s);
 void launch_rhs_local32(int ndim, bool alpha, long N, const double *b, const float *coef, float *chan, float *ymf,
@@ -556,10 +556,10 @@ void launch_row_info32(const double *x, const double *vext, const signed char *z
                        cudaStream_t s);
 void launch_schur_combine32(const double *inv, const signed char *kind, const double *v2, const float *tr,
                             const float *ymf, double *y2, const double *x, cudaStream_t s);
-void launch_schur_local(const double *x, const double *conv, double *chan, double *ymf, const double *coef,
+void launch_schur_local(long N, const double *x, const double *conv, double *chan, double *ymf, const double *coef,
                         cudaStream_t s, bool f32 = false);
 // f32: the per-node Hessian in FP32 arithmetic (FP32 products)
-void launch_jv_local(const double *x, const double *v, double *chan, const double *coef, cudaStream_t s,
+void launch_jv_local(long N, const double *x, const double *v, double *chan, const double *coef, cudaStream_t s,
                      bool f32 = false);
 void launch_schur_combine(const double *x, const double *vext, const signed char *zero, const double *v2,
                           const double *tr, const double *ymf, double *y2, cudaStream_t s);
@@ -589,7 +589,7 @@ void launch_newton_update(double *x, const double *dx, int nunk, long N, double 
                           double *partial, double *result, cudaStream_t s);
 void launch_norm2(const double *x, long n, double *partial, int nblocks, double *result, cudaStream_t s);
 // J^T w local step: A22, A11^T (with B^T), the MF coupling and H g for the rb columns
-void launch_jtv_local(const double *x, const double *vext, const signed char *zero, const double *w,
+void launch_jtv_local(long N, const double *x, const double *vext, const signed char *zero, const double *w,
                       const double *gel, int gstride_ic, int v2_first, double *out, const double *coef,
                       cudaStream_t s);
 void launch_objectives(const double *x, const double *vext, const double *satt, const double *wf, const double *wb,
@@ -607,7 +607,7 @@ void tc_free_slab(TcSlab &sl);
 void launch_sten_tc(const float *pad_channel, const DevGeom &g, const TcSlab &sl, const TcTables &t, double *out,
                     bool accumulate, cudaStream_t s);
 void launch_adj_rb_channels(const double *w, double *chan, cudaStream_t s);
-void launch_a11inv_t(const double *u, double *y, cudaStream_t s);
+void launch_a11inv_t(long N, const double *u, double *y, cudaStream_t s);
 // coarsen.cu: dst[r][i] = src[r][i] where zone[i] == z; buf[r][i] = 0 where zone[i] != z
 void launch_zone_merge(const double *src, double *dst, int nrows, long N, const int *zone, int z, cudaStream_t s);
 void launch_zone_mask(double *buf, int nrows, long N, const int *zone, int z, cudaStream_t s);
