@@ -602,14 +602,14 @@ void fft_tr_sum(Ctx *c, const int *chs, const C *const *kern, int n, double *out
   C *work = std::is_same<C, float2>::value ? (C *)c->d_fbox32[2] : (C *)c->d_fbox[2];
   if constexpr (std::is_same<C, float2>::value) {
     if (c->store32) {   // the FP32 shadow of the transposed-sum output
-      tgpu::rfft_inverse_products(a.data(), kern, n, work, c->fft, 1.0 / (double)c->fft.NR,
+      tgpu::rfft_inverse_products(a.data(), kern, n, work, c->fft,
                                   c->d_tr32 + (out - c->d_tr), accumulate, c->stream);
       c->stats.kernel_launches += 3;
       c->stats.conv_launches++;
       return;
     }
   }
-  tgpu::rfft_inverse_products(a.data(), kern, n, work, c->fft, 1.0 / (double)c->fft.NR, out, accumulate, c->stream, prof);
+  tgpu::rfft_inverse_products(a.data(), kern, n, work, c->fft, out, accumulate, c->stream, prof);
   c->stats.kernel_launches += 3;
   c->stats.conv_launches++;
 }
@@ -627,7 +627,7 @@ void fft_conv_impl(Ctx *c, int ch0, int nin, const DevStencil &st, const std::ve
       while ((int)work.size() < nout) work.push_back(dalloc<C>((size_t)c->fft.NS));
       std::vector<tgpu::FftProfile> prof(nout, tgpu::FftProfile{});
       for (int q = 0; q < nout; q++) add_profile(c, prof[q], st, false, q, ch0);
-      tgpu::rfft_inverse_batch(F, spec.data(), nout, work.data(), c->fft, 1.0 / (double)c->fft.NR, outs, true,
+      tgpu::rfft_inverse_batch(F, spec.data(), nout, work.data(), c->fft, outs, true,
                                c->stream, prof.data());
       c->stats.kernel_launches += 3;
     }
@@ -913,7 +913,6 @@ void forward_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, boo
           add(sten[TGPU_STEN_UATT][ic + g.ncomp * jc], 0, out + (long)(g.nrb + ic) * N);
       copies.resize(os.size(), tgpu::FftCopies{});
       const int n = (int)os.size();
-      const double scale = 1.0 / (double)c->fft.NR;
       if (f32) {
         const float2 *F = fft_channel32(c, jc);
         std::vector<float2 *> &work = tr_boxes<float2>(c);
@@ -921,16 +920,16 @@ void forward_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, boo
         if (c->store32) {   // the FP32 shadows of the sums
           std::vector<float *> os32;
           for (double *o : os) os32.push_back(c->d_conv32 + (o - c->d_conv));
-          tgpu::rfft_inverse_batch(F, ks32.data(), n, work.data(), c->fft, scale, os32.data(), acc, c->stream, copies.data());
+          tgpu::rfft_inverse_batch(F, ks32.data(), n, work.data(), c->fft, os32.data(), acc, c->stream, copies.data());
         } else {
-          tgpu::rfft_inverse_batch(F, ks32.data(), n, work.data(), c->fft, scale, os.data(), acc, c->stream, prof.data(),
+          tgpu::rfft_inverse_batch(F, ks32.data(), n, work.data(), c->fft, os.data(), acc, c->stream, prof.data(),
                                    copies.data());
         }
       } else {
         const double2 *F = fft_channel(c, jc);
         std::vector<double2 *> &work = tr_boxes<double2>(c);
         while ((int)work.size() < n) work.push_back(dalloc<double2>((size_t)c->fft.NS));
-        tgpu::rfft_inverse_batch(F, ks.data(), n, work.data(), c->fft, scale, os.data(), acc, c->stream, prof.data(),
+        tgpu::rfft_inverse_batch(F, ks.data(), n, work.data(), c->fft, os.data(), acc, c->stream, prof.data(),
                                    copies.data());
       }
       c->stats.kernel_launches += 3 * ((n + tgpu::fft_max_batch() - 1) / tgpu::fft_max_batch());
@@ -1958,7 +1957,7 @@ void adj_fft_in(Ctx *c, const std::vector<int> &chs, const std::vector<const dou
   for (int t = 0; t < n; t++) ms[t] = adj_src(c, chs[t]);
   tgpu::rfft_forward_mapped_batch(ms.data(), n, b.data(), c->fft, c->stream);
   std::vector<const double2 *> a(b.begin(), b.begin() + n);
-  tgpu::rfft_inverse_products(a.data(), k.data(), n, b[n], c->fft, 1.0 / (double)c->fft.NR, out, true, c->stream);
+  tgpu::rfft_inverse_products(a.data(), k.data(), n, b[n], c->fft, out, true, c->stream);
   c->stats.kernel_launches += 6;
   c->stats.conv_launches++;
 }
@@ -1969,7 +1968,7 @@ void adj_fft_out(Ctx *c, int ch, const std::vector<const double2 *> &k, double *
   const int n = (int)k.size();
   std::vector<double2 *> &b = adj_boxes(c, n + 1);
   tgpu::rfft_forward_mapped(adj_src(c, ch), b[n], c->fft, c->stream);
-  tgpu::rfft_inverse_batch(b[n], k.data(), n, b.data(), c->fft, 1.0 / (double)c->fft.NR, outs, false, c->stream);
+  tgpu::rfft_inverse_batch(b[n], k.data(), n, b.data(), c->fft, outs, false, c->stream);
   c->stats.kernel_launches += 6;
   c->stats.conv_launches++;
 }

@@ -28,8 +28,8 @@
 // k1, transform them and hold the outputs k1 + R1 k2.  Both steps address global memory themselves, so a y or z pass
 // moves its data through shared memory once.  The y and z passes take 16 lines adjacent in x per CTA (16 lanes read
 // 128 or 256 contiguous bytes; with the line as the fastest index of the exchange no access conflicts).
-// Twiddles are tabulated on the host in extended precision.  The inverse uses conjugate twiddles; its 1/(F0 F1 F2) is
-// applied on output.  The spectral products (one kernel spectrum per output, or the sum of channel-times-kernel
+// Twiddles are tabulated on the host in extended precision.  The inverse uses conjugate twiddles; its 1/(F0 F1 F2) and
+// the 1/2 of the split into two real lines are factors of the kernels' coefficients (1 % of an FP64 fill).  The spectral products (one kernel spectrum per output, or the sum of channel-times-kernel
 // products of a transposed sum) are formed while the first inverse pass loads its lines.
 #include <algorithm>
 #include <cmath>
@@ -441,16 +441,16 @@ __global__ void __launch_bounds__((kXPairs * HI + 31) / 32 * 32) k_rfft_lines(Sr
     C *o = spec + L * g.Fp;
     for (int k = lane; k < g.Fh; k += 32) {
       const C Z = sm[p * lp + k], Zm = sm[p * lp + (k == 0 ? 0 : n - k)];
-      o[k] = C{(T)0.5 * (Z.x + Zm.x), (T)0.5 * (Z.y - Zm.y)};
-      if (two) o[g.Fp + k] = C{(T)0.5 * (Z.y + Zm.y), (T)0.5 * (Zm.x - Z.x)};
+      o[k] = C{Z.x + Zm.x, Z.y - Zm.y};   // twice the spectrum: the kernels carry the factor
+      if (two) o[g.Fp + k] = C{Z.y + Zm.y, Zm.x - Z.x};
     }
   }
 }
 
-// one output line: out = scale * value (+ out when accumulate), every load before the stores; times is a further factor of
+// one output line: out = value (+ out when accumulate), every load before the stores; times is a further factor of
 // an output that is a multiple of the transform's (TIMES)
-template <bool TIMES, class T, class O, class C>
-__device__ __forceinline__ void write_line(const C *z, bool imag, O *o, double times, int nx0, T sc, bool accumulate,
+template <bool TIMES, class O, class C>
+__device__ __forceinline__ void write_line(const C *z, bool imag, O *o, double times, int nx0, bool accumulate,
                                            const FftProfile &prof, int lane)
 {
   for (int x0 = lane; x0 < nx0; x0 += 32 * kXBatch) {
@@ -461,7 +461,7 @@ __device__ __forceinline__ void write_line(const C *z, bool imag, O *o, double t
     for (int u = 0; u < kXBatch; u++)
       if (x0 + 32 * u < nx0) {
         const C r = z[x0 + 32 * u];
-        O v = (O)(sc * (imag ? r.y : r.x));   // scaled in the transform's arithmetic
+        O v = (O)(imag ? r.y : r.x);
         if (prof.n > 0) v += (O)(prof.c[0] * prof.s[0][x0 + 32 * u]);
         if (prof.n > 1) v += (O)(prof.c[1] * prof.s[1][x0 + 32 * u]);
         if (TIMES) v *= (O)times;
@@ -471,13 +471,12 @@ __device__ __forceinline__ void write_line(const C *z, bool imag, O *o, double t
 }
 
 // inverse: two half-spectrum lines as one complex line Z = A + iB, whose inverse's real and imaginary parts are the
-// outputs of the interior nodes (out[node] = scale * value, or += when accumulate)
+// outputs of the interior nodes (out[node] = value, or += when accumulate)
 template <class C, int LO, int HI>
 __global__ void __launch_bounds__((kXPairs * HI + 31) / 32 * 32) k_irfft_lines(OutBatch<C> ob, XGeom g,
                                                                                 Line1d<C> ln, int NP, int lp,
-                                                                                double scale, int accumulate)
+                                                                                int accumulate)
 {
-  using T = typename dft::Real<C>::T;
   const C *__restrict__ spec = ob.spec[blockIdx.y];
   extern __shared__ __align__(16) unsigned char smraw[];
   C *sm = reinterpret_cast<C *>(smraw);
@@ -496,7 +495,6 @@ __global__ void __launch_bounds__((kXPairs * HI + 31) / 32 * 32) k_irfft_lines(O
   }
   tile_fft<LO, HI, true, C>(sm, NP, lp, ln);
   const int nx0 = g.nx[0];
-  const T sc = (T)scale;
   const FftProfile prof = ob.prof[blockIdx.y];
   const int copies = ob.copies[blockIdx.y].n;
   for (int p = warp; p < np; p += nw) {
@@ -510,14 +508,14 @@ __global__ void __launch_bounds__((kXPairs * HI + 31) / 32 * 32) k_irfft_lines(O
       const C *zl = sm + p * lp + g.e[0];
       const bool acc = accumulate != 0;
       if (std::is_same<C, float2>::value && ob.out32[blockIdx.y]) {
-        write_line<false, T, float>(zl, h != 0, ob.out32[blockIdx.y] + row, 1.0, nx0, sc, acc, prof, lane);
+        write_line<false, float>(zl, h != 0, ob.out32[blockIdx.y] + row, 1.0, nx0, acc, prof, lane);
         for (int q = 0; q < copies; q++)
-          write_line<true, T, float>(zl, h != 0, ob.copies[blockIdx.y].out32[q] + row, ob.copies[blockIdx.y].f[q], nx0, sc,
+          write_line<true, float>(zl, h != 0, ob.copies[blockIdx.y].out32[q] + row, ob.copies[blockIdx.y].f[q], nx0,
                                      acc, prof, lane);
       } else {
-        write_line<false, T, double>(zl, h != 0, ob.out[blockIdx.y] + row, 1.0, nx0, sc, acc, prof, lane);
+        write_line<false, double>(zl, h != 0, ob.out[blockIdx.y] + row, 1.0, nx0, acc, prof, lane);
         for (int q = 0; q < copies; q++)
-          write_line<true, T, double>(zl, h != 0, ob.copies[blockIdx.y].out[q] + row, ob.copies[blockIdx.y].f[q], nx0, sc,
+          write_line<true, double>(zl, h != 0, ob.copies[blockIdx.y].out[q] + row, ob.copies[blockIdx.y].f[q], nx0,
                                       acc, prof, lane);
       }
     }
@@ -527,14 +525,14 @@ __global__ void __launch_bounds__((kXPairs * HI + 31) / 32 * 32) k_irfft_lines(O
 // correlation kernel of coefficient q of a stencil in the real box: coef[k * ncoef + q] added at (-dir offset_k) mod F
 // (offsets that wrap onto the same position add up); dir 1: sums over f(i + offset), -1: over f(i - offset)
 __global__ void k_fft_kernel_box(const short *__restrict__ off3, const double *__restrict__ coef, int L, int ncoef,
-                                 int q, int dir, double *__restrict__ box, int F0, int F1, int F2)
+                                 int q, int dir, double scale, double *__restrict__ box, int F0, int F1, int F2)
 {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= L) return;
   const int x = ((-dir * (int)off3[3 * k]) % F0 + F0) % F0;
   const int y = ((-dir * (int)off3[3 * k + 1]) % F1 + F1) % F1;
   const int z = ((-dir * (int)off3[3 * k + 2]) % F2 + F2) % F2;
-  atomicAdd(box + ((long)z * F1 + y) * F0 + x, coef[(long)k * ncoef + q]);
+  atomicAdd(box + ((long)z * F1 + y) * F0 + x, scale * coef[(long)k * ncoef + q]);
 }
 
 // the products of `t` as a spectrum, two points per thread and iteration, every term's loads issued before the sums
@@ -742,7 +740,7 @@ void forward_x(const SrcBatch<Src, C> &sb, int nb, const XGeom &g, const FftPlan
 }
 
 template <class C>
-void inverse_x(const OutBatch<C> &ob, int nb, const FftPlan &p, double scale, bool accumulate, cudaStream_t s)
+void inverse_x(const OutBatch<C> &ob, int nb, const FftPlan &p, bool accumulate, cudaStream_t s)
 {
   const XGeom g = xgeom(p);
   const FftAxis &ax = p.ax[0];
@@ -752,7 +750,7 @@ void inverse_x(const OutBatch<C> &ob, int nb, const FftPlan &p, double scale, bo
   with_range(ax.R1, [&](auto lo, auto hi) {
     constexpr int LO = decltype(lo)::value, HI = decltype(hi)::value;
     k_irfft_lines<C, LO, HI><<<grid, x_threads(ax, np), x_smem<C>(ax, np), s>>>(ob, g, line_of<C>(ax), np, x_pitch(ax),
-                                                                        scale, accumulate ? 1 : 0);
+                                                                        accumulate ? 1 : 0);
   });
 }
 
@@ -789,7 +787,7 @@ void rfft_forward_impl(const Src &src, bool mapped, C *spec, const FftPlan &p, c
 
 // inverse of the products in `terms`, formed by the first inverse pass into `spec` (the work box)
 template <class C>
-void rfft_inverse_impl(const Terms<C> &terms, C *spec, const FftPlan &p, double scale, double *out, float *out32,
+void rfft_inverse_impl(const Terms<C> &terms, C *spec, const FftPlan &p, double *out, float *out32,
                        bool accumulate, const FftProfile &prof, cudaStream_t s)
 {
   const Terms<C> none{};
@@ -807,7 +805,7 @@ void rfft_inverse_impl(const Terms<C> &terms, C *spec, const FftPlan &p, double 
   ob.out[0] = out;
   ob.out32[0] = out32;
   ob.prof[0] = prof;
-  inverse_x<C>(ob, 1, p, scale, accumulate, s);
+  inverse_x<C>(ob, 1, p, accumulate, s);
 }
 
 // nb forward transforms of mapped channels in one launch per pass
@@ -829,7 +827,7 @@ void rfft_forward_mapped_batch_impl(const MapSrc *m, int nb, C *const *spec, con
 
 // nb inverse transforms, output b the inverse of a * k[b] (formed by the first inverse pass in work[b])
 template <class C>
-void rfft_inverse_batch_impl(const C *a, const C *const *k, int nb, C *const *work, const FftPlan &p, double scale,
+void rfft_inverse_batch_impl(const C *a, const C *const *k, int nb, C *const *work, const FftPlan &p,
                              double *const *out, float *const *out32, bool accumulate, const FftProfile *prof,
                              const FftCopies *copies, cudaStream_t s)
 {
@@ -855,7 +853,7 @@ void rfft_inverse_batch_impl(const C *a, const C *const *k, int nb, C *const *wo
   }
   if (pending)
     for (int b = 0; b < nb; b++) launch_spec_terms<C>(pb.terms[b], work[b], p.NS, s);
-  inverse_x<C>(ob, nb, p, scale, accumulate, s);
+  inverse_x<C>(ob, nb, p, accumulate, s);
 }
 
 }  // namespace
@@ -959,23 +957,23 @@ Terms<C> make_terms(const C *const *a, const C *const *k, int n)
 }
 
 void rfft_inverse_products(const double2 *const *a, const double2 *const *k, int nterms, double2 *work,
-                           const FftPlan &p, double scale, double *out, bool accumulate, cudaStream_t s,
+                           const FftPlan &p, double *out, bool accumulate, cudaStream_t s,
                            const FftProfile &prof)
 {
-  rfft_inverse_impl<double2>(make_terms(a, k, nterms), work, p, scale, out, nullptr, accumulate, prof, s);
+  rfft_inverse_impl<double2>(make_terms(a, k, nterms), work, p, out, nullptr, accumulate, prof, s);
 }
 
 void rfft_inverse_products(const float2 *const *a, const float2 *const *k, int nterms, float2 *work,
-                           const FftPlan &p, double scale, double *out, bool accumulate, cudaStream_t s,
+                           const FftPlan &p, double *out, bool accumulate, cudaStream_t s,
                            const FftProfile &prof)
 {
-  rfft_inverse_impl<float2>(make_terms(a, k, nterms), work, p, scale, out, nullptr, accumulate, prof, s);
+  rfft_inverse_impl<float2>(make_terms(a, k, nterms), work, p, out, nullptr, accumulate, prof, s);
 }
 
 void rfft_inverse_products(const float2 *const *a, const float2 *const *k, int nterms, float2 *work,
-                           const FftPlan &p, double scale, float *out, bool accumulate, cudaStream_t s)
+                           const FftPlan &p, float *out, bool accumulate, cudaStream_t s)
 {
-  rfft_inverse_impl<float2>(make_terms(a, k, nterms), work, p, scale, nullptr, out, accumulate, FftProfile{}, s);
+  rfft_inverse_impl<float2>(make_terms(a, k, nterms), work, p, nullptr, out, accumulate, FftProfile{}, s);
 }
 
 int fft_max_terms() { return kMaxTerms; }
@@ -994,28 +992,28 @@ void rfft_forward_mapped_batch(const MapSrc *m, int nb, double2 *const *spec, co
 }
 
 void rfft_inverse_batch(const float2 *a, const float2 *const *k, int nb, float2 *const *work, const FftPlan &p,
-                        double scale, double *const *out, bool accumulate, cudaStream_t s, const FftProfile *prof,
+                        double *const *out, bool accumulate, cudaStream_t s, const FftProfile *prof,
                         const FftCopies *copies)
 {
   for (int b0 = 0; b0 < nb; b0 += kMaxBatch)
-    rfft_inverse_batch_impl<float2>(a, k + b0, std::min(kMaxBatch, nb - b0), work + b0, p, scale, out + b0, nullptr,
+    rfft_inverse_batch_impl<float2>(a, k + b0, std::min(kMaxBatch, nb - b0), work + b0, p, out + b0, nullptr,
                                     accumulate, prof ? prof + b0 : nullptr, copies ? copies + b0 : nullptr, s);
 }
 
 void rfft_inverse_batch(const float2 *a, const float2 *const *k, int nb, float2 *const *work, const FftPlan &p,
-                        double scale, float *const *out, bool accumulate, cudaStream_t s, const FftCopies *copies)
+                        float *const *out, bool accumulate, cudaStream_t s, const FftCopies *copies)
 {
   for (int b0 = 0; b0 < nb; b0 += kMaxBatch)
-    rfft_inverse_batch_impl<float2>(a, k + b0, std::min(kMaxBatch, nb - b0), work + b0, p, scale, nullptr, out + b0,
+    rfft_inverse_batch_impl<float2>(a, k + b0, std::min(kMaxBatch, nb - b0), work + b0, p, nullptr, out + b0,
                                     accumulate, nullptr, copies ? copies + b0 : nullptr, s);
 }
 
 void rfft_inverse_batch(const double2 *a, const double2 *const *k, int nb, double2 *const *work, const FftPlan &p,
-                        double scale, double *const *out, bool accumulate, cudaStream_t s, const FftProfile *prof,
+                        double *const *out, bool accumulate, cudaStream_t s, const FftProfile *prof,
                         const FftCopies *copies)
 {
   for (int b0 = 0; b0 < nb; b0 += kMaxBatch)
-    rfft_inverse_batch_impl<double2>(a, k + b0, std::min(kMaxBatch, nb - b0), work + b0, p, scale, out + b0, nullptr,
+    rfft_inverse_batch_impl<double2>(a, k + b0, std::min(kMaxBatch, nb - b0), work + b0, p, out + b0, nullptr,
                                      accumulate, prof ? prof + b0 : nullptr, copies ? copies + b0 : nullptr, s);
 }
 
@@ -1035,7 +1033,7 @@ void launch_fft_kernel_box(const short *off3, const double *coef, int L, int nco
                            const FftPlan &p, cudaStream_t s)
 {
   cudaMemsetAsync(box, 0, sizeof(double) * p.NR, s);
-  if (L > 0) k_fft_kernel_box<<<(L + 255) / 256, 256, 0, s>>>(off3, coef, L, ncoef, q, dir, box, p.F[0], p.F[1], p.F[2]);
+  if (L > 0) k_fft_kernel_box<<<(L + 255) / 256, 256, 0, s>>>(off3, coef, L, ncoef, q, dir, 0.25 / (double)p.NR, box, p.F[0], p.F[1], p.F[2]);
 }
 
 void launch_to_float2(const double2 *in, float2 *out, long n, cudaStream_t s)

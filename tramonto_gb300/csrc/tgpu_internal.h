@@ -118,32 +118,33 @@ struct MapSrc {
 void rfft_forward_mapped(const MapSrc &m, double2 *spec, const FftPlan &p, cudaStream_t s);
 void rfft_forward_mapped(const MapSrc &m, float2 *spec, const FftPlan &p, cudaStream_t s);
 void fft_free_plan(FftPlan &p);
-// half spectrum of a real box [F2][F1][F0]
+// twice the half spectrum of a real box [F2][F1][F0] (the transforms of real lines leave out the 1/2 of their split, and
+// launch_fft_kernel_box carries both factors and the inverse's 1/(F0 F1 F2))
 void rfft_forward_box(const double *box, double2 *spec, const FftPlan &p, cudaStream_t s);
-// out[node] (+)= scale * inverse transform of sum_t a_t k_t (nterms <= fft_max_terms() spectral products, formed by
+// out[node] (+)= unscaled inverse transform of sum_t a_t k_t (nterms <= fft_max_terms() spectral products, formed by
 // the first inverse pass) at the interior nodes; work holds the half spectrum in between
 void rfft_inverse_products(const double2 *const *a, const double2 *const *k, int nterms, double2 *work,
-                           const FftPlan &p, double scale, double *out, bool accumulate, cudaStream_t s,
+                           const FftPlan &p, double *out, bool accumulate, cudaStream_t s,
                            const FftProfile &prof = FftProfile{});
 void rfft_inverse_products(const float2 *const *a, const float2 *const *k, int nterms, float2 *work,
-                           const FftPlan &p, double scale, double *out, bool accumulate, cudaStream_t s,
+                           const FftPlan &p, double *out, bool accumulate, cudaStream_t s,
                            const FftProfile &prof = FftProfile{});
 void rfft_inverse_products(const float2 *const *a, const float2 *const *k, int nterms, float2 *work,
-                           const FftPlan &p, double scale, float *out, bool accumulate, cudaStream_t s);
+                           const FftPlan &p, float *out, bool accumulate, cudaStream_t s);
 int fft_max_terms();
 // several FP32 transforms of one plan per launch (blockIdx.y selects the transform): forward transforms of nb mapped
-// channels into spec[b]; inverse transforms out[b] (+)= scale * inverse of a * k[b] (work[b] the half spectra)
+// channels into spec[b]; inverse transforms out[b] (+)= unscaled inverse of a * k[b] (work[b] the half spectra)
 int fft_max_batch();
 void rfft_forward_mapped_batch(const MapSrc *m, int nb, float2 *const *spec, const FftPlan &p, cudaStream_t s);
 void rfft_forward_mapped_batch(const MapSrc *m, int nb, double2 *const *spec, const FftPlan &p, cudaStream_t s);
 void rfft_inverse_batch(const float2 *a, const float2 *const *k, int nb, float2 *const *work, const FftPlan &p,
-                        double scale, double *const *out, bool accumulate, cudaStream_t s,
+                        double *const *out, bool accumulate, cudaStream_t s,
                         const FftProfile *prof = nullptr, const FftCopies *copies = nullptr);
 void rfft_inverse_batch(const float2 *a, const float2 *const *k, int nb, float2 *const *work, const FftPlan &p,
-                        double scale, float *const *out, bool accumulate, cudaStream_t s,
+                        float *const *out, bool accumulate, cudaStream_t s,
                         const FftCopies *copies = nullptr);
 void rfft_inverse_batch(const double2 *a, const double2 *const *k, int nb, double2 *const *work, const FftPlan &p,
-                        double scale, double *const *out, bool accumulate, cudaStream_t s,
+                        double *const *out, bool accumulate, cudaStream_t s,
                         const FftProfile *prof = nullptr, const FftCopies *copies = nullptr);
 // per-launch CUDA-event timing of the FP32 y/z FFT passes (off unless enabled; collect reads and resets)
 void pass_timer_enable(bool on);
