@@ -2165,8 +2165,10 @@ __device__ __forceinline__ double warp_sum8(double *a)
 // out[0] = |w|^2.  One read of the basis per launch as long as it has at most eight vectors (MODE 1 keeps a node's eight
 // values in registers between the two uses).  Bound: the FP64 pipe (one FMA per 8 bytes of V and use: 3.4 us per vector
 // of 128^3 nodes) in the solves of large meshes, latency in small ones.  Per iteration of the 128^3 solve (4.7 vectors
-// on average) with dots, updates and norm as five launches: 215 us, as these three: 136 us; 40 401 nodes: 64 and 26 us.
-constexpr int kGsBlocks = 152 * 4;
+// on average) with dots, updates and norm as five launches: 215 us, as these three: 131 us; 40 401 nodes: 64 and 26 us.
+// CTAs: as many as are resident at once, so that the last wave is full and few partial sums are left (MODE 1 holds 91
+// registers: 63 us with 608 CTAs in two waves, 57 with 304; MODE 0 and 2 37 with 608, 42 to 45 with 304).
+constexpr int kGsBlocks = 152 * 4, kGsBlocksUpdate = 152 * 2;
 
 // one chunk of M vectors from V (the first chunk of MODE 1 and 2 also updates w, with all m vectors); M is a constant so
 // that a node's loads are all issued before their first use and no operation is spent on absent vectors
@@ -2261,14 +2263,17 @@ __global__ void __launch_bounds__(kThreads) k_gram_schmidt(double *__restrict__ 
   }
 }
 
-static int gs_blocks(long n) { return (int)std::min<long>(kGsBlocks, (n + kThreads - 1) / kThreads); }
+static int gs_blocks(int mode, long n)
+{
+  return (int)std::min<long>(mode == 1 ? kGsBlocksUpdate : kGsBlocks, (n + kThreads - 1) / kThreads);
+}
 
 // partial: the base of a kPartialWords reduction buffer (its last word is the completion counter)
 void launch_gram_schmidt(int mode, double *w, const double *V, long ldv, int m, long n, const double *hin,
                          double *partial, double *out, cudaStream_t s)
 {
   unsigned *counter = reinterpret_cast<unsigned *>(partial + kPartialWords - 1);
-  const int grid = gs_blocks(n);
+  const int grid = gs_blocks(mode, n);
   if (mode == 0) k_gram_schmidt<0><<<grid, kThreads, 0, s>>>(w, V, ldv, m, n, hin, partial, out, counter);
   else if (mode == 1) k_gram_schmidt<1><<<grid, kThreads, 0, s>>>(w, V, ldv, m, n, hin, partial, out, counter);
   else k_gram_schmidt<2><<<grid, kThreads, 0, s>>>(w, V, ldv, m, n, hin, partial, out, counter);
