@@ -148,10 +148,10 @@ class ClockSampler:
 
 # dram__bytes_read.sum + dram__bytes_write.sum of one k_sten_tc launch at 128^3 (ncu, one launch)
 TC_TRAFFIC_BYTES = 47.724e6 + 0.538e6
-# DRAM bytes per algorithmic byte of the FP32 y/z FFT pass launches (k_fft_stridedw<float2>) of a timed solve at
+# DRAM bytes per algorithmic byte of the FP32 y/z FFT pass launches (k_fft_lines<float2>) of a timed solve at
 # 128^3: ncu dram__bytes_read.sum + dram__bytes_write.sum summed over the launches, divided by their algorithmic
 # bytes (ncu flushes the caches before each profiled launch, so every launch reads from DRAM there)
-FFT32_PASS_TRAFFIC_BYTES_PER_BYTE = (27604.527e6 + 3098.825e6) / (512 * 99.893e6)
+FFT32_PASS_TRAFFIC_BYTES_PER_BYTE = 24557.3e6 / (512 * 76.970e6)
 
 
 def tc_issued_flops(p):
@@ -593,8 +593,8 @@ def main():
             # the largest share of the timed solve's launch list: the y and z passes of the FP32 FFT stencil sums
             # (every stencil sum of the Schur products and FP32 fills), each reading and writing the half spectrum
             "roofline": {"bound": "hbm",
-                         "kernel": "k_fft_stridedw<float2>: the y and z passes of the FP32 FFT stencil sums (one warp "
-                                   "per line, 16 lines per CTA), each launch a batch of transforms over the half "
+                         "kernel": "k_fft_lines<float2>: the y and z passes of the FP32 FFT stencil sums (two register "
+                                   "DFTs per line, 16 lines per CTA), each launch a batch of transforms over the half "
                                    "spectrum",
                          "achieved": launch_gbs, "peak": hbm, "unit": "GB/s", "frac": launch_gbs / hbm,
                          "peak_source": f"{peak_src} HBM copy (burst)",
@@ -611,7 +611,7 @@ def main():
                                            "timed solve at 128^3, per algorithmic byte, times this launch average",
                          "single_transform_pass": {"ms_y": t_pass_y, "ms_z": t_pass_z,
                                                    "achieved_gbs": pass_bytes / (t_pass * 1e-3) / 1e9,
-                                                   "note": "one transform per launch, 768 CTAs: 1.26 waves"},
+                                                   "note": "one transform per launch, 768 CTAs of 16 lines"},
                          "fp64_pass_ms_per_launch": t_pass64,
                          "fft32_attraction_sum": {
                              "ms_per_sum": t_wca_fft32,

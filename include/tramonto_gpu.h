@@ -186,7 +186,8 @@ int tgpu_set_fill_arithmetic(tgpu_handle h, int arith, double tau, double switch
  * model (direct float-float sum against the transforms) chooses. */
 int tgpu_set_fft_threshold(tgpu_handle h, int min_points);
 /* FP32 stencil sums (products, FP32 fills) as FP32 FFT convolutions: -1 (default) each sum's first use times
- * the FFT against its direct kernel and keeps the faster; 0 never; 1 always (3-D problems). */
+ * the FFT against its direct kernel and keeps the faster (in 2-D problems the sums of a pass together); 0 never;
+ * 1 always (3-D problems). */
 int tgpu_set_fft32_policy(tgpu_handle h, int policy);
 /* The choices of that policy so far, for stencil (type, index): choice[0] forward, choice[1] transposed sums
  * (1 FFT, -1 direct kernel, 0 not yet decided); ms[4] the timed direct and FFT sums behind them (forward direct,

@@ -13,24 +13,27 @@
 // (points that wrap onto the same position add up, as the reference folds a stencil wider than a periodic box),
 // one forward transform of the field, a product with the kernel's spectrum and one inverse transform give the
 // sum at a cost that does not depend on the stencil's length.  At 128^3 with the attraction reach of 25 nodes
-// that is a 180 x 128 x 128 box: 2.9e6 points against 5.8e6 for a box padded in every dimension.
+// that is a 160 x 128 x 128 box: 2.6e6 points (180 with both ends padded) against 5.8e6 for a box padded in every
+// dimension.
 //
 // The field is real, so only the half spectrum k0 < F0/2 + 1 is kept ([F2][F1][F0/2 + 1] complex): along x two
 // real lines are packed as the real and imaginary parts of one complex line, transformed together and split
-// by Hermitian symmetry (A[k] = (Z[k] + conj Z[-k]) / 2, B[k] = (Z[k] - conj Z[-k]) / 2i); the inverse packs
+// by Hermitian symmetry (2A[k] = Z[k] + conj Z[-k], 2B[k] = (Z[k] - conj Z[-k]) / i); the inverse packs
 // two half-spectrum lines as Z = A + iB (extended by conjugate symmetry) and returns them as the real and
 // imaginary parts of one inverse transform.  The x passes read the padded channel directly and write the
 // interior outputs directly (no load or extraction pass); the y and z passes are batches of complex transforms
 // over the half-spectrum box.
-//// Each 1-D transform of n = R1 R2 points (R1 >= R2, both <= 27) is two steps held in registers with one exchange
+//
+// Each 1-D transform of n = R1 R2 points (R1 >= R2, both <= 27) is two steps held in registers with one exchange
 // through shared memory between them (the four-step decomposition, Bailey 1990): R2 threads per line take the R1
 // points j2 + R2 r, transform them, multiply by W_n^{j2 k1} and store them; R1 threads read the R2 values of their
 // k1, transform them and hold the outputs k1 + R1 k2.  Both steps address global memory themselves, so a y or z pass
 // moves its data through shared memory once.  The y and z passes take 16 lines adjacent in x per CTA (16 lanes read
 // 128 or 256 contiguous bytes; with the line as the fastest index of the exchange no access conflicts).
 // Twiddles are tabulated on the host in extended precision.  The inverse uses conjugate twiddles; its 1/(F0 F1 F2) and
-// the 1/2 of the split into two real lines are factors of the kernels' coefficients (1 % of an FP64 fill).  The spectral products (one kernel spectrum per output, or the sum of channel-times-kernel
-// products of a transposed sum) are formed while the first inverse pass loads its lines.
+// the 1/2 of the split into two real lines are factors of the kernels' coefficients (1.6% of an FP64 fill).  The
+// spectral products (one kernel spectrum per output, or the sum of channel-times-kernel products of a transposed sum)
+// are formed while the first inverse pass loads its lines; FP32 sums of several products by a pass of their own.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -41,7 +44,7 @@
 
 namespace tgpu {
 
-using dft::cadd;
+using dft::cfma;
 using dft::cmul;
 
 namespace {
@@ -251,7 +254,8 @@ struct OutBatch {
 // Bound: FP32 by latency (issue 50%, L2 27%: load, exchange, store with four CTAs per SM), FP64 by the FP64 pipe
 // (~80% of its 304 operations per clock).  Measured on the 180 x 128 x 128 box (91 x 128 x 128 half spectrum), five
 // FP32 forward transforms per launch 26 us = 4.6 TB/s of spectrum read and written (39 us with radix-4 stages that
-// each went through shared memory); six FP64 inverse transforms with their products 400 us (430).
+// each went through shared memory); six FP64 inverse transforms with their products 400 us (430).  On the 160 x 128 x 128
+// box 21.7 and 365 us.
 // lines_per_cta adjacent lines (element stride es) at one outer index; reads `in` (or, inverse, the products of `terms`) and
 // writes `out` (in place when out == in: a CTA has read its lines before it writes them).  R1 in (LO, HI]: one kernel
 // per range of radices, so that short ones do not carry the registers of long ones.
@@ -301,7 +305,7 @@ __global__ void __launch_bounds__(lines_per_cta<C>() * HI) k_fft_lines(PassBatch
               a = terms.a[t] + i0;
               k = terms.k[t] + i0;
 #pragma unroll
-              for (int r = 0; r < R; r++) v[r] = cadd(v[r], cmul(a[r * step], __ldg(k + r * step)));
+              for (int r = 0; r < R; r++) v[r] = cfma(a[r * step], __ldg(k + r * step), v[r]);
             }
           }
         }
@@ -338,7 +342,8 @@ __global__ void __launch_bounds__(lines_per_cta<C>() * HI) k_fft_lines(PassBatch
 // shared memory: one warp reads or writes a line with consecutive lanes, and the two register steps work on the tile.
 // (Register steps that read and wrote global memory themselves, in runs of R1 or R2 elements, took 87 instead of 36 us
 // per FP32 inverse launch.)  Bound as the y and z passes; 128^3 workload, per launch of 1 and 5 or 6 lines' transforms:
-// forward 42 us in FP32 (47 with radix-4 stages), inverse 35 (33); FP64 271 (318) and 274 (338).
+// forward 42 us in FP32 (47 with radix-4 stages), inverse 35 (33); FP64 271 (318) and 274 (338) on the 180 x 128 x 128 box,
+// 35, 28, 232 and 278 on the 160 x 128 x 128 one.
 // Eight pairs per CTA: more and smaller CTAs than sixteen overlap one's loads with another's steps in FP32 (forward 37.3
 // -> 35.0 us, inverse 29.1 -> 27.7 on the 160 x 128 x 128 box; four: the same).
 constexpr int kXPairs = 8;
@@ -559,7 +564,7 @@ __global__ void __launch_bounds__(256) k_spec_terms(Terms<C> t, C *__restrict__ 
     C v[2] = {cmul(a[0][0], k[0][0]), cmul(a[0][1], k[0][1])};
 #pragma unroll
     for (int j = 1; j < N; j++)
-      for (int h = 0; h < 2; h++) v[h] = cadd(v[h], cmul(a[j][h], k[j][h]));
+      for (int h = 0; h < 2; h++) v[h] = cfma(a[j][h], k[j][h], v[h]);
     out[i] = v[0];
     out[i + 1] = v[1];
   }
@@ -791,7 +796,7 @@ void rfft_inverse_impl(const Terms<C> &terms, C *spec, const FftPlan &p, double 
                        bool accumulate, const FftProfile &prof, cudaStream_t s)
 {
   const Terms<C> none{};
-  // A sum of several FP32 products is formed by a pass of its own (five terms at 128^3: 24 + 9 us; 70 us inside the
+  // A sum of several FP32 products is formed by a pass of its own (five terms at 128^3: 20 + 9 us; 70 us inside the
   // z pass, whose threads wait for each term in turn).  FP64 sums stay in the z pass, bound by their arithmetic there.
   bool pending = !(std::is_same<C, float2>::value && terms.n > 1) && p.F[2] * p.F[1] > 1;   // products not formed yet
   if (!pending) launch_spec_terms<C>(terms, spec, p.NS, s);

@@ -29,6 +29,12 @@ __device__ __forceinline__ C cmul(C a, C b)
 {
   return C{a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x};
 }
+// c + a b, in four operations (a product and a sum: six)
+template <class C>
+__device__ __forceinline__ C cfma(C a, C b, C c)
+{
+  return C{fma(-a.y, b.y, fma(a.x, b.x, c.x)), fma(a.y, b.x, fma(a.x, b.y, c.y))};
+}
 template <class C>
 __device__ __forceinline__ C cadd(C a, C b)
 {
