@@ -348,6 +348,7 @@ __global__ void __launch_bounds__(kLineThreads) k_gmres_line(LineArgs<T> a)
     // ---- phase 1
     if (owner) {
       const double rhn = 1.0 / hn;
+      const bool quick = sizeof(T) == sizeof(float) && hn > 1e-300 && hn < 1e300;   // (rhn neither infinite nor subnormal)
       for (int t = kLineThreads - 1 - tid; t < nc * own; t += kLineThreads) {
         const int ic = t / own, il = t - ic * own;
         const double v = w[ic * per + il] / hn;
@@ -361,7 +362,7 @@ __global__ void __launch_bounds__(kLineThreads) k_gmres_line(LineArgs<T> a)
           T v = m == -1 ? (T)0 : (T)__longlong_as_double(0x7ff8000000000000ULL);
           if (m >= 0) {
             const double u = __ldcg(wbuf + (long)ic * N + m);
-            v = (T)(sizeof(T) == sizeof(double) ? u / hn : u * rhn);
+            v = (T)(quick ? u * rhn : u / hn);
           }
           win[ic * nw + t] = v;
         }
