@@ -192,7 +192,7 @@ struct Ctx : tgpu_ctx {
   float t32_att[2][2] = {{0.f, 0.f}, {0.f, 0.f}};   // [slab context, tensor-core context][direct, FFT] ms
   long fft32_gen = -1;
   int fft32_ch = -1;
-  double *d_dscr = nullptr;      // [4 + 2 ndim][N] outputs of the timing runs that make the choices
+  double *d_dscr = nullptr;      // [nrb + ncomp][N] outputs of the timing runs that make the choices
   bool spec32_built = false;
   // the channels of the last pad(): the padded box is written only when a direct kernel needs it (FFT sums read
   // the channels through the boundary maps)
@@ -792,6 +792,13 @@ void decide_fft32(Ctx *c)
   c->t32_att[c->tc_on ? 1 : 0][1] = 0.5f * t_fft;
 }
 
+// where the timing runs below write their sums (never the pass's own rows, which may hold sums to add to)
+double *choice_scratch(Ctx *c)
+{
+  if (!c->d_dscr) c->d_dscr = dalloc<double>((size_t)(c->dg.nrb + c->dg.ncomp) * c->dg.N);
+  return c->d_dscr;
+}
+
 // The same choice for one short stencil (theta, delta) and direction: its FP32 slab / point sum against the
 // FP32 FFT, timed once on the padded channels ch0.. into d_dscr.  The FFT runs after the first reuse the
 // field's transform when it is the one the forward sums share (the channel's spectrum stays cached).
@@ -803,9 +810,8 @@ void decide_fft32_sten(Ctx *c, DevStencil &st, bool tr, int ch0, int nin, int no
   if (!prepare_spec32(c)) return;
   if (tr ? (int)st.spec_tr32.size() != nin : (int)st.spec_fwd32.size() != nout) return;
   const long N = c->dg.N;
-  if (!c->d_dscr) c->d_dscr = dalloc<double>((size_t)tgpu::kMaxRb * N);
   double *o[tgpu::kMaxRb];
-  for (int q = 0; q < nout; q++) o[q] = c->d_dscr + (long)q * N;
+  for (int q = 0; q < nout; q++) o[q] = choice_scratch(c) + (long)q * N;
   cudaEvent_t ev[4];
   for (auto &e : ev) ck(cudaEventCreate(&e), "event");
   conv(c, ch0, nin, st, tr, o, nout, true);   // warm-up of the direct sum
@@ -995,7 +1001,8 @@ void transpose_convs(Ctx *c, const std::vector<DevStencil> *sten, double *out, b
 // In 2-D the FP32 sums of a pass choose together: one transform of the field (or of the channels) serves them all and a
 // pass of FFTs is a few launches whatever the stencils, so a sum alone says little (201 x 201 slit: theta 11 us and
 // delta 17 us direct against 42 us as an FFT of its own, but 38 us of direct sums next to the attraction's FFT against
-// 8 us more for its outputs).  The whole pass is timed both ways, on the recorded channels into the pass's own output.
+// 8 us more for its outputs).  The whole pass is timed both ways, on the recorded channels into scratch rows (a refined
+// fill's own rows hold its reference sums).
 void decide_fft32_2d(Ctx *c, bool tr)
 {
   const tgpu::DevGeom &g = c->dg;
@@ -1011,9 +1018,10 @@ void decide_fft32_2d(Ctx *c, bool tr)
   if (!open) return;
   for (int *f : flags) *f = -1;
   if (!prepare_spec32(c)) return;
+  double *scr = choice_scratch(c);
   auto pass = [&] {
-    if (tr) transpose_convs(c, c->sten, c->d_tr, true);
-    else forward_convs(c, c->sten, c->d_conv, true);
+    if (tr) transpose_convs(c, c->sten, scr, true);
+    else forward_convs(c, c->sten, scr, true);
   };
   cudaEvent_t ev[4];
   for (auto &e : ev) ck(cudaEventCreate(&e), "event");
