@@ -1546,7 +1546,7 @@ tgpu::LineResult gmres_line(Ctx *c, int per, const double *d_rhs, double *d_x2, 
   }
   if (!c->d_line_kind) {
     c->d_line_kind = dalloc<signed char>(c->n2);
-    c->d_line_bar = dalloc<unsigned>(2);
+    c->d_line_bar = dalloc<unsigned>(tgpu::kLineBarWords);
     c->d_line_res = dalloc<tgpu::LineResult>(1);
     ck(cudaMallocHost(&c->h_line_res, sizeof(tgpu::LineResult) + 2 * sizeof(unsigned)), "cudaMallocHost");
   }
@@ -1576,7 +1576,7 @@ tgpu::LineResult gmres_line(Ctx *c, int per, const double *d_rhs, double *d_x2, 
   q.kind = c->d_line_kind;
   q.bar = c->d_line_bar;
   q.res = c->d_line_res;
-  ck(cudaMemsetAsync(c->d_line_bar, 0, 2 * sizeof(unsigned), c->stream), "memset");
+  ck(cudaMemsetAsync(c->d_line_bar, 0, tgpu::kLineBarWords * sizeof(unsigned), c->stream), "memset");
   ck(tgpu::launch_gmres_line(q, c->stream), "one-launch GMRES");
   unsigned *h_bar = reinterpret_cast<unsigned *>(c->h_line_res + 1);
   ck(cudaMemcpyAsync(c->h_line_res, c->d_line_res, sizeof(tgpu::LineResult), cudaMemcpyDeviceToHost, c->stream), "d2h");

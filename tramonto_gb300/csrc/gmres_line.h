@@ -43,7 +43,7 @@ struct LineArgs {
   double *V, *part, *R, *y, *xout;
   T *chan;
   signed char *kind;
-  unsigned *bar;        // arrivals, error
+  unsigned *bar;        // arrivals, error, stop (set by the block without nodes, nothing clears it within the launch)
   LineResult *res;
   long ldv;             // ncomp * N
   int per, kdim, m;     // nodes per CTA, vectors that R holds, steps of this cycle
@@ -498,10 +498,10 @@ __global__ void __launch_bounds__(kLineThreads) k_gmres_line(LineArgs<T> a)
       }
     } else if (k > 0 && tid == 0) {
       rotate(k - 1);
-      a.res->its = rel < a.tol ? -k : 0;   // its < 0: converged after -its steps
+      if (rel < a.tol) __stcg(a.bar + 2, 1u);   // converged after k steps
     }
     if (!line_barrier(a.bar, gen)) return;
-    if (k > 0 && __ldcg(&a.res->its) < 0) {
+    if (k > 0 && __ldcg(a.bar + 2) != 0u) {   // (a word of its own: late readers must not meet the result's)
       cols = k;
       break;
     }
@@ -721,7 +721,7 @@ static cudaError_t gmres_line_t(const LineCall &q, cudaStream_t s)
   return line_launch_nt<T, false>(a, nc, grid, smem, s);
 }
 
-// One GMRES cycle of a 1-D problem (the caller has zeroed q.bar's two words)
+// One GMRES cycle of a 1-D problem (the caller has zeroed q.bar's kLineBarWords words)
 cudaError_t launch_gmres_line(const LineCall &q, cudaStream_t s)
 {
   return q.f32 ? gmres_line_t<float>(q, s) : gmres_line_t<double>(q, s);

@@ -635,6 +635,7 @@ struct LineResult {
   int status, its;      // status 1: a non-finite norm
   double r0, rel;       // |M^-1 b|, the last residual estimate over it
 };
+constexpr int kLineBarWords = 3;
 struct LineCall {
   const std::vector<DevStencil> *sten;   // [3]
   int ncomp, attraction, per, h, kdim, m;
@@ -646,7 +647,7 @@ struct LineCall {
   double *V, *part, *R, *y, *xout;
   void *chan;
   signed char *kind;
-  unsigned *bar;        // two words, zero before the launch; the second is set when a barrier gave up
+  unsigned *bar;        // kLineBarWords words, zero before the launch; the second is set when a barrier gave up
   LineResult *res;
 };
 // the point sums of a pass of a 1-D problem in one launch (line_sums.h)
