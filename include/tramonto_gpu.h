@@ -526,6 +526,10 @@ int tgpu_time_fft_pass(tgpu_handle h, int precision, int axis, int reps, double 
  * reports as TGPU_ERR_CUDA ("a bounded wait ran out").  A tiny limit makes the waits run out on purpose, to
  * exercise that path.  No reference counterpart. */
 int tgpu_set_tc_wait_limit(tgpu_handle h, long spins);
+/* The same for the grid barriers of the one-launch GMRES of 1-D problems (polls; at most and by default 2^24): a block
+ * whose wait runs out sets the error flag and returns, as then do all others, and the solve reports TGPU_ERR_CUDA ("a
+ * bounded wait ran out").  The handle stays usable.  No reference counterpart. */
+int tgpu_set_gmres_wait_limit(tgpu_handle h, long spins);
 
 /* Timing of the device work of the last call, per kernel family (ms), for benchmarks. */
 typedef struct {

@@ -216,7 +216,7 @@ struct Ctx : tgpu_ctx {
   signed char *d_line_kind = nullptr;
   unsigned *d_line_bar = nullptr;
   tgpu::LineResult *d_line_res = nullptr, *h_line_res = nullptr;
-  int line_kdim = 0, nsm = 0, smem_max = 0;
+  int line_kdim = 0, line_spin = tgpu::kLineSpin, nsm = 0, smem_max = 0;
   double *d_inv32 = nullptr;           // 1/rho of the state's Euler-Lagrange rows, and their kinds (k_row_info32)
   signed char *d_kind32 = nullptr;
   int hcoef32_form = -1;
@@ -1558,6 +1558,7 @@ tgpu::LineResult gmres_line(Ctx *c, int per, const double *d_rhs, double *d_x2, 
   q.h = g.h[0];
   q.kdim = kdim;
   q.m = m;
+  q.spin = c->line_spin;
   q.transpose = c->gmres_transpose;
   q.f32 = prod_f32(c) && !c->gmres_transpose;
   q.N = g.N;
@@ -3736,6 +3737,17 @@ int tgpu_time_stencil_sum(tgpu_handle h, int type, int index, int precision, int
     c->fft32_slab = fft32_prev[1];
     tc_check(c);
     *ms_per_sum = ms / reps;
+    return TGPU_OK;
+  });
+}
+
+int tgpu_set_gmres_wait_limit(tgpu_handle h, long spins)
+{
+  return guard([&] {
+    Ctx *c = C(h);
+    need_final(c);
+    if (c->dg.ndim != 1) throw Error(TGPU_ERR_UNSUPPORTED, "one-launch GMRES exists for 1-D problems only");
+    c->line_spin = spins > 0 ? (int)std::min<long>(spins, tgpu::kLineSpin) : tgpu::kLineSpin;
     return TGPU_OK;
   });
 }

@@ -25,7 +25,6 @@
 // TR: the transposed Schur complement (adjoint solves), from the stencils with negated offsets.
 
 constexpr int kLineThreads = 256, kLineTile = 8, kLineGroups = 32, kLineWarps = kLineThreads / 32;
-constexpr int kLineSpin = 1 << 24;   // polls before a barrier gives up
 
 template <class T>
 struct LineSten {
@@ -47,11 +46,12 @@ struct LineArgs {
   LineResult *res;
   long ldv;             // ncomp * N
   int per, kdim, m;     // nodes per CTA, vectors that R holds, steps of this cycle
+  int spin;             // polls before a barrier gives up
   double tol;
 };
 
 // Barrier over the grid; false when it gave up (then every block returns)
-__device__ __forceinline__ bool line_barrier(unsigned *bar, unsigned &gen)
+__device__ __forceinline__ bool line_barrier(unsigned *bar, unsigned &gen, int limit)
 {
   __shared__ int s_ok;
   __syncthreads();
@@ -63,7 +63,7 @@ __device__ __forceinline__ bool line_barrier(unsigned *bar, unsigned &gen)
     unsigned seen;
     do {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-      if (++spins > kLineSpin) {
+      if (++spins > limit) {
         atomicExch(bar + 1, 1u);
         ok = 0;
         break;
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(kLineThreads) k_gmres_line(LineArgs<T> a)
       tab[r * per + il] = (T)v;
     }
   }
-  if (!line_barrier(a.bar, gen)) return;
+  if (!line_barrier(a.bar, gen, a.spin)) return;
   const double r0 = line_norm(partA, nblk);
   if (!(r0 > 0.0)) {   // a zero or non-finite right-hand side: the host decides
     for (int t = tid; t < nc * own; t += kLineThreads) {
@@ -500,7 +500,7 @@ __global__ void __launch_bounds__(kLineThreads) k_gmres_line(LineArgs<T> a)
       rotate(k - 1);
       if (rel < a.tol) __stcg(a.bar + 2, 1u);   // converged after k steps
     }
-    if (!line_barrier(a.bar, gen)) return;
+    if (!line_barrier(a.bar, gen, a.spin)) return;
     if (k > 0 && __ldcg(a.bar + 2) != 0u) {   // (a word of its own: late readers must not meet the result's)
       cols = k;
       break;
@@ -557,14 +557,14 @@ __global__ void __launch_bounds__(kLineThreads) k_gmres_line(LineArgs<T> a)
       }
       dots(partA);
     }
-    if (!line_barrier(a.bar, gen)) return;
+    if (!line_barrier(a.bar, gen, a.spin)) return;
     // ---- phase 3
     line_reduce(partA, k + 1, nblk, h1);
     if (owner) {
       combine(h1, k + 1, [&](int ic, int il, double d) { w[ic * per + il] -= d; });
       dots(partB);
     }
-    if (!line_barrier(a.bar, gen)) return;
+    if (!line_barrier(a.bar, gen, a.spin)) return;
     // ---- phase 4
     line_reduce(partB, k + 1, nblk, h2);
     if (owner) {
@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(kLineThreads) k_gmres_line(LineArgs<T> a)
       }
       if (tid == 0) partA[blockIdx.x] = d;   // (every block has read h1's partials)
     }
-    if (!line_barrier(a.bar, gen)) return;
+    if (!line_barrier(a.bar, gen, a.spin)) return;
     hn = line_norm(partA, nblk);
     if (!isfinite(hn) || hn == 0.0) {   // (the same in every block)
       status = isfinite(hn) ? 0 : 1;
@@ -624,7 +624,7 @@ __global__ void __launch_bounds__(kLineThreads) k_gmres_line(LineArgs<T> a)
     }
     if (tid == 0) *a.res = LineResult{status, cols, r0, rel};
   }
-  if (!line_barrier(a.bar, gen)) return;
+  if (!line_barrier(a.bar, gen, a.spin)) return;
   if (status != 0 || !owner) return;
   for (int j = tid; j < cols; j += kLineThreads) h1[j] = __ldcg(a.y + j);
   __syncthreads();
@@ -713,6 +713,7 @@ static cudaError_t gmres_line_t(const LineCall &q, cudaStream_t s)
   a.per = q.per;
   a.kdim = q.kdim;
   a.m = q.m;
+  a.spin = q.spin;
   a.tol = q.tol;
   const int grid = (int)((q.N + q.per - 1) / q.per) + 1;
   const size_t smem = gmres_line_smem(nc, q.transpose, sizeof(T) == sizeof(float), q.kdim, q.per, q.h);

@@ -636,9 +636,10 @@ struct LineResult {
   double r0, rel;       // |M^-1 b|, the last residual estimate over it
 };
 constexpr int kLineBarWords = 3;
+constexpr int kLineSpin = 1 << 24;   // polls before a barrier of the grid gives up, unless the caller sets a limit
 struct LineCall {
   const std::vector<DevStencil> *sten;   // [3]
-  int ncomp, attraction, per, h, kdim, m;
+  int ncomp, attraction, per, h, kdim, m, spin;
   bool transpose, f32;
   long N;
   double tol;

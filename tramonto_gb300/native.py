@@ -91,7 +91,7 @@ def load(build_if_missing: bool = False):
         "tgpu_set_fft_threshold": [vp, C.c_int],
         "tgpu_set_fft32_policy": [vp, C.c_int],
         "tgpu_fft32_choice": [vp, C.c_int, C.c_int, ip, dp],
-        "tgpu_set_tc_wait_limit": [vp, C.c_long],
+        "tgpu_set_tc_wait_limit": [vp, C.c_long], "tgpu_set_gmres_wait_limit": [vp, C.c_long],
         "tgpu_time_fft_pass": [vp, C.c_int, C.c_int, C.c_int, dp, C.POINTER(C.c_long), C.POINTER(C.c_long)],
         "tgpu_pass_timer_begin": [vp],
         "tgpu_pass_timer_end": [vp, C.POINTER(C.c_long), dp, dp, C.POINTER(C.c_long)],
