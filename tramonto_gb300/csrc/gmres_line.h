@@ -194,6 +194,22 @@ __device__ __forceinline__ void line_taps(const LineSten<T> &st, const T *win, i
   }
 }
 
+// the same for one input into sums over components; FP32 sums are added to them in FP64
+template <int NO, int NT, class T, class A>
+__device__ __forceinline__ void line_add(const LineSten<T> &st, const T *win, int ld, int grp, A (*acc)[NT])
+{
+  if constexpr (std::is_same<A, T>::value) {
+    line_taps<1, NO, NT, T>(st, win, ld, grp, acc);
+  } else {
+    T d[NO][NT] = {};
+    line_taps<1, NO, NT, T>(st, win, ld, grp, d);
+#pragma unroll
+    for (int o = 0; o < NO; o++)
+#pragma unroll
+      for (int u = 0; u < NT; u++) acc[o][u] += (A)d[o][u];
+  }
+}
+
 // shared memory of a CTA; `per` nodes, a window of nw = per + 2 h positions, NT tiles at a time
 constexpr int kLineRb = 6, kLineTable = kHessCoef + kLineRb;   // 1-D weighted densities; a node's table: n, coefficients
 struct LineSmem {
@@ -201,12 +217,12 @@ struct LineSmem {
 };
 __host__ __device__ inline LineSmem line_layout(int nc, int ncols, bool tr, int kdim, int per, int nw, int nt, size_t t)
 {
-  const size_t nch = (size_t)(tr ? 4 * nc : 3 * nc), rows = kLineRb + ncols;
+  const size_t nch = (size_t)(tr ? 4 * nc : 3 * nc), rows = kLineRb + ncols, ts = ncols > 1 ? sizeof(double) : t;
   LineSmem m;
   m.win = 0;
   m.red = (t * nch * nw + 15) & ~(size_t)15;
   m.tab = m.red + sizeof(double) * rows * nt * kLineWarps * kLineTile;
-  m.dbl = (m.tab + t * ((size_t)kLineTable * per + rows * nt * kLineTile) + 15) & ~(size_t)15;
+  m.dbl = (m.tab + t * (size_t)kLineTable * per + ts * rows * nt * kLineTile + 15) & ~(size_t)15;
   // w, -u_MF, V_k, rho, V_k / rho; h1, h2; rotations and right-hand side
   m.idx = m.dbl + sizeof(double) * (5 * (size_t)nc * per + 2 * (kdim + 2) + 3 * (size_t)kdim + 1);
   m.bytes = m.idx + sizeof(int) * (size_t)(nc + 1) * nw + (size_t)nc * per;
@@ -217,6 +233,7 @@ template <class T, bool TR, int NC, int NT>
 __global__ void __launch_bounds__(kLineThreads) k_gmres_line(LineArgs<T> a)
 {
   constexpr int NRB = kLineRb, CPC = 3, STEP = NT * kLineTile, ROWS = NRB + NC;
+  using A = typename std::conditional<NC == 1, T, double>::type;   // sums over components: of FP32 sums in FP64
   extern __shared__ __align__(16) unsigned char smraw[];
   const int nc = NC == 1 ? 1 : c_g.ncomp, per = a.per, h = c_g.h[0], nw = per + 2 * h;
   const long N = c_g.N;
@@ -226,8 +243,9 @@ __global__ void __launch_bounds__(kLineThreads) k_gmres_line(LineArgs<T> a)
   const LineSmem lay = line_layout(nc, NC, TR, a.kdim, per, nw, NT, sizeof(T));
   T *win = reinterpret_cast<T *>(smraw);
   double *red = reinterpret_cast<double *>(smraw + lay.red);
-  T *redT = reinterpret_cast<T *>(red);
-  T *tab = reinterpret_cast<T *>(smraw + lay.tab), *sums = tab + kLineTable * per;   // [kLineTable][per], [ROWS][STEP]
+  A *redA = reinterpret_cast<A *>(red);
+  T *tab = reinterpret_cast<T *>(smraw + lay.tab);           // [kLineTable][per]
+  A *sums = reinterpret_cast<A *>(tab + kLineTable * per);   // [ROWS][STEP]
   double *w = reinterpret_cast<double *>(smraw + lay.dbl), *ymf = w + nc * per, *vown = ymf + nc * per;
   double *rho = vown + nc * per, *vr = rho + nc * per;
   double *h1 = vr + nc * per, *h2 = h1 + a.kdim + 2, *cs = h2 + a.kdim + 2, *sn = cs + a.kdim, *gv = sn + a.kdim;
@@ -371,25 +389,25 @@ __global__ void __launch_bounds__(kLineThreads) k_gmres_line(LineArgs<T> a)
         const int at = t0 + nl + h;
         if constexpr (NC == 1 && !TR) {
           if (one) {   // rows n3, n2, V2 and the mean field
-            T acc[4][NT] = {};
+            A acc[4][NT] = {};
             line_taps<1, 1, NT, T>(a.th[0], win + at, nw, grp, acc);
             line_taps<1, 2, NT, T>(a.de[0], win + at, nw, grp, acc + 1);
             if (att) {
               line_taps<1, 1, NT, T>(a.ua[0], win + at, nw, grp, acc + 3);
-              line_warp_sums(reinterpret_cast<const T (&)[4 * NT]>(acc), redT);
+              line_warp_sums(reinterpret_cast<const A (&)[4 * NT]>(acc), redA);
             } else {
-              line_warp_sums(reinterpret_cast<const T (&)[3 * NT]>(acc), redT);
+              line_warp_sums(reinterpret_cast<const A (&)[3 * NT]>(acc), redA);
             }
             __syncthreads();
             if (tid < (att ? 4 : 3) * STEP) {
               const int r = tid / STEP;
               const int row = r == 0 ? 0 : r == 1 ? 1 : r == 2 ? 4 : NRB;
-              sums[row * STEP + tid % STEP] = line_final<T>(redT, tid / kLineTile, nl);
+              sums[row * STEP + tid % STEP] = line_final<A>(redA, tid / kLineTile, nl);
             }
           }
         }
         if (NC != 1 || TR || !one) {
-          T acc[ROWS][NT] = {};
+          A acc[ROWS][NT] = {};
           if constexpr (TR) {
             // per component (scalar, vector) of the delta shell and the ball: combined at once into the rows of g
             // (n ordering: acc 0..5 = g0 g1 g2 g3 gV1 gV2)
@@ -413,27 +431,27 @@ __global__ void __launch_bounds__(kLineThreads) k_gmres_line(LineArgs<T> a)
             for (int jc = 0; jc < NC; jc++)
               if (jc < nc) {
                 const T *wj = win + jc * nw + at;
-                line_taps<1, 1, NT, T>(a.th[jc], wj, nw, grp, acc);          // n3
+                line_add<1, NT>(a.th[jc], wj, nw, grp, acc);             // n3
                 if (one) {
                   T d[2][NT] = {};
-                  line_taps<1, 2, NT, T>(a.de[jc], wj, nw, grp, d);          // n2, V2
+                  line_taps<1, 2, NT, T>(a.de[jc], wj, nw, grp, d);      // n2, V2
 #pragma unroll
                   for (int u = 0; u < NT; u++) {
-                    acc[1][u] += d[0][u];
-                    acc[4][u] += d[1][u];
+                    acc[1][u] += (A)d[0][u];
+                    acc[4][u] += (A)d[1][u];
                   }
                 } else {
-                  line_taps<1, 5, NT, T>(a.de[jc], wj, nw, grp, acc + 1);    // n2, n1, n0, V2, V1
+                  line_add<5, NT>(a.de[jc], wj, nw, grp, acc + 1);       // n2, n1, n0, V2, V1
                 }
                 if (att)
 #pragma unroll
                   for (int ic = 0; ic < NC; ic++)
-                    if (ic < nc) line_taps<1, 1, NT, T>(a.ua[ic + nc * jc], wj, nw, grp, acc + NRB + ic);
+                    if (ic < nc) line_add<1, NT>(a.ua[ic + nc * jc], wj, nw, grp, acc + NRB + ic);
               }
           }
-          line_warp_sums(reinterpret_cast<const T (&)[ROWS * NT]>(acc), redT);
+          line_warp_sums(reinterpret_cast<const A (&)[ROWS * NT]>(acc), redA);
           __syncthreads();
-          if (tid < ROWS * STEP) sums[tid] = line_final<T>(redT, tid / kLineTile, nl);
+          if (tid < ROWS * STEP) sums[tid] = line_final<A>(redA, tid / kLineTile, nl);
         }
         __syncthreads();
         // local step; another warp forms what depends on the vector alone
@@ -459,14 +477,14 @@ __global__ void __launch_bounds__(kLineThreads) k_gmres_line(LineArgs<T> a)
             T n[NRB], y[NRB], z[NRB];
             HessCoefT<T> c;
             if constexpr (TR) {
-              for (int r = 0; r < NRB; r++) y[r] = sums[r * STEP + tl];
+              for (int r = 0; r < NRB; r++) y[r] = (T)sums[r * STEP + tl];
             } else {
               T ysv[NRB];
               for (int r = 0; r < NRB; r++) {
                 int src;
                 double cd;
-                if (dep_rb(r, &src, &cd)) ysv[r] = -to_arith<T>(cd) * sums[src * STEP + tl];   // -u_dep - B u_ind
-                else ysv[r] = -sums[r * STEP + tl];
+                if (dep_rb(r, &src, &cd)) ysv[r] = -to_arith<T>(cd) * (T)sums[src * STEP + tl];   // -u_dep - B u_ind
+                else ysv[r] = -(T)sums[r * STEP + tl];
               }
               y[0] = ysv[3]; y[1] = ysv[2]; y[2] = ysv[1]; y[3] = ysv[0]; y[4] = ysv[5]; y[5] = ysv[4];
             }
