@@ -1229,24 +1229,24 @@ void launch_hess_coef32(long N, int ndim, int fn, const double *x, float *coef, 
 }
 
 // H y from a node's rows of the FP32 table (state's scalars, V1 and V2 per dimension) in the n ordering.  ALPHA: the
-// functionals whose third term has the alpha form; for the others (FMT1, FMT3) g2v f = -6 f, g_vv f = -h22, no outer
-// product, and a^2 is formed: seven scalars are read instead of twelve.
+// functionals whose third term has the alpha form; for the others (FMT1, FMT3) the n2-V2 entries of both sides are one
+// row, g_vv f = -h22 and there is no outer product: eight scalars are read instead of twelve.
 template <int ND, bool ALPHA>
 struct Hess32 {
-  float a, h13, h22, h23, h33, ff, gvf1, a2, g2vr, g2vc, gvv, gvvo, V1[ND], V2[ND];
+  float a, a2, h13, h22, h23, h33, ff, gvf1, g2vr, g2vc, gvv, gvvo, V1[ND], V2[ND];
   __device__ __forceinline__ void load(const float *__restrict__ coef, long N, long i)
   {
     const float *c = coef + i;
     a = c[0];
+    a2 = c[N];
     h13 = c[2 * N];
     h22 = c[3 * N];
     h23 = c[4 * N];
     h33 = c[5 * N];
-    ff = c[6 * N];
     gvf1 = c[7 * N];
+    g2vr = c[8 * N];
     if (ALPHA) {
-      a2 = c[N];
-      g2vr = c[8 * N];
+      ff = c[6 * N];
       g2vc = c[9 * N];
       gvv = c[10 * N];
       gvvo = c[11 * N];
@@ -1259,19 +1259,19 @@ struct Hess32 {
   }
   __device__ __forceinline__ void apply(const float *y, float *z) const
   {
-    const float aa = ALPHA ? a2 : a * a, row = ALPHA ? g2vr : -6.0f * ff, col = ALPHA ? g2vc : row;
+    const float col = ALPHA ? g2vc : g2vr;
     float Vy = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll
     for (int d = 0; d < ND; d++) Vy += V2[d] * y[4 + ND + d];
 #pragma unroll
     for (int d = 0; d < ND; d++) {
-      const float h3v2 = gvf1 * V2[d] - V1[d] * aa;
-      s3 += h3v2 * y[4 + ND + d] - V2[d] * aa * y[4 + d];
-      z[4 + d] = -V2[d] * aa * y[3] - a * y[4 + ND + d];
+      const float h3v2 = gvf1 * V2[d] - V1[d] * a2;
+      s3 += h3v2 * y[4 + ND + d] - V2[d] * a2 * y[4 + d];
+      z[4 + d] = -V2[d] * a2 * y[3] - a * y[4 + ND + d];
       const float vv = ALPHA ? ff * (gvv * y[4 + ND + d] + gvvo * V2[d] * Vy) : -h22 * y[4 + ND + d];
       z[4 + ND + d] = col * V2[d] * y[2] + h3v2 * y[3] - a * y[4 + d] + vv;
     }
-    s2 = row * Vy;
+    s2 = g2vr * Vy;
     z[0] = a * y[3];
     z[1] = a * y[2] + h13 * y[3];
     z[2] = a * y[1] + h22 * y[2] + h23 * y[3] + s2;
@@ -1306,8 +1306,8 @@ __device__ __forceinline__ void write_chan32(const float *z, const float (*s_c)[
 
 // k_schur_local with every operand in FP32 storage (conv [nrb + ncomp][N] the stencil sums of A12 v, chan the
 // transposed-sum channels, ymf = -u_MF); ND the dimension, so that the per-node arrays stay in registers and a node's
-// loads are issued together.  Bound: memory latency and bandwidth, 100 bytes read and written per node (128^3: 73 ->
-// 38 us with the rows that the functional needs, 5.5 TB/s).
+// loads are issued together.  Bound: memory latency and bandwidth, 104 bytes read and written per node (128^3: 73 ->
+// 41 us with the rows that the functional needs, 5.3 TB/s).
 template <int ND, bool ALPHA>
 __global__ void __launch_bounds__(kThreads) k_schur_local32(const float *__restrict__ conv, const float *__restrict__ coef,
                                                              float *__restrict__ chan, float *__restrict__ ymf)
