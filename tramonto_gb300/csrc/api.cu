@@ -1320,11 +1320,14 @@ const double *prolonged(Ctx *c, const double *v, int nrows)
 }
 
 // The FP32 Schur product with FP32 storage: every stencil sum an FP32 FFT (the choices already made by timing), in
-// 2-D or 3-D, with one quadrature zone, no hard-wall corrections and no coarsened nodes
+// 3-D, or in 2-D with one component, with one quadrature zone, no hard-wall corrections and no coarsened nodes.  With
+// one component each row is one FP32 sum, of which an FP64 row holds no more; with several, 2-D problems add the
+// densities' FP32 sums to FP64 rows (they may cancel each other).
 bool schur_store32_ok(Ctx *c)
 {
   const tgpu::DevGeom &g = c->dg;
-  if (!prod_f32(c) || !c->spec32_built || g.ndim < 2 || c->nzone != 1 || !c->hw_targets.empty() || c->coarse())
+  if (!prod_f32(c) || !c->spec32_built || g.ndim < 2 || (g.ndim == 2 && g.ncomp > 1) || c->nzone != 1 ||
+      !c->hw_targets.empty() || c->coarse())
     return false;
   const int nde = 1 + (g.single_size ? 0 : 2) + g.ndim * (g.single_size ? 1 : 2);
   for (int jc = 0; jc < g.ncomp; jc++) {
@@ -1377,7 +1380,7 @@ void schur_device_store32(Ctx *c, const double *d_v2, double *d_y2, bool precond
   }
   c->store32 = false;
   c->pad_src32 = nullptr;
-  tgpu::launch_schur_combine32(c->d_inv32, c->d_kind32, d_v2, c->d_tr32, c->d_ymf32, d_y2,
+  tgpu::launch_schur_combine32(g.ndim, c->d_inv32, c->d_kind32, d_v2, c->d_tr32, c->d_ymf32, d_y2,
                                 precond ? c->d_x : nullptr, c->stream);
   c->stats.kernel_launches += 2;
   c->stats.schur_applies++;
@@ -1443,9 +1446,9 @@ void schur_rhs_device(Ctx *c, const double *d_b, double *d_b2s)
     b = c->d_cscr;
   }
   TcScope tcs(c);
-  if (prod_f32(c) && schur_store32_ok(c)) {   // the FP32 products' right-hand side in FP32 storage
+  if (prod_f32(c) && g.ndim == 3 && schur_store32_ok(c)) {   // the FP32 products' right-hand side in FP32 storage
     ensure_store32(c);
-    tgpu::launch_rhs_local32(g.ndim, tgpu::fmt_alpha_form(g.functional), g.N, b, c->d_hcoef32, c->d_chan32, c->d_ymf32, c->stream);
+    tgpu::launch_rhs_local32(tgpu::fmt_alpha_form(g.functional), g.N, b, c->d_hcoef32, c->d_chan32, c->d_ymf32, c->stream);
     c->store32 = true;
     try {
       transpose_pass(c, c->pads.tr_jac, true);

@@ -1435,7 +1435,9 @@ void launch_row_info32(const double *x, const double *vext, const signed char *z
 
 // k_schur_combine with the transposed sums and -u_MF in FP32 storage and the rows of k_row_info32 (no FP64 division
 // or comparison per product)
-// (x: also multiplied by the diagonal preconditioner, rho on rows with a logarithm)
+// (x: also multiplied by the diagonal preconditioner, rho on rows with a logarithm).  WIDE: the two sums are added in
+// FP64, as the 2-D products without FP32 storage add them; 3-D adds them in FP32 (the FP64 pipe is the kernel's bound).
+template <bool WIDE>
 __global__ void k_schur_combine32(const double *__restrict__ inv, const signed char *__restrict__ kind,
                                   const double *__restrict__ v2, const float *__restrict__ tr,
                                   const float *__restrict__ ymf, double *__restrict__ y2, const double *__restrict__ x)
@@ -1448,16 +1450,20 @@ __global__ void k_schur_combine32(const double *__restrict__ inv, const signed c
       y2[k] = v2[k];
     } else {
       const double t = v2[k] * inv[k];
-      const double r = kd == 0 ? t - (double)(att ? tr[k] + ymf[k] : tr[k]) : t;
+      double a21y = 0.0;
+      if (WIDE) a21y = att ? (double)tr[k] + (double)ymf[k] : (double)tr[k];
+      else a21y = (double)(att ? tr[k] + ymf[k] : tr[k]);
+      const double r = kd == 0 ? t - a21y : t;
       y2[k] = x ? r * x[(long)c_g.first_rho * c_g.N + k] : r;
     }
   }
 }
 
-void launch_schur_combine32(const double *inv, const signed char *kind, const double *v2, const float *tr,
+void launch_schur_combine32(int ndim, const double *inv, const signed char *kind, const double *v2, const float *tr,
                             const float *ymf, double *y2, const double *x, cudaStream_t s)
 {
-  k_schur_combine32<<<1184, kThreads, 0, s>>>(inv, kind, v2, tr, ymf, y2, x);
+  if (ndim == 3) k_schur_combine32<false><<<1184, kThreads, 0, s>>>(inv, kind, v2, tr, ymf, y2, x);
+  else k_schur_combine32<true><<<1184, kThreads, 0, s>>>(inv, kind, v2, tr, ymf, y2, x);
 }
 
 __global__ void k_jv_combine(const double *__restrict__ x, const double *__restrict__ vext,
@@ -1566,17 +1572,12 @@ __global__ void __launch_bounds__(kThreads) k_rhs_local32(const double *__restri
   }
 }
 
-void launch_rhs_local32(int ndim, bool alpha, long N, const double *b, const float *coef, float *chan, float *ymf,
+void launch_rhs_local32(bool alpha, long N, const double *b, const float *coef, float *chan, float *ymf,
                         cudaStream_t s)
 {
   const int grid = node_blocks(N);
-  if (ndim == 3) {
-    if (alpha) k_rhs_local32<3, true><<<grid, kThreads, 0, s>>>(b, coef, chan, ymf);
-    else k_rhs_local32<3, false><<<grid, kThreads, 0, s>>>(b, coef, chan, ymf);
-  } else {
-    if (alpha) k_rhs_local32<2, true><<<grid, kThreads, 0, s>>>(b, coef, chan, ymf);
-    else k_rhs_local32<2, false><<<grid, kThreads, 0, s>>>(b, coef, chan, ymf);
-  }
+  if (alpha) k_rhs_local32<3, true><<<grid, kThreads, 0, s>>>(b, coef, chan, ymf);
+  else k_rhs_local32<3, false><<<grid, kThreads, 0, s>>>(b, coef, chan, ymf);
 }
 
 // b2s = b2 - A21 y1 on full Euler-Lagrange rows (the rows' kinds from k_row_info32), b2 elsewhere

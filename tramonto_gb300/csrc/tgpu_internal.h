@@ -549,13 +549,13 @@ void launch_hess_coef(long N, int ndim, int fn, const double *x, double *coef, c
 void launch_hess_coef32(long N, int ndim, int fn, const double *x, float *coef, cudaStream_t s);
 void launch_schur_local32(int ndim, bool alpha, long N, const float *conv, const float *coef, float *chan, float *ymf,
                           cudaStream_t s);
-void launch_rhs_local32(int ndim, bool alpha, long N, const double *b, const float *coef, float *chan, float *ymf,
+void launch_rhs_local32(bool alpha, long N, const double *b, const float *coef, float *chan, float *ymf,
                         cudaStream_t s);
 void launch_rhs_combine32(const signed char *kind, const double *b, const float *tr, const float *ymf, double *b2s,
                           cudaStream_t s);
 void launch_row_info32(const double *x, const double *vext, const signed char *zero, double *inv, signed char *kind,
                        cudaStream_t s);
-void launch_schur_combine32(const double *inv, const signed char *kind, const double *v2, const float *tr,
+void launch_schur_combine32(int ndim, const double *inv, const signed char *kind, const double *v2, const float *tr,
                             const float *ymf, double *y2, const double *x, cudaStream_t s);
 void launch_schur_local(long N, const double *x, const double *conv, double *chan, double *ymf, const double *coef,
                         cudaStream_t s, bool f32 = false);
