@@ -1031,7 +1031,8 @@ void decide_fft32_2d(Ctx *c, bool tr)
     pass();   // warm-up
     ck(cudaEventRecord(ev[2 * way], c->stream), "event");
     for (int r = 0; r < 2; r++) {
-      c->fft32_gen = -1;   // each FFT pass transforms its field afresh
+      c->fft32_gen = -1;        // each FFT pass transforms its field afresh
+      c->pad_pending = true;    // and each direct one writes its padded box
       pass();
     }
     ck(cudaEventRecord(ev[2 * way + 1], c->stream), "event");
@@ -1039,9 +1040,7 @@ void decide_fft32_2d(Ctx *c, bool tr)
     ck(cudaEventElapsedTime(&t[way], ev[2 * way], ev[2 * way + 1]), "event");
   }
   for (auto &e : ev) cudaEventDestroy(e);
-  // once both directions take FFTs the product runs in FP32 storage, which saves about 12 us of conversions and copies
-  const float bias = tr && c->sten[TGPU_STEN_THETA][0].fft32_fwd == 1 ? 2 * 0.012f : 0.f;   // (ms, two passes timed)
-  for (int *f : flags) *f = t[1] < t[0] + bias ? 1 : -1;
+  for (int *f : flags) *f = t[1] < t[0] ? 1 : -1;
 }
 
 // a 1-D pass's sums in one launch, all rows of the output written (one quadrature zone)
