@@ -183,7 +183,9 @@ enum { TGPU_FILL_FP64 = 0, TGPU_FILL_FP32 = 1, TGPU_FILL_REFINED = 2, TGPU_FILL_
  * everywhere else it is the FP64 fill. */
 int tgpu_set_fill_arithmetic(tgpu_handle h, int arith, double tau, double switch_norm);
 /* Stencils of at least min_points points take the FFT in TGPU_FILL_FFT; min_points < 0 (default): a cost
- * model (direct float-float sum against the transforms) chooses. */
+ * model (direct float-float sum against the transforms) chooses.  The transposed sums of J^T w (tgpu_jtv, the adjoint
+ * solves and gradients; 3-D) share their transforms and take the FFT together: when every stencil has at least
+ * min_points points, or by a cost model against the direct FP64 sums; INT_MAX keeps them direct. */
 int tgpu_set_fft_threshold(tgpu_handle h, int min_points);
 /* FP32 stencil sums (products, FP32 fills) as FP32 FFT convolutions: -1 (default) each sum's first use times
  * the FFT against its direct kernel and keeps the faster (in 2-D problems the sums of a pass together); 0 never;
@@ -212,7 +214,13 @@ int tgpu_sizes(tgpu_handle h, long *nnodes, int *nunk, int *ncomp);
  * mode 1 is residual only (resid_only_flag CALC_RESID_ONLY). */
 int tgpu_fill(tgpu_handle h, const double *x, double *resid, int mode);
 int tgpu_fill_device(tgpu_handle h, const double *d_x, double *d_resid, int mode);
-/* J v and J^T w with the Jacobian of the last mode-0 fill ([nunk][N] each) */
+/* J v and J^T w with the Jacobian of the last mode-0 fill ([nunk][N] each).  J v in the products' arithmetic
+ * (tgpu_set_precision).  J^T w in FP64 whatever that is: in 1-D, 2-D, with reflecting boundaries or with several
+ * quadrature zones by direct sums; in the other 3-D problems the transposed sums are FP64 FFT convolutions where that is
+ * faster (by a cost model, with memory for the spectra) or where tgpu_set_fft_threshold asks for it.  Their rounding is
+ * relative to the largest entry of the vector, eps log2 of the box, and a non-finite entry of w spreads over the whole
+ * result; with direct sums it stays within the stencils' reach.  The same holds for the adjoint solves and the gradients
+ * of the objectives below. */
 int tgpu_jv(tgpu_handle h, const double *v, double *out);
 int tgpu_jv_device(tgpu_handle h, const double *d_v, double *d_out);
 int tgpu_jtv(tgpu_handle h, const double *w, double *out);

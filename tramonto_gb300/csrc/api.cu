@@ -2,6 +2,7 @@
 // the fill, Jacobian and Schur products, the Schur-complement GMRES and the
 // damped Newton loop.  All device work is issued on the handle's stream.
 #include <algorithm>
+#include <climits>
 #include <functional>
 #include <map>
 #include <cmath>
@@ -1894,7 +1895,7 @@ void adj_conv(Ctx *c, int ch0, int nin, const DevStencil &st, const double *coef
 // rate, a transform 7e-12 s per half-spectrum point and log2 of the box (as fft_worth).  Binary pore 96 x 96 x 64:
 // 11.6 ms of direct sums (theta 1015 and 123, delta 844 and 208 points) against 24 transforms, 1.5 ms.  Both are FP64
 // sums; the transforms' error against 64-bit values is not the larger one (eps log2 of the box against eps times the
-// root of the number of terms).
+// root of the number of terms); tgpu_set_fft_threshold fixes the choice.
 bool adj_use_fft(Ctx *c)
 {
   if (c->adj_fft != 0) return c->adj_fft == 1;
@@ -1905,16 +1906,20 @@ bool adj_use_fft(Ctx *c)
   if (!c->fft_plan_ok) return false;
   double terms = 0.0;
   size_t nspec = 0;
+  int shortest = INT_MAX;
   for (int t = 0; t < 3; t++)
     for (auto &st : c->sten[t]) {
       const int nq = t == TGPU_STEN_DELTA ? 1 + g.ndim : 1;
       if (st.L == 0) continue;
+      shortest = std::min(shortest, st.L);
       terms += (t == TGPU_STEN_UATT ? 1.0 : 2.0) * nq * st.L;
       nspec += nq;
     }
   const double transforms = g.ncomp * (2.0 * (g.ndim + 2) + 2.0 + (g.attraction ? g.ncomp : 0));
   const double NH = (double)c->fft.NH;
-  if (terms * (double)g.N * 1.65e-12 <= transforms * NH * std::log2((double)c->fft.NR) * 7.0e-12) return false;
+  if (c->fft_min_points >= 0 ? shortest < c->fft_min_points
+                             : terms * (double)g.N * 1.65e-12 <= transforms * NH * std::log2((double)c->fft.NR) * 7.0e-12)
+    return false;
   const size_t nbox = (size_t)(g.ndim + 3 + g.ncomp);
   size_t free_b = 0, total_b = 0;
   ck(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");

@@ -369,7 +369,8 @@ class Solver:
         _check(self.lib.tgpu_set_fill_arithmetic(self.h, int(arith), float(tau), float(switch_norm)), self.lib)
 
     def set_fft_threshold(self, min_points: int):
-        """Stencils of at least min_points points take the FFT in FILL_FFT; < 0: the cost model decides."""
+        """Stencils of at least min_points points take the FFT in FILL_FFT, and in J^T products when all of them have
+        (2**31 - 1: direct sums there); < 0: the cost model decides."""
         _check(self.lib.tgpu_set_fft_threshold(self.h, int(min_points)), self.lib)
 
     def set_fft32_policy(self, policy: int):
