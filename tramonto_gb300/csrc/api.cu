@@ -181,7 +181,7 @@ struct Ctx : tgpu_ctx {
   long pad_gen = 0, fft_gen = -1;
   int fft_ch = -1;
   int fft_min_points = -1;       // < 0: the cost model decides which stencils take the FFT
-  bool fft_plan_ok = false;
+  int fft_plan = 0;              // the plan alone: 0 not made, 1 ready, -1 not available
   // FP32 FFT sums of the long stencils in FP32 arithmetic: chosen per context by timing against the
   // tensor-core sum (products) and the FP32 slab sum (FP32 fills): 0 undecided, 1 FFT, -1 direct
   float2 *d_fbox32[3] = {nullptr, nullptr, nullptr};
@@ -461,18 +461,17 @@ void kernel_spectrum(Ctx *c, const DevStencil &st, int side, int q, double *rbox
   tgpu::rfft_forward_box(rbox, spec, c->fft, c->stream);
 }
 
-// plan, work boxes and the spectra of every zone-0 stencil coefficient (forward outputs, transpose inputs)
-void ensure_fft(Ctx *c)
+// the transforms' plan, with the profiles of unequal x ends; false where the problem has none
+bool ensure_fft_plan(Ctx *c)
 {
-  if (c->fft_state != 0) return;
-  c->fft_state = -1;
+  if (c->fft_plan != 0) return c->fft_plan == 1;
+  c->fft_plan = -1;
   const tgpu::DevGeom &dg = c->dg;
-  if (dg.ndim < 2) return;
+  if (dg.ndim < 2) return false;
   int P[3], nx[3], h[3], per[3], share[3];
   plan_geometry_args(c, P, nx, h, per);
   share_args(c, share);
-  if (!tgpu::fft_make_plan(c->fft, P, nx, h, per, share, dg.ndim, c->stream)) return;
-  c->fft_plan_ok = true;
+  if (!tgpu::fft_make_plan(c->fft, P, nx, h, per, share, dg.ndim, c->stream)) return false;
   if (share[0] && (c->g.bc[0][0] != c->g.bc[0][1] || c->g.interface == 2))
     for (int t = 0; t < 3; t++)
       for (auto &st : c->sten[t]) {
@@ -480,7 +479,17 @@ void ensure_fft(Ctx *c)
         if (!st.d_prof_fwd) st.d_prof_fwd = low_end_profile(c, st, st.d_coef_fwd, st.nout_fwd);
         if (!st.d_prof_tr && st.d_coef_tr) st.d_prof_tr = low_end_profile(c, st, st.d_coef_tr, st.nin_tr);
       }
-  if (dg.ndim != 3) return;   // in 2-D the accurate fills keep the direct FP64 sums
+  c->fft_plan = 1;
+  return true;
+}
+
+// plan, work boxes and the spectra of every zone-0 stencil coefficient (forward outputs, transpose inputs)
+void ensure_fft(Ctx *c)
+{
+  if (c->fft_state != 0) return;
+  c->fft_state = -1;
+  if (!ensure_fft_plan(c)) return;
+  if (c->dg.ndim != 3) return;   // in 2-D the accurate fills keep the direct FP64 sums
   const long NH = c->fft.NS, NR = c->fft.NR;   // stored half-spectrum points
   // device memory: three work spectra and one spectrum per stencil coefficient
   size_t nspec = 0;
@@ -528,7 +537,7 @@ bool prepare_spec32(Ctx *c)
 {
   if (c->spec32_built) return true;
   ensure_fft(c);
-  if (!c->fft_plan_ok) return false;
+  if (c->fft_plan != 1) return false;
   const long NH = c->fft.NS, NR = c->fft.NR;
   double2 *tmp = dalloc<double2>((size_t)NH);
   double *rbox = dalloc<double>((size_t)NR);
@@ -1308,6 +1317,17 @@ const double *hess_coef(Ctx *c)
   return c->d_hcoef;
 }
 
+// the same for J^T: null, and evaluated in place, where the table cannot be had
+const double *hess_coef_if_room(Ctx *c)
+{
+  if (!c->d_hcoef && cudaMalloc(&c->d_hcoef, sizeof(double) * tgpu::kHessCoef * (size_t)c->dg.N) != cudaSuccess) {
+    cudaGetLastError();
+    c->d_hcoef = nullptr;
+    return nullptr;
+  }
+  return hess_coef(c);
+}
+
 // With coarsened nodes the Schur complement is that of the step on the other nodes: the densities, and
 // the block-1 vector between A12 and A21, are interpolated onto the coarsened nodes, whose rows are dropped.
 const double *prolonged(Ctx *c, const double *v, int nrows)
@@ -1889,21 +1909,26 @@ void adj_conv(Ctx *c, int ch0, int nin, const DevStencil &st, const double *coef
   }
 }
 
+std::vector<double2 *> &adj_boxes(Ctx *c, size_t n)
+{
+  while (c->d_trbox.size() < n) c->d_trbox.push_back(dalloc<double2>((size_t)c->fft.NS));
+  return c->d_trbox;
+}
+
 // Whether the adjoint's transposed sums run as FP64 FFT convolutions (3-D, one quadrature zone, no reflecting
 // boundary, whose mirrored positions are folded back by the direct sums), with the spectra built on first use.  The
 // rule compares the direct FP64 point sums with the transforms: a term and output takes 1.65e-12 s at the FP64 pipe's
 // rate, a transform 7e-12 s per half-spectrum point and log2 of the box (as fft_worth).  Binary pore 96 x 96 x 64:
 // 11.6 ms of direct sums (theta 1015 and 123, delta 844 and 208 points) against 24 transforms, 1.5 ms.  Both are FP64
 // sums; the transforms' error against 64-bit values is not the larger one (eps log2 of the box against eps times the
-// root of the number of terms); tgpu_set_fft_threshold fixes the choice.
+// root of the number of terms); tgpu_set_fft_threshold fixes the choice, and where the spectra and boxes do not fit into
+// half of the free memory the sums stay direct.
 bool adj_use_fft(Ctx *c)
 {
   if (c->adj_fft != 0) return c->adj_fft == 1;
-  const tgpu::DevGeom &g = c->dg;
   c->adj_fft = -1;
-  if (g.ndim != 3 || c->nzone != 1 || has_reflect(c)) return false;
-  ensure_fft(c);
-  if (!c->fft_plan_ok) return false;
+  const tgpu::DevGeom &g = c->dg;
+  if (g.ndim != 3 || c->nzone != 1 || has_reflect(c) || !ensure_fft_plan(c)) return false;
   double terms = 0.0;
   size_t nspec = 0;
   int shortest = INT_MAX;
@@ -1924,19 +1949,30 @@ bool adj_use_fft(Ctx *c)
   size_t free_b = 0, total_b = 0;
   ck(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
   if ((nspec + nbox) * (size_t)c->fft.NS * sizeof(double2) + (size_t)c->fft.NR * sizeof(double) > free_b / 2) return false;
-  double *rbox = dalloc<double>((size_t)c->fft.NR);
-  for (int t = 0; t < 3; t++)
-    for (auto &st : c->sten[t]) {
-      if (st.L == 0) continue;
-      const int nq = t == TGPU_STEN_DELTA ? 1 + g.ndim : 1;
-      for (int q = 0; q < nq; q++) {
-        double2 *k = dalloc<double2>((size_t)c->fft.NS);
-        tgpu::launch_fft_kernel_box(st.d_off, t == TGPU_STEN_DELTA ? st.d_coef_adj : st.d_coef_fwd, st.L, nq, q, -1,
-                                    rbox, c->fft, c->stream);
-        tgpu::rfft_forward_box(rbox, k, c->fft, c->stream);
-        st.spec_adj.push_back(k);
+  double *rbox = nullptr;
+  try {   // (others may take the memory in between)
+    adj_boxes(c, nbox);
+    for (int t = 0; t < 3; t++)
+      for (auto &st : c->sten[t])
+        for (int q = 0; st.L > 0 && q < (t == TGPU_STEN_DELTA ? 1 + g.ndim : 1); q++)
+          st.spec_adj.push_back(dalloc<double2>((size_t)c->fft.NS));
+    rbox = dalloc<double>((size_t)c->fft.NR);
+  } catch (const Error &) {
+    cudaGetLastError();
+    for (int t = 0; t < 3; t++)
+      for (auto &st : c->sten[t]) {
+        for (auto &k : st.spec_adj) dfree(k);
+        st.spec_adj.clear();
       }
-    }
+    return false;
+  }
+  for (int t = 0; t < 3; t++)
+    for (auto &st : c->sten[t])
+      for (size_t q = 0; q < st.spec_adj.size(); q++) {
+        tgpu::launch_fft_kernel_box(st.d_off, t == TGPU_STEN_DELTA ? st.d_coef_adj : st.d_coef_fwd, st.L,
+                                    (int)st.spec_adj.size(), (int)q, -1, rbox, c->fft, c->stream);
+        tgpu::rfft_forward_box(rbox, st.spec_adj[q], c->fft, c->stream);
+      }
   ck(cudaStreamSynchronize(c->stream), "sync");
   dfree(rbox);
   c->adj_fft = 1;
@@ -1956,12 +1992,6 @@ tgpu::MapSrc adj_src(const Ctx *c, int ch)
   }
   m.N = g.N;
   return m;
-}
-
-std::vector<double2 *> &adj_boxes(Ctx *c, size_t n)
-{
-  while (c->d_trbox.size() < n) c->d_trbox.push_back(dalloc<double2>((size_t)c->fft.NS));
-  return c->d_trbox;
 }
 
 // out += the transposed sums of channels chs with kernels k, by one inverse transform
@@ -2092,7 +2122,7 @@ void jtv_device(Ctx *c, const double *d_w_in, double *d_out)
         adj_conv(c, ic, 1, st, st.d_coef_fwd, o + nd + 1, 1);
       }
     }
-    tgpu::launch_jtv_local(c->dg.N, c->d_x, c->d_vext, c->d_zero, d_w, c->d_adj_g, gst, 1, d_out, hess_coef(c), c->stream);
+    tgpu::launch_jtv_local(c->dg.N, c->d_x, c->d_vext, c->d_zero, d_w, c->d_adj_g, gst, 1, d_out, hess_coef_if_room(c), c->stream);
     c->stats.kernel_launches += 4;
   }
   if (c->coarse()) {
@@ -3377,7 +3407,7 @@ int tgpu_set_fft_threshold(tgpu_handle h, int min_points)
   return guard([&] {
     Ctx *c = C(h);
     c->fft_min_points = min_points < 0 ? -1 : min_points;
-    if (c->fft_state != 0) {   // spectra are rebuilt for the new choice at the next FFT fill
+    if (c->fft_plan != 0 || c->fft_state != 0) {   // spectra are rebuilt for the new choice at their next use
       ck(cudaStreamSynchronize(c->stream), "sync");
       for (int t = 0; t < 3; t++)
         for (auto &st : c->sten[t]) {
@@ -3403,7 +3433,7 @@ int tgpu_set_fft_threshold(tgpu_handle h, int min_points)
       tgpu::fft_free_plan(c->fft);
       c->fft_state = 0;
       c->fft_gen = -1;
-      c->fft_plan_ok = false;
+      c->fft_plan = 0;
       c->spec32_built = false;
       c->adj_fft = 0;
       c->fft32_tc = c->fft32_slab = 0;
