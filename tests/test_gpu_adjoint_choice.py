@@ -68,3 +68,19 @@ def test_reflecting_boundaries_stay_direct():
         sums.append(s.stats()["conv_launches"])
     assert sums[0] == sums[1] == sums[2] >= 4
     s.close()
+
+
+def test_adjoint_products_do_not_build_the_fills_spectra():
+    import torch
+    from tramonto_gb300 import native, setup
+    p = setup.config2(n=64)[0]
+    s = native.Solver(p)
+    x = setup.initial_state(s, p)
+    s.fill(x)
+    s.jtv(np.ones(s.shape))
+    free = torch.cuda.mem_get_info()[0]
+    s.set_fill_arithmetic(native.FILL_FFT)
+    s.fill(x)
+    # theta, delta and attraction: twelve spectra and three boxes of (F / 2 + 1) x 64 x 64 points, F at least 64
+    assert free - torch.cuda.mem_get_info()[0] >= 15 * 33 * 64 * 64 * 16
+    s.close()
