@@ -632,7 +632,7 @@ def main():
                          "fp32_slab_ms_per_launch": t_wca32, "fp32_slab_tflops": flops_att / (t_wca32 * 1e-3) / 1e12,
                          "fp64_ms_per_launch": t_wca64},
             # the attraction sum of the accurate fills: an FP64 FFT convolution by default (--accurate-fill fft;
-            # its cost is two real transforms of the 180 x 128 x 128 box, independent of the stencil's length),
+            # its cost is two real transforms of the 160 x 128 x 128 box, independent of the stencil's length),
             # else the float-float sum, bound by the FP32 issue rate (12 FP32 operations per term; nominal 152 SMs
             # x 128 lanes x clock), reported here for comparison
             "fill_attraction_sum": {"fft_ms_per_sum": t_wca_fft,

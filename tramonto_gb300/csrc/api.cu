@@ -206,8 +206,8 @@ struct Ctx : tgpu_ctx {
   // domain flags of the last fill (tgpu::kDomainN3 | tgpu::kDomainRho), set by its local kernels
   unsigned *d_domain = nullptr;
   int hcoef_form = -1;           // the Jacobian form they were made with; -1: stale
-  // FP32 storage of the FP32 Schur products whose every stencil sum is an FP32 FFT (3-D, one zone, no hard-wall
-  // corrections or coarsened nodes): the sums, channels, transposed sums, -u_MF and the state's Hessian scalars
+  // FP32 storage of the FP32 Schur products whose every stencil sum is an FP32 FFT (3-D, or 2-D with one component; one
+  // zone, no hard-wall corrections or coarsened nodes): the sums, channels, transposed sums, -u_MF and the state's Hessian scalars
   // with its weighted densities ([kHessCoef + nrb][N]) in FP32; store32 routes the FFT sums' outputs and inputs
   // there while such a product runs
   bool store32 = false;
@@ -369,7 +369,8 @@ tgpu::MapSrc map_src(const Ctx *c, int ch)
 // Direct, measured on GB300: 5.4e-13 s per term and output of the 128 x 16 tiles, plus 13 us per z-plane of the
 // stencil and wave of tiles for the slabs (one CTA per SM): 81 + 5 ms for the attraction stencil at 128^3 (81), 0.5 +
 // 0.6 ms for the 844-point delta shell on 83 x 101 x 70 nodes (1.02), 0.05 + 0.2 ms for a 123-point ball on 96 x 96 x
-// 64 (0.25).  A transform: 7e-12 s per half-spectrum point and log2 of the box (0.22 ms for the 180 x 128 x 128 box).
+// 64 (0.25).  A transform: 7e-12 s per half-spectrum point and log2 of the box (0.20 ms for the 160 x 128 x 128 box of
+// 128^3 nodes).
 bool fft_worth(const Ctx *c, const DevStencil &st, int nq)
 {
   if (c->fft_min_points >= 0) return st.L >= c->fft_min_points;
@@ -1535,7 +1536,7 @@ bool has_reflect(const Ctx *c);
 // Whether a cycle of kdim steps runs as one cooperative launch (gmres_line.h): 1-D, one quadrature zone, no hard-wall
 // corrections, coarsened nodes or (transposed) reflecting boundaries, at most 64 nodes per SM, and windows that fit in
 // shared memory.  Measured per iteration, launches and host wait against the one launch: HS wall, 2001 nodes, FP64 210
-// -> 43 us; slit pore, 1487 nodes, FP32 products 185 -> 38 us; its adjoint at 801 nodes 400 -> 36 us.
+// -> 27 us; slit pore, 1487 nodes, FP32 products 185 -> 25 us; its adjoint at 801 nodes 400 -> 25 us.
 int line_per(Ctx *c, int kdim)
 {
   const tgpu::DevGeom &g = c->dg;

@@ -252,10 +252,10 @@ struct OutBatch {
 
 // ---- y and z passes ---------------------------------------------------------------------------------------------
 // Bound: FP32 by latency (issue 50%, L2 27%: load, exchange, store with four CTAs per SM), FP64 by the FP64 pipe
-// (~80% of its 304 operations per clock).  Measured on the 180 x 128 x 128 box (91 x 128 x 128 half spectrum), five
-// FP32 forward transforms per launch 26 us = 4.6 TB/s of spectrum read and written (39 us with radix-4 stages that
-// each went through shared memory); six FP64 inverse transforms with their products 400 us (430).  On the 160 x 128 x 128
-// box 21.7 and 365 us.
+// (~80% of its 304 operations per clock).  Measured on the 160 x 128 x 128 box of 128^3 nodes (81 x 128 x 128 half
+// spectrum), five FP32 forward transforms per launch 21.7 us = 4.9 TB/s of spectrum read and written; six FP64 inverse
+// transforms with their products 365 us.  Against radix-4 stages that each went through shared memory, both on a 180 x
+// 128 x 128 box: 39 -> 26 us and 430 -> 400.
 // lines_per_cta adjacent lines (element stride es) at one outer index; reads `in` (or, inverse, the products of `terms`) and
 // writes `out` (in place when out == in: a CTA has read its lines before it writes them).  R1 in (LO, HI]: one kernel
 // per range of radices, so that short ones do not carry the registers of long ones.
@@ -341,9 +341,9 @@ __global__ void __launch_bounds__(lines_per_cta<C>() * HI) k_fft_lines(PassBatch
 // A CTA takes up to kXPairs complex lines (pairs of real ones).  A line's values lie along x, so they are staged through
 // shared memory: one warp reads or writes a line with consecutive lanes, and the two register steps work on the tile.
 // (Register steps that read and wrote global memory themselves, in runs of R1 or R2 elements, took 87 instead of 36 us
-// per FP32 inverse launch.)  Bound as the y and z passes; 128^3 workload, per launch of 1 and 5 or 6 lines' transforms:
-// forward 42 us in FP32 (47 with radix-4 stages), inverse 35 (33); FP64 271 (318) and 274 (338) on the 180 x 128 x 128 box,
-// 35, 28, 232 and 278 on the 160 x 128 x 128 one.
+// per FP32 inverse launch.)  Bound as the y and z passes; 128^3 workload (160 x 128 x 128 box), per launch of 1 and 5 or 6
+// lines' transforms: forward 35 us in FP32, inverse 28; FP64 232 and 278.  Against radix-4 stages, both on a 180 x 128 x 128
+// box: 47 -> 42, 33 -> 35, 318 -> 271 and 338 -> 274.
 // Eight pairs per CTA: more and smaller CTAs than sixteen overlap one's loads with another's steps in FP32 (forward 37.3
 // -> 35.0 us, inverse 29.1 -> 27.7 on the 160 x 128 x 128 box; four: the same).
 constexpr int kXPairs = 8;

@@ -19,7 +19,7 @@
 // Hessian's coefficients, densities.
 // Bound: latency (a warp's FP64 operation holds its scheduler's pipe for 64 cycles, so short serial steps count) and
 // four barriers; 2001 nodes of hard spheres in FP64: 27 us per iteration against 210, 1487 nodes of the slit pore with
-// FP32 products 24 against 185, adjoint of 801 nodes 25 (with a barrier after phase 4's norm, a tile at a time and global
+// FP32 products 25 against 185, adjoint of 801 nodes 25 (with a barrier after phase 4's norm, a tile at a time and global
 // memory for the nodes' tables 43, 38 and 36).  The channels of the local step formed by a warp each: 2 % less, not kept.
 //
 // TR: the transposed Schur complement (adjoint solves), from the stencils with negated offsets.

@@ -68,7 +68,8 @@ constexpr double kDensityMin = 1.e-20;   // integrands vanish at or below this d
 // 3-D real-to-complex FFTs for the stencil sums (fft.cu): real box [F2][F1][F0] with F_d = n_d on periodic
 // dimensions (no padding) and F_d >= the padded extent elsewhere
 // (n_d + h_d where one boundary value serves both ends), half spectrum [F2][F1][F0/2 + 1]; each axis's
-// length is a product of radices 2, 3, 4, 5
+// length is a product of two register DFT lengths (radices_of in fft.cu: the products of 2, 3, 5 and 7 up to 432 but 245,
+// 343 and 392)
 struct FftAxis {
   int n = 1, R1 = 1, R2 = 1;   // length and its two radices
   double2 *d_tw = nullptr;   // exp(-2 pi i k / n), k < n
